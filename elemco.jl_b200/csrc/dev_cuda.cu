@@ -255,13 +255,6 @@ struct GemmArgs {
   double alpha, beta;
   int a_kfast, b_nfast;  // loader thread order follows the unit-stride index
   int64_t klast;         // split-K: depth of the last z-slice (0 = all slices use k)
-  int64_t dn = 0, scn2 = 0;  // dn > 0: column n at (n % dn)*scn + (n / dn)*scn2
-  int64_t kseg = 0;          // kseg > 0: k >= kseg reads A1/B1 with strides sak1/sbk1
-  const double* A1 = nullptr;
-  int64_t sak1 = 0;
-  const double* B1 = nullptr;
-  int64_t sbk1 = 0;
-  const int64_t* ptab = nullptr;  // GF_PTAB: offsets of A, B, C, A1, B1 per batch item
 };
 
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool pred) {
@@ -323,11 +316,7 @@ struct GemmCfg {
 };
 
 // KMMA = 0: mma.m8n8k4 (8-row fragments); KMMA = 4, 8, 16: mma.m16n8kKMMA.
-// FLAGS: bit 0 = two K segments (kseg/A1/B1), bit 1 = split column index (dn),
-// bit 2 = batch items placed by an offset table (ptab) instead of strides;
-// plain GEMMs instantiate none, so their loader and epilogue stay minimal.
-constexpr int GF_SEG = 1, GF_DN = 2, GF_PTAB = 4;
-template <int BM, int BN, int BK, int WM, int WN, int STAGES, int MINB, int KMMA, int FLAGS>
+template <int BM, int BN, int BK, int WM, int WN, int STAGES, int MINB, int KMMA>
 __global__ void __launch_bounds__(GemmCfg<BM, BN, BK, WM, WN, STAGES>::THREADS, MINB)
     dgemm_kernel(GemmArgs g) {
   using Cfg = GemmCfg<BM, BN, BK, WM, WN, STAGES>;
@@ -341,25 +330,9 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, BK, WM, WN, STAGES>::THREADS, 
   double* Bs = smem + STAGES * Cfg::A_STAGE;
 
   const int64_t bz = blockIdx.z;
-  const double* A;
-  const double* B;
-  double* C;
-  const double* A1 = g.A1;
-  const double* B1 = g.B1;
-  if constexpr ((FLAGS & GF_PTAB) != 0) {
-    const int64_t* pt = g.ptab + 5 * bz;
-    A = g.A + pt[0];
-    B = g.B + pt[1];
-    C = g.C + pt[2];
-    if constexpr ((FLAGS & GF_SEG) != 0) {
-      A1 = g.A1 + pt[3];
-      B1 = g.B1 + pt[4];
-    }
-  } else {
-    A = g.A + bz * g.sab;
-    B = g.B + bz * g.sbb;
-    C = g.C + bz * g.scb;
-  }
+  const double* A = g.A + bz * g.sab;
+  const double* B = g.B + bz * g.sbb;
+  double* C = g.C + bz * g.scb;
   const int64_t m0 = (int64_t)blockIdx.x * BM;
   const int64_t n0 = (int64_t)blockIdx.y * BN;
   const int tid = threadIdx.x;
@@ -383,13 +356,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, BK, WM, WN, STAGES>::THREADS, 
         int64_t gm = m0 + mm, gk = k0 + kk;
         bool ok = gm < g.m && gk < kdep;
         const double* src = A;
-        if constexpr ((FLAGS & GF_SEG) != 0) {
-          if (ok)
-            src = (gk >= g.kseg) ? A1 + gm * g.sam + (gk - g.kseg) * g.sak1
-                                 : A + gm * g.sam + gk * g.sak;
-        } else {
-          if (ok) src = A + gm * g.sam + gk * g.sak;
-        }
+        if (ok) src = A + gm * g.sam + gk * g.sak;
         cp_async8(as + kk * Cfg::LDA_S + mm, src, ok);
       }
     }
@@ -402,13 +369,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, BK, WM, WN, STAGES>::THREADS, 
         int64_t gn = n0 + nn, gk = k0 + kk;
         bool ok = gn < g.n && gk < kdep;
         const double* src = B;
-        if constexpr ((FLAGS & GF_SEG) != 0) {
-          if (ok)
-            src = (gk >= g.kseg) ? B1 + (gk - g.kseg) * g.sbk1 + gn * g.sbn
-                                 : B + gk * g.sbk + gn * g.sbn;
-        } else {
-          if (ok) src = B + gk * g.sbk + gn * g.sbn;
-        }
+        if (ok) src = B + gk * g.sbk + gn * g.sbn;
         cp_async8(bs + kk * Cfg::LDB_S + nn, src, ok);
       }
     }
@@ -491,10 +452,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, BK, WM, WN, STAGES>::THREADS, 
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int64_t col = n0 + wn0 + j * 8 + 2 * tq + h;
-      if constexpr ((FLAGS & GF_DN) != 0)
-        coff[j][h] = (col % g.dn) * g.scn + (col / g.dn) * g.scn2;
-      else
-        coff[j][h] = col * g.scn;
+      coff[j][h] = col * g.scn;
     }
   if (g.beta == 0.0) {
 #pragma unroll
@@ -540,18 +498,17 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, BK, WM, WN, STAGES>::THREADS, 
     }
 }
 
-template <int BM, int BN, int BK, int WM, int WN, int STAGES, int MINB = 1, int KMMA = 0,
-          int FLAGS = 0>
+template <int BM, int BN, int BK, int WM, int WN, int STAGES, int MINB = 1, int KMMA = 0>
 static int launch_gemm(const GemmArgs& g, int64_t batch, cudaStream_t st) {
   using Cfg = GemmCfg<BM, BN, BK, WM, WN, STAGES>;
   static DeviceFlags attr;
   if (!attr.test())
-    attr.set(cudaFuncSetAttribute(dgemm_kernel<BM, BN, BK, WM, WN, STAGES, MINB, KMMA, FLAGS>,
+    attr.set(cudaFuncSetAttribute(dgemm_kernel<BM, BN, BK, WM, WN, STAGES, MINB, KMMA>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM));
   int64_t gx = (g.m + BM - 1) / BM, gy = (g.n + BN - 1) / BN;
   if (gy > 65535 || batch > 65535) return (int)cudaErrorInvalidConfiguration;
   dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)batch);
-  dgemm_kernel<BM, BN, BK, WM, WN, STAGES, MINB, KMMA, FLAGS>
+  dgemm_kernel<BM, BN, BK, WM, WN, STAGES, MINB, KMMA>
       <<<grid, Cfg::THREADS, Cfg::SMEM, st>>>(g);
   return launched();
 }
@@ -860,8 +817,7 @@ int gemm_strided(stream_t s, const Gemm& q) {
 
 static int gemm_launch(stream_t s, const Gemm& q) {
   if (q.m <= 0 || q.n <= 0 || q.batch <= 0) return 0;
-  if ((q.n + 63) / 64 > 65535 && (q.m + 63) / 64 <= 65535 && q.kseg == 0 && q.dn == 0 &&
-      !q.ptab) {
+  if ((q.n + 63) / 64 > 65535 && (q.m + 63) / 64 <= 65535) {
     // more column tiles than the grid's y extent: C^T = B^T A^T puts the long
     // dimension on the grid's x axis
     Gemm t = q;
@@ -879,7 +835,6 @@ static int gemm_launch(stream_t s, const Gemm& q) {
     t.scn = q.scm;
     return gemm_launch(s, t);
   }
-  cudaStream_t st = (cudaStream_t)s;
   if (q.k <= 0 || q.alpha == 0.0) {
     // empty contraction: C = beta C
     if (q.beta == 1.0) return 0;
@@ -903,37 +858,6 @@ static int gemm_launch(stream_t s, const Gemm& q) {
   GemmArgs g{q.A, q.B, q.C, q.m, q.n, q.k, q.sam, q.sak, q.sab, q.sbk, q.sbn, q.sbb,
              q.scm, q.scn, q.scb, q.alpha, q.beta, (q.sam != 1 && q.sak == 1) ? 1 : 0,
              (q.sbk != 1 && q.sbn == 1) ? 1 : 0, 0};
-  const int flags = (q.kseg > 0 ? GF_SEG : 0) | (q.dn > 0 ? GF_DN : 0) | (q.ptab ? GF_PTAB : 0);
-  if (q.mapped_tma && (flags & ~GF_DN) == 0 && dgemm_tma_usable_mapped(q)) {
-    const int e = dgemm_tma(s, q, 0, 1);
-    if (e != -1) return e;
-  }
-  if (flags) {
-    if ((!q.ptab && q.batch != 1) || (q.kseg > 0 && (q.kseg >= q.k || !q.A1 || !q.B1)))
-      return (int)cudaErrorInvalidValue;
-    g.dn = q.dn;
-    g.scn2 = q.scn2;
-    g.kseg = q.kseg;
-    g.A1 = q.A1;
-    g.sak1 = q.sak1;
-    g.B1 = q.B1;
-    g.sbk1 = q.sbk1;
-    g.ptab = q.ptab;
-    const int64_t nb = q.batch;
-    switch (flags) {
-      case GF_SEG: return launch_gemm<64, 64, 16, 32, 32, 3, 3, 0, GF_SEG>(g, nb, st);
-      case GF_DN: return launch_gemm<64, 64, 16, 32, 32, 3, 3, 0, GF_DN>(g, nb, st);
-      case GF_SEG | GF_DN:
-        return launch_gemm<64, 64, 16, 32, 32, 3, 3, 0, GF_SEG | GF_DN>(g, nb, st);
-      case GF_PTAB: return launch_gemm<64, 64, 16, 32, 32, 3, 3, 0, GF_PTAB>(g, nb, st);
-      case GF_PTAB | GF_SEG:
-        return launch_gemm<64, 64, 16, 32, 32, 3, 3, 0, GF_PTAB | GF_SEG>(g, nb, st);
-      case GF_PTAB | GF_DN:
-        return launch_gemm<64, 64, 16, 32, 32, 3, 3, 0, GF_PTAB | GF_DN>(g, nb, st);
-      default:
-        return launch_gemm<64, 64, 16, 32, 32, 3, 3, 0, GF_PTAB | GF_SEG | GF_DN>(g, nb, st);
-    }
-  }
   return plain_gemm(s, g, q);
 }
 

@@ -1,8 +1,7 @@
 // dev_dgemm.cu — FP64 GEMM with TMA-staged operands (sm_100a).
 //
-// C(m,n) = alpha * A(m,k) B(k,n) + beta * C with C addressed through a row
-// stride and a column map (plain column stride, or a split column index as the
-// (T) K builds use), batched (3-D tensor maps, one batch item per grid z) or split over
+// C(m,n) = alpha * A(m,k) B(k,n) + beta * C with unit row stride in C,
+// batched (3-D tensor maps, one batch item per grid z) or split over
 // K (grid z = K slice, partial products into the stream's split-K buffer,
 // summed in a fixed order by splitk_reduce).  tcgen05 has no FP64 kind, so the
 // products run on the FP64 MMA pipe (mma.sync m8n8k4 f64).  What the Tensor
@@ -38,6 +37,7 @@
 #include <cstring>
 
 #include "ecg_dev.h"
+#include "dgemm_frag.cuh"
 #include "tma_util.cuh"
 
 namespace ecg {
@@ -46,8 +46,7 @@ namespace dev {
 namespace {
 
 using namespace tma;
-
-constexpr int DK = 16;  // k depth of a stage: 16 doubles, one 128-byte swizzle row
+using namespace dfrag;
 
 __device__ int g_dtma_error = 0;
 
@@ -66,77 +65,13 @@ struct DCfg {
 };
 
 struct DOut {
-  // element (i, j) of grid-z item z at C + z*scb + i*scm + colmap(j), colmap(j)
-  // = (j % dn)*scn + (j / dn)*scn2 (dn = 0: j*scn)
+  // element (i, j) of grid-z item z at C + z*scb + i + j*scn
   double* C;
   int64_t m, n, scn, scb;
   double alpha, beta;
-  int64_t scm = 1, dn = 0, scn2 = 0;
 };
 
-__device__ __forceinline__ void dmma884(double (&d)[2], double a, double b) {
-  asm volatile(
-      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-      : "+d"(d[0]), "+d"(d[1])
-      : "d"(a), "d"(b));
-}
-
-// Row (within a 16-row block) that lane group g reads in MMA s of an i-fast
-// operand.
-__device__ __forceinline__ int jmap(int g, int s) {
-  return (g & 1) + 8 * ((g >> 1) & 1) + 2 * (g >> 2) + 4 * s;
-}
-// Row (within an 8-row block) that lane group g reads of a k-fast operand.
-__device__ __forceinline__ int pmap(int g) { return 2 * (g & 3) + (g >> 2); }
-
-// Per-lane fragment offsets (doubles, within one stage's tile) of an operand
-// whose warp sub-tile starts at row w0 and has NB 8-row blocks.  k-fast:
-// o[q] for k-step kb = 4q, block rb at o[q] + 128 rb.  i-fast: o[2 rb + (q & 1)]
-// + 64 q.
-template <bool KF, int NB>
-struct FragOff {
-  static constexpr int N = KF ? 4 : 2 * NB;
-  uint32_t o[N];
-  __device__ __forceinline__ FragOff(int w0, int g, int t) {
-    if constexpr (KF) {
-      const int p = pmap(g);
-      const uint32_t rowbase = (uint32_t)((w0 + p) * 16 + (t & 1));
-      const int y = (t >> 1) ^ p;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) o[q] = rowbase + (uint32_t)((4 * q) ^ (y << 1));
-    } else {
-#pragma unroll
-      for (int rb = 0; rb < NB; ++rb) {
-        const int j = jmap(g, rb & 1);
-        const uint32_t base = (uint32_t)(((w0 >> 4) + (rb >> 1)) * 256 + t * 16 + (j & 1) +
-                                         (((j >> 1) ^ t) << 1));
-        o[2 * rb] = base;
-        o[2 * rb + 1] = base ^ 8u;
-      }
-    }
-  }
-  __device__ __forceinline__ uint32_t at(int rb, int q) const {
-    if constexpr (KF)
-      return o[q] + 128u * rb;
-    else
-      return o[2 * rb + (q & 1)] + 64u * q;
-  }
-};
-
-// Row (or column) of the tile that accumulator row g of block rb stands for.
-template <bool KF>
-__device__ __forceinline__ int frag_row(int w0, int rb, int g) {
-  if constexpr (KF)
-    return w0 + 8 * rb + pmap(g);
-  else
-    return w0 + 16 * (rb >> 1) + jmap(g, rb & 1);
-}
-
-// RMW2: read-modify-write epilogue that loads a group of C values before
-// storing any (the (T) K builds, whose beta = 1 GEMMs spend most of their
-// epilogue waiting on those loads); the CCSD GEMMs run faster with the
-// one-by-one epilogue, so it is a separate instantiation.
-template <int BM, int BN, int WM, int WN, int STAGES, int MINB, bool AKF, bool BKF, bool RMW2>
+template <int BM, int BN, int WM, int WN, int STAGES, int MINB, bool AKF, bool BKF>
 __global__ void __launch_bounds__(DCfg<BM, BN, WM, WN, STAGES>::THREADS, MINB)
     dgemm_tma_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ CUtensorMap mb,
                      DOut out, int64_t k, int64_t kslice, int split,
@@ -221,8 +156,8 @@ __global__ void __launch_bounds__(DCfg<BM, BN, WM, WN, STAGES>::THREADS, MINB)
     // MMAs that wait for them, let the refill overwrite rows that a load still
     // queued behind a neighbouring CTA's epilogue had yet to read (10-15% of
     // the beta = 1 K builds at v = 318 came out with wrong elements).  The
-    // later release costs nothing: 4096^3 runs at 34.5 instead of 31.8 TF/s
-    // (both operands contiguous along k, 64x64 tiles).
+    // later release costs nothing: 4096^3 runs at 34.5 instead of
+    // 31.8 TF/s (both operands contiguous along k, 64x64 tiles).
     if (t >= 1 && lane == 0) mbar_arrive(&empty[(t - 1) % STAGES]);
     const double* As = (const double*)(smem + s * Cfg::STAGE_BYTES);
     const double* Bs = (const double*)(smem + s * Cfg::STAGE_BYTES + Cfg::A_BYTES);
@@ -263,87 +198,25 @@ __global__ void __launch_bounds__(DCfg<BM, BN, WM, WN, STAGES>::THREADS, MINB)
   }
 
   double* C = out.C + (int64_t)z * out.scb;
-  int64_t coff[NTL][2];
 #pragma unroll
-  for (int j = 0; j < NTL; ++j)
+  for (int i = 0; i < MT; ++i) {
+    const int64_t row = m0 + frag_row<AKF>(wm0, i, g);
+    if (row >= out.m) continue;
+    double* Cr = C + row;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int64_t col = n0 + frag_row<BKF>(wn0, j, 2 * t4 + h);
-      coff[j][h] = col >= out.n ? -1
-                   : out.dn > 0 ? (col % out.dn) * out.scn + (col / out.dn) * out.scn2
-                                : col * out.scn;
-    }
-  if (!RMW2 || out.beta == 0.0) {
+    for (int j = 0; j < NTL; ++j)
 #pragma unroll
-    for (int i = 0; i < MT; ++i) {
-      const int64_t row = m0 + frag_row<AKF>(wm0, i, g);
-      if (row >= out.m) continue;
-      double* Cr = C + row * out.scm;
-#pragma unroll
-      for (int j = 0; j < NTL; ++j)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (coff[j][h] >= 0) {
-            double* cp = Cr + coff[j][h];
-            double v = out.alpha * acc[i][j][h];
-            if (out.beta != 0.0) v += out.beta * *cp;
-            *cp = v;
-          }
+      for (int h = 0; h < 2; ++h) {
+        const int64_t col = n0 + frag_row<BKF>(wn0, j, 2 * t4 + h);
+        if (col < out.n) {
+          double* cp = Cr + col * out.scn;
+          double v = out.alpha * acc[i][j][h];
+          if (out.beta != 0.0) v += out.beta * *cp;
+          *cp = v;
         }
-    }
-    return;
-  }
-  // read-modify-write: ER rows of fragments at a time (16 C values a lane)
-  // are all loaded before any store, so the loads overlap instead of waiting
-  // one by one behind stores the compiler cannot prove disjoint
-  constexpr int ER = NTL > 4 ? 1 : 2;
-#pragma unroll
-  for (int i0 = 0; i0 < MT; i0 += ER) {
-    double cv[ER][NTL][2];
-#pragma unroll
-    for (int ii = 0; ii < ER; ++ii) {
-      const int64_t row = m0 + frag_row<AKF>(wm0, i0 + ii, g);
-      const double* Cr = C + row * out.scm;
-#pragma unroll
-      for (int j = 0; j < NTL; ++j)
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          cv[ii][j][h] = (row < out.m && coff[j][h] >= 0) ? Cr[coff[j][h]] : 0.0;
-    }
-#pragma unroll
-    for (int ii = 0; ii < ER; ++ii) {
-      const int64_t row = m0 + frag_row<AKF>(wm0, i0 + ii, g);
-      if (row >= out.m) continue;
-      double* Cr = C + row * out.scm;
-#pragma unroll
-      for (int j = 0; j < NTL; ++j)
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          if (coff[j][h] >= 0)
-            Cr[coff[j][h]] = out.alpha * acc[i0 + ii][j][h] + out.beta * cv[ii][j][h];
-    }
+      }
   }
 }
-
-// 3-D map over a double operand: inner extent d0 (unit stride), d1 rows
-// s1 doubles apart, d2 batch items s2 doubles apart; box (16, b1, 1),
-// 128-byte swizzle, out-of-range elements read as zero.
-int dmap(CUtensorMap* m, const double* base, int64_t d0, int64_t d1, int64_t s1, int64_t d2,
-         int64_t s2, int b1) {
-  EncodeFn enc = nullptr;
-  if (int e = encode_fn(&enc)) return e;
-  cuuint64_t dims[3] = {(cuuint64_t)d0, (cuuint64_t)d1, (cuuint64_t)d2};
-  cuuint64_t strides[2] = {(cuuint64_t)(s1 * 8), (cuuint64_t)(s2 * 8)};
-  cuuint32_t box[3] = {(cuuint32_t)DK, (cuuint32_t)b1, 1};
-  cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double*>(base), dims,
-                   strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
-}
-
-// a stride (doubles) TMA accepts: a positive multiple of 16 bytes below 2^40 bytes
-bool stride_ok(int64_t s) { return s > 0 && s % 2 == 0 && s < ((int64_t)1 << 37); }
 
 // The map of operand X(i, k) = X[i*si + k*sk + z*sz] (i < ni, k < nk, z <
 // nz): k-fast when sk == 1 (box 16 k x rows), else i-fast (si == 1; box
@@ -369,12 +242,11 @@ bool operand_map(CUtensorMap* m, bool* kfast, const double* X, int64_t ni, int64
   return false;
 }
 
-template <int BM, int BN, int WM, int WN, int STAGES, int MINB, bool AKF, bool BKF,
-          bool RMW2 = false>
+template <int BM, int BN, int WM, int WN, int STAGES, int MINB, bool AKF, bool BKF>
 int launch_dtma(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap& mb, const DOut& out,
                 int64_t k, int64_t kslice, int nz, int split) {
   using Cfg = DCfg<BM, BN, WM, WN, STAGES>;
-  auto kern = dgemm_tma_kernel<BM, BN, WM, WN, STAGES, MINB, AKF, BKF, RMW2>;
+  auto kern = dgemm_tma_kernel<BM, BN, WM, WN, STAGES, MINB, AKF, BKF>;
   // cudaFuncSetAttribute acts on the current device only: one flag per device
   static std::atomic<bool> done[128] = {};
   int d = 0;
@@ -415,22 +287,13 @@ DtmaLaunch pick(int cfg) {
     default: return launch_dtma<64, 64, 32, 32, 4, 3, AKF, BKF>;
   }
 }
-// The (T) K builds' configuration: 64x64 with the grouped read-modify-write.
-template <bool AKF, bool BKF>
-DtmaLaunch pick_rmw() {
-  return launch_dtma<64, 64, 32, 32, 4, 3, AKF, BKF, true>;
-}
 constexpr int CFG_BM[DTMA_CONFIGS] = {64, 128, 64, 128};
 constexpr int CFG_BN[DTMA_CONFIGS] = {64, 64, 128, 128};
 
 }  // namespace
 
 bool dgemm_tma_usable(const Gemm& q) {
-  return q.scm == 1 && q.dn == 0 && dgemm_tma_usable_mapped(q);
-}
-
-bool dgemm_tma_usable_mapped(const Gemm& q) {
-  if (q.kseg || q.ptab || q.m <= 0 || q.n <= 0 || q.k <= 0 || q.dn < 0) return false;
+  if (q.scm != 1 || q.m <= 0 || q.n <= 0 || q.k <= 0) return false;
   if (q.m >= ((int64_t)1 << 31) || q.n >= ((int64_t)1 << 31) || q.k >= ((int64_t)1 << 31))
     return false;
   CUtensorMap m;
@@ -442,8 +305,7 @@ bool dgemm_tma_usable_mapped(const Gemm& q) {
 int dgemm_tma(stream_t s, const Gemm& q, int cfg, int nsplit) {
   if (cfg < 0 || cfg >= DTMA_CONFIGS) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)s;
-  // the split-K reduction writes C through plain strides only
-  if (nsplit > 1 && (q.batch != 1 || q.dn > 0)) return (int)cudaErrorInvalidValue;
+  if (q.scm != 1 || (nsplit > 1 && q.batch != 1)) return (int)cudaErrorInvalidValue;
   CUtensorMap ma, mb;
   bool akf = false, bkf = false;
   if (!operand_map(&ma, &akf, q.A, q.m, q.k, q.sam, q.sak, q.batch, q.sab, CFG_BM[cfg]) ||
@@ -451,11 +313,8 @@ int dgemm_tma(stream_t s, const Gemm& q, int cfg, int nsplit) {
     return -1;
   DtmaLaunch f = akf ? (bkf ? pick<true, true>(cfg) : pick<true, false>(cfg))
                      : (bkf ? pick<false, true>(cfg) : pick<false, false>(cfg));
-  if (q.mapped_tma && cfg == 0)
-    f = akf ? (bkf ? pick_rmw<true, true>() : pick_rmw<true, false>())
-            : (bkf ? pick_rmw<false, true>() : pick_rmw<false, false>());
   if (nsplit <= 1) {
-    DOut o{q.C, q.m, q.n, q.scn, q.scb, q.alpha, q.beta, q.scm, q.dn, q.scn2};
+    DOut o{q.C, q.m, q.n, q.scn, q.scb, q.alpha, q.beta};
     return f(st, ma, mb, o, q.k, q.k, (int)q.batch, 0);
   }
   int64_t kc = (q.k + nsplit - 1) / nsplit;

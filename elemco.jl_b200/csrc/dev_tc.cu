@@ -1087,7 +1087,7 @@ int tc_gemm_batched(stream_t s, const TcGemm& g, int batch, const void* mtab, in
 // gemm_strided (batch 1): split both operands into three slices, run the
 // tensor-core kernel.
 int gemm_strided_mixed(stream_t s, const Gemm& q) {
-  if (q.batch != 1 || q.dn != 0 || q.kseg != 0) return (int)cudaErrorInvalidValue;
+  if (q.batch != 1) return (int)cudaErrorInvalidValue;
   if (q.m <= 0 || q.n <= 0) return 0;
   if (q.k <= 0 || q.alpha == 0.0) return gemm_strided(s, q);
   EncodeFn enc = nullptr;
@@ -1185,10 +1185,11 @@ int tc_error(int* code) {
     int zero = 0;
     cudaMemcpyToSymbol(g_tc_error, &zero, sizeof(int));
   }
-  int d = 0, en = 0;
+  int d = 0, en = 0, kb = 0;
   if (int r = dtma_error(&d)) return r;
   if (int r = energy_error(&en)) return r;
-  *code = h ? h : d ? 16 + d : (en ? 32 + en : 0);
+  if (int r = kbuild_error(&kb)) return r;
+  *code = h ? h : d ? 16 + d : en ? 32 + en : (kb ? 48 + kb : 0);
   return 0;
 }
 

@@ -47,13 +47,6 @@ int gemm(stream_t s, char ta, char tb, int64_t m, int64_t n, int64_t k, double a
 // with A(m,k) = A[b*sab + m*sam + k*sak], B(k,n) = B[b*sbb + k*sbk + n*sbn],
 // C(m,n) = C[b*scb + m*scm + n*scn] for batch b.  Batches must not write
 // overlapping C elements.
-// Optional (batch 1 only):
-//   dn > 0    C(m,n) = C[m*scm + (n % dn)*scn + (n / dn)*scn2]  (n splits into
-//             two tensor indices, e.g. (b,c) of a v^3 cube written permuted)
-//   kseg > 0  two K segments: k < kseg reads A, B as above; k >= kseg reads
-//             A1[m*sam + (k-kseg)*sak1] and B1[(k-kseg)*sbk1 + n*sbn].
-//   ptab      device table of 5 offsets (elements) per batch item b, for A, B,
-//             C, A1, B1, used in place of b*sab, b*sbb, b*scb (batch >= 1).
 struct Gemm {
   int64_t m = 0, n = 0, k = 0, batch = 1;
   double alpha = 1.0, beta = 0.0;
@@ -63,35 +56,51 @@ struct Gemm {
   int64_t sbk = 1, sbn = 0, sbb = 0;
   double* C = nullptr;
   int64_t scm = 1, scn = 0, scb = 0;
-  int64_t dn = 0, scn2 = 0;
-  int64_t kseg = 0;
-  const double* A1 = nullptr;
-  int64_t sak1 = 0;
-  const double* B1 = nullptr;
-  int64_t sbk1 = 0;
-  const int64_t* ptab = nullptr;
-  // run on the TMA-staged kernel whenever it can address the operands, also
-  // with a row stride or column map (the (T) K builds; other callers keep
-  // the dispatcher's choice)
-  bool mapped_tma = false;
 };
 int gemm_strided(stream_t s, const Gemm& g);
-// FP64 GEMM with TMA-staged operands (dev_dgemm.cu): no kseg/ptab (C through
-// scm and scn or the dn/scn2 column map; no K split with dn), each operand
-// contiguous along its row index or along k with its other strides even
-// (16-byte multiples) and a 16-byte-aligned base.  cfg selects the tile (0: 64x64, 1: 128x64, 2: 64x128,
-// 3: 128x128); nsplit > 1 (batch 1) cuts K into slices summed in a fixed
-// order.  Returns -1, launching nothing, when TMA cannot address an operand.
-// dgemm_tma_usable: the cases the plain-GEMM dispatcher sends to it (C with
-// unit row stride, no column map); dgemm_tma_usable_mapped: all it accepts.
+// FP64 GEMM with TMA-staged operands (dev_dgemm.cu): C with unit row stride,
+// each operand contiguous along its row index or along k with its other
+// strides even (16-byte multiples) and a 16-byte-aligned base.  cfg selects the
+// tile (0: 64x64, 1: 128x64, 2: 64x128, 3: 128x128); nsplit > 1 (batch 1) cuts
+// K into slices summed in a fixed order.  Returns -1, launching nothing, when
+// TMA cannot address an operand; dgemm_tma_usable tells beforehand.
 constexpr int DTMA_CONFIGS = 4;
 bool dgemm_tma_usable(const Gemm& q);
-bool dgemm_tma_usable_mapped(const Gemm& q);
 int dgemm_tma(stream_t s, const Gemm& q, int cfg, int nsplit);
 // Time-out code of the TMA FP64 GEMM's bounded waits since the last call
 // (0 = none); reading clears it.
 int dtma_error(int* code);
-// Split-BF16 tensor-core version of gemm_strided (batch 1, no dn/kseg).
+
+// The (T) K builds in FP64 (dev_kbuild.cu): for each item z of a batch
+//   C_z(r,c) = beta C_z(r,c) + sum_{s < nseg} sum_{k < k[s]} A_s(r,k) B_s(c,k)
+// with r < m, c < n and beta 0 or 1.  Operand X(i,k) of item index z sits at
+// X[i + k*sk + z*sz] (i < ni, z < nz; X 16-byte aligned, sk and sz even);
+// items[z] (device memory) names the item of each segment's A and B and the
+// offset of C_z.  C(r,c) sits at (r % dm)*scm + (r / dm)*scm2 + c*scn (dm = 0:
+// r*scm + c*scn).  even_items: every item's C offset is even.  One launch.
+constexpr int KB_MAX_SEG = 4;
+struct KbOperand {
+  const double* X = nullptr;
+  int64_t ni = 0, sk = 0, nz = 1, sz = 2;
+};
+struct KbItem {
+  int32_t a[KB_MAX_SEG], b[KB_MAX_SEG];
+  int64_t c;
+};
+struct KbGemm {
+  int64_t m = 0, n = 0;
+  int nseg = 0;
+  int64_t k[KB_MAX_SEG] = {0, 0, 0, 0};
+  KbOperand A[KB_MAX_SEG], B[KB_MAX_SEG];
+  double beta = 0.0;
+  double* C = nullptr;
+  int64_t scm = 1, dm = 0, scm2 = 0, scn = 0;
+  bool even_items = false;
+};
+int kbuild(stream_t s, const KbGemm& g, int nitems, const KbItem* items);
+// Time-out code of its bounded waits (0 = none); reading clears it.
+int kbuild_error(int* code);
+// Split-BF16 tensor-core version of gemm_strided (batch 1).
 int gemm_strided_mixed(stream_t s, const Gemm& g);
 
 // Pre-split operand of the tensor-core GEMM: X(r,k) as `slices` (2 or 3)
@@ -284,7 +293,7 @@ int gemm_splitk_noalloc(stream_t s, char ta, char tb, int64_t m, int64_t n, int6
 // Split-BF16 tensor-core GEMM (tcgen05, FP32 accumulate, ~FP32 accuracy),
 // same interface as gemm().  tc_error() returns and clears the time-out code
 // of the kernels with bounded mbarrier waits (0 = none; 1-4 tensor-core GEMM,
-// 17 TMA-staged FP64 GEMM, 33 FP32 (T) energy kernel).
+// 17 TMA-staged FP64 GEMM, 33 FP32 (T) energy kernel, 49 FP64 K builds).
 int gemm_mixed(stream_t s, char ta, char tb, int64_t m, int64_t n, int64_t k, double alpha,
                const double* A, int64_t lda, const double* B, int64_t ldb, double beta,
                double* C, int64_t ldc);

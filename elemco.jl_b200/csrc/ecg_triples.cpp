@@ -11,11 +11,15 @@
 // held in two layouts, [b,c,d,k] and [c,b,d,k], chosen per permutation so
 // that the (b',c') pair maps to K through at most one index split; with that
 // choice the permutations pair up into three GEMMs of K depth 2v whose two
-// halves write the same K positions.  On the
-// tensor cores, whose epilogue lanes run along the GEMM rows, a GEMM whose
-// a' index is not the unit stride of K is run transposed (rows (b',c')).
-// With T^{xy}_{ab} = T^{yx}_{ba} the six ovoo GEMMs pair up into three GEMMs
-// with a two-segment K of 2o, also accumulated into K.  A fused kernel forms
+// halves write the same K positions.  With T^{xy}_{ab} = T^{yx}_{ba} the six
+// ovoo GEMMs pair up too, and each ovoo pair writes K through the same index
+// map, with the same rows and columns, as one vvvo pair, so every K
+// orientation is one GEMM of four K segments (v, v, o, o; ovoo held negated):
+// three launches per batch of triplets, each with a single pass over K.  The
+// FP64 builds run their rows over the pair index and their columns over a'.
+// On the tensor cores, whose epilogue lanes run along the GEMM rows, the
+// orientation whose a' index is the unit stride of K runs its rows over a'.
+// A fused kernel forms
 // X and both energy sums (sum K X and the singles/Fock term sum X Y,
 // cc_triples.jl:113-156); per-triplet energies are summed on the host in
 // triplet order, so the result is deterministic.
@@ -23,10 +27,7 @@
 // Mixed precision: every operand is split into two BF16 slices once per call
 // (vvvo in both layouts, T^{xy} per pair, T2[:,:,x,:] and T2[:,:,:,x] per
 // occupied index, -ovoo per pair), the GEMMs run on the tensor cores and K is
-// kept in FP32.  Each ovoo pair writes K through the same index map, and with
-// the same rows and columns, as one vvvo pair, so every K orientation is one
-// tensor-core GEMM of four K segments (v, v, o, o): three launches per batch,
-// each with a single pass over K.
+// kept in FP32.
 #include "ecg_triples.h"
 
 #include <algorithm>
@@ -107,15 +108,36 @@ void split_amps(Ctx& c, const double* T, SplitAmps& S) {
   }
 }
 
-// Everything the K builds read: FP64 integrals and amplitudes, or their
-// BF16 splits.
+// Everything the K builds read: FP64 integrals, or their BF16 splits.  The
+// FP64 operands have even pitches, so that TMA can address them at odd v.
 struct TriplesOps {
   bool mixed = false;
-  const double* V1 = nullptr;  // [b,c,d,k]
-  const double* V2 = nullptr;  // [c,b,d,k]
-  const double* On = nullptr;  // [l,j,c,k]
+  int64_t v2p = 0, vq = 0;     // pitches of a (b,c) pair and of a virtual index
+  const double* V1 = nullptr;  // [b,c,d,k], (b,c) in pitch v2p
+  const double* V2 = nullptr;  // [c,b,d,k], (c,b) in pitch v2p
+  const double* On = nullptr;  // -(lj|ck) as [c,l,j,k], c in pitch vq
   std::vector<dev::TcOperand> V1s, V2s, Ons;
 };
+
+// FP64 amplitudes (T2 or covariant U2) as the K builds read them.
+struct FpAmps {
+  const double* pair = nullptr;  // T^{xy}[a,d], a in pitch vq, per pair x + o*y
+  const double* ab = nullptr;    // T2[(a,b)], pitch v2p, per pair
+};
+
+// A copy in even pitches where v is odd (or the array starts off 16 bytes).
+FpAmps fp_amps(Ctx& c, const double* T, const TriplesOps& ops) {
+  const int64_t o = c.no, v = c.nv, v2 = v * v;
+  FpAmps f{T, T};
+  if (v % 2 == 0 && ((uintptr_t)T & 15) == 0) return f;
+  double* p = c.alloc(ops.vq * v * o * o, "(T) T^{xy} padded");
+  double* ab = c.alloc(ops.v2p * o * o, "(T) T2 padded");
+  check(dev::geam(c.st, v, v * o * o, 1.0, T, v, 0.0, p, ops.vq), "pad T^{xy}");
+  check(dev::geam(c.st, v2, o * o, 1.0, T, v2, 0.0, ab, ops.v2p), "pad T2");
+  f.pair = p;
+  f.ab = ab;
+  return f;
+}
 
 // One occupied triplet of the sweep: indices, weight (cc_triples.jl:62-72) and
 // the denominator shift e_i + e_j + e_k.
@@ -125,43 +147,48 @@ struct Trip {
 };
 
 // Host-built tables of one amplitude tensor's K builds for the whole sweep,
-// uploaded once: FP64 offset tables [9 GEMMs][triplet][A, B, C, A1, B1] or
-// tensor-core descriptor tables [3 GEMMs][triplet][maps of 4 segments].  The C offset is the
-// triplet's slot in its batch.
+// uploaded once: FP64 item tables [3 GEMMs][triplet] (the C offset is the
+// triplet's slot in its batch) or tensor-core descriptor tables [3 GEMMs]
+// [triplet][maps of 4 segments].
 struct KTables {
-  std::vector<int64_t> ptab;
+  std::vector<dev::KbItem> items;
   std::vector<unsigned char> mtab;
-  int64_t* ptab_d = nullptr;
+  dev::KbItem* items_d = nullptr;
   unsigned char* mtab_d = nullptr;
 };
 
-constexpr int kGemmsFP64 = 9, kGemmsMixed = 3;
+constexpr int kGemms = 3;
+// the permutations whose W land in K through one index map
+constexpr int kPairs[kGemms][2] = {{0, 2}, {1, 4}, {3, 5}};
 
 void fill_tables(Ctx& c, const TriplesOps& ops, const SplitAmps* Sp, const std::vector<Trip>& tr,
                  int NB, int64_t kstride, int64_t vp, KTables& kt) {
-  const int64_t o = c.no, v = c.nv, v2 = v * v, v3 = v2 * v, o2 = o * o;
+  const int64_t o = c.no, v = c.nv, v2 = v * v;
   const int64_t nt = (int64_t)tr.size();
-  auto on = [&](int y, int z) { return o * y + o2 * v * z; };
   if (!ops.mixed) {
-    kt.ptab.assign(kGemmsFP64 * nt * 5, 0);
+    kt.items.resize(kGemms * nt);
     for (int64_t t = 0; t < nt; ++t) {
       const int i = tr[t].i, j = tr[t].j, k = tr[t].k;
-      const int64_t offC = (t % NB) * kstride;
       PermW P[6];
       perm_table(i, j, k, v, vp, P);
-      auto put = [&](int q, int64_t a, int64_t b, int64_t a1, int64_t b1) {
-        int64_t* e = kt.ptab.data() + (q * nt + t) * 5;
-        e[0] = a; e[1] = b; e[2] = offC; e[3] = a1; e[4] = b1;
-      };
-      for (int q = 0; q < 6; ++q) put(q, v2 * (P[q].x + o * P[q].y), v3 * P[q].z, 0, 0);
-      put(6, v2 * i, on(j, k), v2 * o * j, on(i, k));
-      put(7, on(k, j), v2 * i, on(i, j), v2 * o * k);
-      put(8, v2 * o * k, on(j, i), v2 * j, on(k, i));
+      auto on = [&](int y, int z) { return (int32_t)(y + o * z); };
+      // ovoo segments: the occupied index of the T2 slices (see build_K_batch)
+      // and the pair of -ovoo
+      const int32_t ov[3][4] = {{k, j, on(j, i), on(k, i)},
+                                {i, k, on(k, j), on(i, j)},
+                                {i, j, on(j, k), on(i, k)}};
+      for (int q = 0; q < kGemms; ++q) {
+        const PermW &p0 = P[kPairs[q][0]], &p1 = P[kPairs[q][1]];
+        kt.items[q * nt + t] = {{p0.z, p1.z, ov[q][0], ov[q][1]},
+                                {(int32_t)(p0.x + o * p0.y), (int32_t)(p1.x + o * p1.y),
+                                 ov[q][2], ov[q][3]},
+                                (t % NB) * kstride};
+      }
     }
     return;
   }
   const size_t mb = dev::tc_maps_bytes();
-  kt.mtab.assign(kGemmsMixed * nt * mb, 0);
+  kt.mtab.assign(kGemms * nt * mb, 0);
   auto op = [&](int y, int z) { return &ops.Ons[y + o * z]; };
   for (int64_t t = 0; t < nt; ++t) {
     const int i = tr[t].i, j = tr[t].j, k = tr[t].k;
@@ -173,10 +200,9 @@ void fill_tables(Ctx& c, const TriplesOps& ops, const SplitAmps* Sp, const std::
         {op(j, i), op(k, i), &Sp->C[k], &Sp->G[j]},   // rows a, columns (b,c)
         {&Sp->G[i], &Sp->C[k], op(k, j), op(i, j)},   // rows (a,c), columns b
         {&Sp->G[i], &Sp->C[j], op(j, k), op(i, k)}};  // rows (a,b), columns c
-    const int pairs[3][2] = {{0, 2}, {1, 4}, {3, 5}};
-    for (int q = 0; q < 3; ++q) {
-      const PermW& p0 = P[pairs[q][0]];
-      const PermW& p1 = P[pairs[q][1]];
+    for (int q = 0; q < kGemms; ++q) {
+      const PermW& p0 = P[kPairs[q][0]];
+      const PermW& p1 = P[kPairs[q][1]];
       const dev::TcOperand* T0 = &Sp->pair[p0.x + o * p0.y];
       const dev::TcOperand* T1 = &Sp->pair[p1.x + o * p1.y];
       const dev::TcOperand* V0 = p0.l2 ? &ops.V2s[p0.z] : &ops.V1s[p0.z];
@@ -192,9 +218,10 @@ void fill_tables(Ctx& c, const TriplesOps& ops, const SplitAmps* Sp, const std::
 
 void upload_tables(Ctx& c, KTables& kt) {
   dev::stream_t s = c.st;
-  if (!kt.ptab.empty()) {
-    kt.ptab_d = reinterpret_cast<int64_t*>(c.alloc((int64_t)kt.ptab.size(), "(T) offset table"));
-    check(dev::h2d(kt.ptab_d, kt.ptab.data(), kt.ptab.size() * 8, s), "h2d");
+  if (!kt.items.empty()) {
+    const size_t bytes = kt.items.size() * sizeof(dev::KbItem);
+    kt.items_d = reinterpret_cast<dev::KbItem*>(c.alloc((int64_t)(bytes / 8), "(T) item table"));
+    check(dev::h2d(kt.items_d, kt.items.data(), bytes, s), "h2d");
   }
   if (!kt.mtab.empty()) {
     kt.mtab_d = reinterpret_cast<unsigned char*>(
@@ -204,50 +231,37 @@ void upload_tables(Ctx& c, KTables& kt) {
 }
 
 // K^{ijk} = P[W] for triplets t0 .. t0+nb-1 into K slots 0 .. nb-1 (FP64 or
-// FP32), one launch per GEMM kind.
-void build_K_batch(Ctx& c, const TriplesOps& ops, const double* T, const SplitAmps* Sp,
+// FP32), one launch per K orientation.
+void build_K_batch(Ctx& c, const TriplesOps& ops, const FpAmps& F, const SplitAmps* Sp,
                    const KTables& kt, int64_t nt, int64_t t0, int nb, void* K, int64_t kstride,
                    int64_t vp) {
-  const int64_t o = c.no, v = c.nv, v2 = v * v, o2 = o * o;
+  const int64_t o = c.no, v = c.nv, v2 = v * v;
   dev::stream_t s = c.st;
   PermW P[6];
   perm_table(0, 0, 0, v, vp, P);  // output maps and layouts do not depend on i, j, k
   if (!ops.mixed) {
-    auto tab = [&](int q) { return kt.ptab_d + (q * nt + t0) * 5; };
-    // The vvvo GEMMs (M = v, N = v^2, K = v): one GEMM per triplet, its
-    // operands placed from the host copy of the offset table; each fills the
-    // GPU by itself (v/64 x v^2/64 tiles) and runs on the TMA-staged kernel
-    // through K's index map.  Per K element the six contributions still add in
-    // the order q = 0..5.
-    for (int q = 0; q < 6; ++q)
-      for (int it = 0; it < nb; ++it) {
-        const int64_t* e = kt.ptab.data() + (q * nt + t0 + it) * 5;
-        dev::Gemm g;
-        g.m = v; g.n = v2; g.k = v; g.batch = 1; g.alpha = 1.0; g.beta = q ? 1.0 : 0.0;
-        g.A = T + e[0]; g.sam = 1; g.sak = v;
-        g.B = (P[q].l2 ? ops.V2 : ops.V1) + e[1]; g.sbk = v2; g.sbn = 1;
-        g.C = (double*)K + e[2];
-        g.scm = P[q].scm; g.scn = P[q].scn; g.dn = P[q].dn; g.scn2 = P[q].scn2;
-        g.mapped_tma = true;
-        check(dev::gemm_strided(s, g), "W vvvo");
-      }
-    dev::Gemm g;
-    g.k = 2 * o; g.kseg = o; g.alpha = -1.0; g.beta = 1.0; g.C = (double*)K; g.batch = nb;
-    // (1) rows (a,b), columns c
-    g.m = v2; g.n = v; g.A = T; g.sam = 1; g.sak = v2 * o; g.A1 = T; g.sak1 = v2;
-    g.B = ops.On; g.sbk = 1; g.sbn = o2; g.B1 = ops.On; g.sbk1 = 1;
-    g.scm = 1; g.scn = v2; g.dn = 0; g.scn2 = 0; g.ptab = tab(6);
-    check(dev::gemm_strided(s, g), "W ovoo 1");
-    // (2) rows b, columns (a,c)
-    g.m = v; g.n = v2; g.A = ops.On; g.sam = o2; g.sak = 1; g.A1 = ops.On; g.sak1 = 1;
-    g.B = T; g.sbk = v2 * o; g.sbn = 1; g.B1 = T; g.sbk1 = v2;
-    g.scm = v; g.scn = 1; g.dn = v; g.scn2 = v2; g.ptab = tab(7);
-    check(dev::gemm_strided(s, g), "W ovoo 2");
-    // (3) rows (b,c), columns a
-    g.m = v2; g.n = v; g.A = T; g.sam = 1; g.sak = v2; g.A1 = T; g.sak1 = v2 * o;
-    g.B = ops.On; g.sbk = 1; g.sbn = o2; g.B1 = ops.On; g.sbk1 = 1;
-    g.scm = v; g.scn = 1; g.dn = 0; g.scn2 = 0; g.ptab = tab(8);
-    check(dev::gemm_strided(s, g), "W ovoo 3");
+    const int64_t v2p = ops.v2p, vq = ops.vq;
+    const dev::KbOperand V1{ops.V1, v2, v2p, o, v2p * v}, V2{ops.V2, v2, v2p, o, v2p * v};
+    const dev::KbOperand Tp{F.pair, v, vq, o * o, vq * v};
+    const dev::KbOperand G{F.ab, v2, v2p * o, o, v2p};  // T2[:,:,x,l]: k = l, item x
+    const dev::KbOperand C{F.ab, v2, v2p, o, v2p * o};  // T2[:,:,l,x]
+    const dev::KbOperand On{ops.On, v, vq, o * o, vq * o};
+    // T2 slices of the two ovoo segments: rows (b,c), (a,c) and (a,b) of K
+    const dev::KbOperand* ab[kGemms][2] = {{&C, &G}, {&G, &C}, {&G, &C}};
+    for (int q = 0; q < kGemms; ++q) {
+      const PermW &p0 = P[kPairs[q][0]], &p1 = P[kPairs[q][1]];
+      dev::KbGemm g;
+      g.m = v2; g.n = v; g.nseg = 4;
+      g.k[0] = g.k[1] = v; g.k[2] = g.k[3] = o;
+      g.A[0] = p0.l2 ? V2 : V1; g.A[1] = p1.l2 ? V2 : V1;
+      g.A[2] = *ab[q][0]; g.A[3] = *ab[q][1];
+      g.B[0] = g.B[1] = Tp; g.B[2] = g.B[3] = On;
+      g.beta = q ? 1.0 : 0.0;
+      g.C = (double*)K;
+      g.scm = p0.scn; g.dm = p0.dn; g.scm2 = p0.scn2; g.scn = p0.scm;
+      g.even_items = kstride % 2 == 0;
+      check(dev::kbuild(s, g, nb, kt.items_d + q * nt + t0), "W");
+    }
     return;
   }
   const size_t mb = dev::tc_maps_bytes();
@@ -257,9 +271,8 @@ void build_K_batch(Ctx& c, const TriplesOps& ops, const double* T, const SplitAm
   const dev::TcOperand* Vp = &ops.V1s[0];
   const dev::TcOperand* Op = &ops.Ons[0];
   const dev::TcOperand* Gp = &Sp->G[0];
-  const int pairs[3][2] = {{0, 2}, {1, 4}, {3, 5}};
-  for (int q = 0; q < 3; ++q) {
-    const PermW& p0 = P[pairs[q][0]];
+  for (int q = 0; q < kGemms; ++q) {
+    const PermW& p0 = P[kPairs[q][0]];
     dev::TcGemm g;
     g.alpha = 1.0; g.beta = q ? 1.0 : 0.0; g.C = K; g.f32 = true;
     if (p0.scm == 1) {  // rows a', columns (b',c'); ovoo rows a
@@ -291,8 +304,9 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
 
   TriplesOps ops;
   ops.mixed = mixed;
+  ops.vq = (v + 1) / 2 * 2;
+  ops.v2p = (v2 + 1) / 2 * 2;
   double* On = c.alloc(o * o * o * v, "(T) ovoo");
-  ops.On = On;
   Contractor con = c.con();
   con(1.0, c.Boo, "ljQ", c.Bvo, "ckQ", 0.0, On, "ljck");
   // vvvo[b,c,d,k] = (bd|ck): per k, a GEMM batched over d; [c,b,d,k] by permutation
@@ -307,14 +321,30 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
     check(dev::gemm_strided(s, g), "vvvo");
   };
   if (!mixed) {
-    double* V1 = c.alloc(v3 * o, "(T) vvvo [b,c,d,k]");
-    double* V2 = c.alloc(v3 * o, "(T) vvvo [c,b,d,k]");
+    const int64_t slab = ops.v2p * v;
+    double* V1 = c.alloc(slab * o, "(T) vvvo [b,c,d,k]");
+    double* V2 = c.alloc(slab * o, "(T) vvvo [c,b,d,k]");
+    double* Onp = c.alloc(ops.vq * o * o * o, "(T) -ovoo");
+    const bool pad = ops.v2p != v2;  // dense slabs first, then copies in the even pitch
+    double* Vt = pad ? c.alloc(2 * v3, "(T) vvvo slabs") : nullptr;
     for (int64_t kk = 0; kk < o; ++kk) {
-      build_v(kk, V1 + v3 * kk);
-      check(dev::permute(s, 3, d3, swap01, 1.0, V1 + v3 * kk, 0.0, V2 + v3 * kk), "vvvo perm");
+      double* d1 = pad ? Vt : V1 + slab * kk;
+      double* d2 = pad ? Vt + v3 : V2 + slab * kk;
+      build_v(kk, d1);
+      check(dev::permute(s, 3, d3, swap01, 1.0, d1, 0.0, d2), "vvvo perm");
+      if (!pad) continue;
+      check(dev::geam(s, v2, v, 1.0, d1, v2, 0.0, V1 + slab * kk, ops.v2p), "pad vvvo");
+      check(dev::geam(s, v2, v, 1.0, d2, v2, 0.0, V2 + slab * kk, ops.v2p), "pad vvvo");
     }
+    // -ovoo as [c,l,j,k]
+    const int64_t dl[4] = {o, o, v, o};
+    const int pl[4] = {2, 0, 1, 3};
+    double* Oc = c.alloc(o * o * o * v, "(T) ovoo [c,l,j,k]");
+    check(dev::permute(s, 4, dl, pl, -1.0, On, 0.0, Oc), "-ovoo");
+    check(dev::geam(s, v, o * o * o, 1.0, Oc, v, 0.0, Onp, ops.vq), "-ovoo pitch");
     ops.V1 = V1;
     ops.V2 = V2;
+    ops.On = Onp;
   } else {
     const size_t evs = dev::tc_operand_elems(v2, v, kTriplesSlices);
     const size_t eos = dev::tc_operand_elems(v, o, kTriplesSlices);
@@ -357,6 +387,11 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
     con.permute(1.0 / 3.0, U2, "baij", 1.0, U2c, "abij");
   }
   SplitAmps ST, SU;
+  FpAmps FT, FU;
+  if (!mixed) {
+    FT = fp_amps(c, c.T2(), ops);
+    if (lam) FU = fp_amps(c, U2c, ops);
+  }
   if (mixed) {
     split_amps(c, c.T2(), ST);
     if (lam) split_amps(c, U2c, SU);
@@ -480,8 +515,8 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
       if (bi == 1) check(dev::graph_capture_begin(s), "graph capture");
       const int64_t t0 = bi * NB;
       const int nb = (int)std::min<int64_t>(NB, nt - t0);
-      build_K_batch(c, ops, c.T2(), &ST, KT, nt, t0, nb, K, kstride, vp);
-      if (lam) build_K_batch(c, ops, U2c, &SU, KUt, nt, t0, nb, KU, kstride, vp);
+      build_K_batch(c, ops, FT, &ST, KT, nt, t0, nb, K, kstride, vp);
+      if (lam) build_K_batch(c, ops, FU, &SU, KUt, nt, t0, nb, KU, kstride, vp);
       if (mixed)
         check(dev::triples_energy_f32_batched(s, (int)v, (int)vp, nb, NB,
                                               static_cast<const float*>(K),
