@@ -871,18 +871,22 @@ struct PlainChoice {
   int cfg, S;
 };
 
-// The fixed rule: 64x64 tiles, TMA-staged where TMA can address both operands
-// (15-20% faster than cp.async staging on every CCSD shape measured on B200,
-// bitwise the same results); K split when the output covers too few tiles to
-// fill the SMs and K is long enough.
+// The fixed rule: where TMA can address both operands, the TMA configuration
+// and split with the least estimated time (dgemm_tma_rule); else 64x64
+// cp.async tiles, K split when the output covers too few tiles to fill the SMs
+// and K is long enough.
 static PlainChoice default_plain(const Gemm& q, bool tma = true) {
-  const int cfg = (tma && dgemm_tma_usable(q)) ? CFG_TMA : 0;
+  if (tma && dgemm_tma_usable(q)) {
+    int cfg, S;
+    dgemm_tma_rule(q, &cfg, &S);
+    return PlainChoice{CFG_TMA + cfg, S};
+  }
   const int64_t tiles64 = ((q.m + 63) / 64) * ((q.n + 63) / 64);
   if (q.batch == 1 && tiles64 < 148 && q.k >= 512) {
     int64_t S = std::min<int64_t>((2 * 148 + tiles64 - 1) / tiles64, q.k / 256);
-    return PlainChoice{cfg, (int)std::max<int64_t>(2, std::min<int64_t>(S, 64))};
+    return PlainChoice{0, (int)std::max<int64_t>(2, std::min<int64_t>(S, 64))};
   }
-  return PlainChoice{cfg, 1};
+  return PlainChoice{0, 1};
 }
 
 static int launch_plain(stream_t s, const GemmArgs& g, const Gemm& q, PlainChoice c) {
@@ -937,8 +941,7 @@ static int plain_gemm(stream_t s, const GemmArgs& g, const Gemm& q) {
     const PlainChoice d = default_plain(q, false);
     if (q.batch == 1 && q.k >= 512) {
       // split counts around the rule's and the small ones that round the
-      // CTA count up to whole waves; long contractions also try the
-      // 128x128 TMA tile split
+      // CTA count up to whole waves
       for (int S : {d.S, 2 * d.S, d.S / 2, 2, 3, 4, 6, 8, 12, 16})
         if (S >= 2 && S <= 64 && q.k / S >= 64) {
           auto add = [&](int cfg) {
@@ -947,8 +950,8 @@ static int plain_gemm(stream_t s, const GemmArgs& g, const Gemm& q) {
             cand.push_back({cfg, S});
           };
           add(0);
-          if (tma) add(CFG_TMA);
-          if (tma && q.k >= 4096) add(CFG_TMA + 3);
+          if (tma)
+            for (int t = 0; t < DTMA_CONFIGS; ++t) add(CFG_TMA + t);
         }
     }
     // tune_pick restores the output region it is given: the m x n columns of

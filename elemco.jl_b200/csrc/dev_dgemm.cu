@@ -5,8 +5,8 @@
 // K (grid z = K slice, partial products into the stream's split-K buffer,
 // summed in a fixed order by splitk_reduce).  tcgen05 has no FP64 kind, so the
 // products run on the FP64 MMA pipe (mma.sync m8n8k4 f64).  What the Tensor
-// Memory Accelerator takes over is the operand staging: one thread issues the
-// TMA copies of a 16-deep k-slab of the A and B tiles into a ring of STAGES
+// Memory Accelerator takes over is the operand staging: a producer warp issues
+// the TMA copies of a 16-deep k-slab of the A and B tiles into a ring of STAGES
 // shared-memory stages (128-byte swizzle, mbarrier completion), so the MMA
 // warps spend no instructions on address arithmetic or copies, and each warp
 // releases a stage through an `empty` mbarrier instead of a block barrier
@@ -54,7 +54,7 @@ template <int BM, int BN, int WM, int WN, int STAGES>
 struct DCfg {
   static constexpr int WARPS_M = BM / WM;
   static constexpr int WARPS = (BM / WM) * (BN / WN);
-  static constexpr int THREADS = WARPS * 32;
+  static constexpr int THREADS = WARPS * 32 + 32;  // and the producer warp
   static constexpr int A_BYTES = BM * DK * 8;
   static constexpr int B_BYTES = BN * DK * 8;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
@@ -121,11 +121,28 @@ __global__ void __launch_bounds__(DCfg<BM, BN, WM, WN, STAGES>::THREADS, MINB)
     }
   };
 
-  int issued = 0;
-  if (tid == 0) {
-    asm volatile("prefetch.tensormap [%0];\n" ::"l"((uint64_t)&ma) : "memory");
-    asm volatile("prefetch.tensormap [%0];\n" ::"l"((uint64_t)&mb) : "memory");
-    for (; issued < KT && issued < STAGES; ++issued) issue(issued);
+  if (warp == Cfg::WARPS) {
+    // The producer warp: a warp of its own keeps the copies' address
+    // arithmetic, waits and issue off the MMA warps, which at one block an SM
+    // had been what the others waited for (684^3, 64x64 tiles of four warps:
+    // 51 us with thread 0 of an MMA warp issuing, 37 us with this warp).
+    if (lane == 0) {
+      asm volatile("prefetch.tensormap [%0];\n" ::"l"((uint64_t)&ma) : "memory");
+      asm volatile("prefetch.tensormap [%0];\n" ::"l"((uint64_t)&mb) : "memory");
+      int t = 0;
+      for (; t < KT; ++t) {
+        if (t >= STAGES &&
+            !mbar_wait(&empty[t % STAGES], (uint32_t)((t / STAGES - 1) & 1), wait_ns)) {
+          atomicExch(&g_dtma_error, 1);
+          break;
+        }
+        issue(t);
+      }
+      // nothing of this CTA's may be in flight when it exits
+      for (int u = t > STAGES ? t - STAGES : 0; u < t; ++u)
+        mbar_wait(&full[u % STAGES], (uint32_t)((u / STAGES) & 1), WAIT_NS);
+    }
+    return;
   }
 
   const int g = lane >> 2, t4 = lane & 3;
@@ -139,25 +156,20 @@ __global__ void __launch_bounds__(DCfg<BM, BN, WM, WN, STAGES>::THREADS, MINB)
 #pragma unroll
     for (int j = 0; j < NTL; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
-  bool ok = true;
-  int consumed = 0;
   for (int t = 0; t < KT; ++t) {
     const int s = t % STAGES;
     const bool ready = mbar_wait(&full[s], (uint32_t)((t / STAGES) & 1), wait_ns);
     if (!__all_sync(~0u, ready)) {
-      ok = false;
-      break;
+      if (lane == 0) atomicExch(&g_dtma_error, 1);
+      return;
     }
-    consumed = t + 1;
     // Release the stage of tile t-1 only now, past the wait on tile t: the
     // MMAs of tile t-1 stand before that wait in program order and take its
     // fragments as register operands, so every shared-memory read of that
     // stage has returned.  Releasing it right behind the loads, before the
     // MMAs that wait for them, let the refill overwrite rows that a load still
     // queued behind a neighbouring CTA's epilogue had yet to read (10-15% of
-    // the beta = 1 K builds at v = 318 came out with wrong elements).  The
-    // later release costs nothing: 4096^3 runs at 34.5 instead of
-    // 31.8 TF/s (both operands contiguous along k, 64x64 tiles).
+    // the beta = 1 K builds at v = 318 came out with wrong elements).
     if (t >= 1 && lane == 0) mbar_arrive(&empty[(t - 1) % STAGES]);
     const double* As = (const double*)(smem + s * Cfg::STAGE_BYTES);
     const double* Bs = (const double*)(smem + s * Cfg::STAGE_BYTES + Cfg::A_BYTES);
@@ -173,28 +185,6 @@ __global__ void __launch_bounds__(DCfg<BM, BN, WM, WN, STAGES>::THREADS, MINB)
 #pragma unroll
         for (int j = 0; j < NTL; ++j) dmma884(acc[i][j], af[i], bf[j]);
     }
-    // thread 0 refills the stage of tile t-1 once every warp has released it
-    bool refill_ok = true;
-    if (tid == 0 && t >= 1 && issued < KT) {
-      const int tp = t - 1;
-      if (mbar_wait(&empty[tp % STAGES], (uint32_t)((tp / STAGES) & 1), wait_ns))
-        issue(issued++);
-      else
-        refill_ok = false;
-    }
-    if (!__all_sync(~0u, refill_ok)) {
-      ok = false;
-      break;
-    }
-  }
-  if (!ok) {
-    if (lane == 0) atomicExch(&g_dtma_error, 1);
-    // nothing of this CTA's may be in flight when it exits: thread 0 waits
-    // (bounded) for the tiles it issued that no wait has seen complete
-    if (tid == 0)
-      for (int t = consumed; t < issued; ++t)
-        mbar_wait(&full[t % STAGES], (uint32_t)((t / STAGES) & 1), WAIT_NS);
-    return;
   }
 
   double* C = out.C + (int64_t)z * out.scb;
@@ -275,20 +265,41 @@ int launch_dtma(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap& mb, c
 typedef int (*DtmaLaunch)(cudaStream_t, const CUtensorMap&, const CUtensorMap&, const DOut&,
                           int64_t, int64_t, int, int);
 
-// Tile configurations: 0: 64x64 (4 warps of 32x32, 4 stages, 3 CTAs/SM);
-// 1: 128x64 (4 warps of 64x32, 4 stages, 2 CTAs/SM); 2: 64x128 (4 warps of
-// 32x64, 4 stages, 2 CTAs/SM); 3: 128x128 (8 warps of 64x32, 4 stages).
+// Tile configurations (blocks an SM, MMA warps): 0: 64x64 (3, four of 32x32);
+// 1: 32x32 (4, four of 16x16); 2: 64x32 (3, four of 32x16); 3: 64x64 (2, eight
+// of 32x16).  Measured us, configurations 0..3 (4224^3 is 35.0, 32.6, 34.8 and
+// 34.3 TF/s; a 128x128 tile of eight warps took 5461 us, 128x64 of four 4622):
+//   4224^3           4318  4633  4337  4399
+//   1216^3            139   122   115   135
+//   684^3              37    33    31    29
+//   400^3              23    12    16    18
+//   256x256x5776      270   104   163   207
+// Large outputs want few operand reads per MMA (0), outputs of about a tile
+// per SM the eight warps that hide each other's latency (3), smaller ones
+// more blocks (2, 1).
 template <bool AKF, bool BKF>
 DtmaLaunch pick(int cfg) {
   switch (cfg) {
-    case 1: return launch_dtma<128, 64, 64, 32, 4, 2, AKF, BKF>;
-    case 2: return launch_dtma<64, 128, 32, 64, 4, 2, AKF, BKF>;
-    case 3: return launch_dtma<128, 128, 64, 32, 4, 1, AKF, BKF>;
+    case 1: return launch_dtma<32, 32, 16, 16, 6, 4, AKF, BKF>;
+    case 2: return launch_dtma<64, 32, 32, 16, 4, 3, AKF, BKF>;
+    case 3: return launch_dtma<64, 64, 32, 16, 4, 2, AKF, BKF>;
     default: return launch_dtma<64, 64, 32, 32, 4, 3, AKF, BKF>;
   }
 }
-constexpr int CFG_BM[DTMA_CONFIGS] = {64, 128, 64, 128};
-constexpr int CFG_BN[DTMA_CONFIGS] = {64, 64, 128, 128};
+constexpr int CFG_BM[DTMA_CONFIGS] = {64, 32, 64, 64};
+constexpr int CFG_BN[DTMA_CONFIGS] = {64, 32, 32, 64};
+
+// Whole calls: a CCSD iteration of o=24, v=318 662 -> 626 ms (33.8 TF/s over
+// its FP64 GEMMs; 628 ms with the shapes tuned one by one for the earlier
+// kernel), of o=12, v=57 2.53 -> 2.18 ms, Lambda residual of o=16, v=76 9.15
+// -> 7.7 ms.
+
+// Share of the FP64 MMA rate that r resident blocks of a configuration reach
+// on their SM (from the timings above and 1024^3, 2048^3).
+constexpr int CFG_OCC[DTMA_CONFIGS] = {3, 4, 3, 2};
+constexpr double CFG_EFF[DTMA_CONFIGS][4] = {
+    {0.70, 0.88, 0.93, 0.93}, {0.45, 0.68, 0.73, 0.77}, {0.58, 0.80, 0.90, 0.90},
+    {0.88, 0.94, 0.94, 0.94}};
 
 }  // namespace
 
@@ -300,6 +311,39 @@ bool dgemm_tma_usable(const Gemm& q) {
   bool kf;
   return operand_map(&m, &kf, q.A, q.m, q.k, q.sam, q.sak, q.batch, q.sab, 64) &&
          operand_map(&m, &kf, q.B, q.n, q.k, q.sbn, q.sbk, q.batch, q.sbb, 64);
+}
+
+// Estimated time (us) of configuration cfg with K in S slices: the busiest
+// SM's blocks at the rate its residents reach (64x64x16 multiply-adds take
+// 0.521 us of an SM), a launch, and the reduction of the partial products.
+static double dgemm_tma_cost(const Gemm& q, int cfg, int64_t S) {
+  const int64_t bm = CFG_BM[cfg], bn = CFG_BN[cfg];
+  const int64_t kt = ((q.k + S - 1) / S + DK - 1) / DK;
+  const int64_t ctas = ((q.m + bm - 1) / bm) * ((q.n + bn - 1) / bn) * q.batch * S;
+  const int64_t x = (ctas + 147) / 148;
+  const double eff = CFG_EFF[cfg][std::min<int64_t>(x, CFG_OCC[cfg]) - 1];
+  double t = 3.0 + 0.521 * (double)(bm * bn) / 4096.0 * (double)(kt * x) / eff;
+  if (S > 1) t += 3.0 + 8.0e-6 * (double)(S + 1) * (double)q.m * (double)q.n / 4.0;
+  return t;
+}
+
+void dgemm_tma_rule(const Gemm& q, int* cfg, int* nsplit) {
+  *cfg = 0;
+  *nsplit = 1;
+  double best = -1.0;
+  for (int c = 0; c < DTMA_CONFIGS; ++c) {
+    if ((q.n + CFG_BN[c] - 1) / CFG_BN[c] > 65535) continue;
+    for (int64_t S : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64}) {
+      // partial products within 128 MiB of scratch
+      if (S > 1 && (q.batch != 1 || q.k / S < 64 || S * q.m * q.n > ((int64_t)1 << 24))) break;
+      const double t = dgemm_tma_cost(q, c, S);
+      if (best < 0.0 || t < best) {
+        best = t;
+        *cfg = c;
+        *nsplit = (int)S;
+      }
+    }
+  }
 }
 
 int dgemm_tma(stream_t s, const Gemm& q, int cfg, int nsplit) {

@@ -61,11 +61,13 @@ int gemm_strided(stream_t s, const Gemm& g);
 // FP64 GEMM with TMA-staged operands (dev_dgemm.cu): C with unit row stride,
 // each operand contiguous along its row index or along k with its other
 // strides even (16-byte multiples) and a 16-byte-aligned base.  cfg selects the
-// tile (0: 64x64, 1: 128x64, 2: 64x128, 3: 128x128); nsplit > 1 (batch 1) cuts
-// K into slices summed in a fixed order.  Returns -1, launching nothing, when
-// TMA cannot address an operand; dgemm_tma_usable tells beforehand.
+// tile (0: 64x64, 1: 32x32, 2: 64x32, 3: 64x64 with eight MMA warps); nsplit > 1
+// (batch 1) cuts K into slices summed in a fixed order.  Returns -1, launching
+// nothing, when TMA cannot address an operand; dgemm_tma_usable tells
+// beforehand.  dgemm_tma_rule picks cfg and nsplit by estimated time.
 constexpr int DTMA_CONFIGS = 4;
 bool dgemm_tma_usable(const Gemm& q);
+void dgemm_tma_rule(const Gemm& q, int* cfg, int* nsplit);
 int dgemm_tma(stream_t s, const Gemm& q, int cfg, int nsplit);
 // Time-out code of the TMA FP64 GEMM's bounded waits since the last call
 // (0 = none); reading clears it.
