@@ -925,7 +925,79 @@ static int launch_plain(stream_t s, const GemmArgs& g, const Gemm& q, PlainChoic
   }
 }
 
-static int plain_gemm(stream_t s, const GemmArgs& g, const Gemm& q) {
+// Operands that TMA cannot address (an odd pitch, as every tensor has one at
+// an odd virtual count, or a base off 16 bytes) are copied into even pitches
+// first where that pays: the estimated time of the TMA kernel and the copies
+// (an operand element is read and written once, at about 4 TB/s, against 2 m or
+// 2 n flops) is below the cp.async kernel's, which reaches 45-66% of the FP64
+// MMA rate at one to three blocks an SM.  FP64 GEMMs of a DCSD iteration of
+// o=25, v=169: 61.5 -> 52.4 ms (26.7 -> 31.4 TF/s).
+static bool pack_for_tma(stream_t s, const Gemm& q, Gemm* out) {
+  const int64_t lim = (int64_t)1 << 31;
+  if (q.batch != 1 || q.scm != 1 || q.m >= lim || q.n >= lim || q.k >= lim || dgemm_tma_usable(q))
+    return false;
+  struct Side {
+    const double* X;
+    int64_t ni, si, sk;
+    bool ok, kfast;
+    int64_t rows, len, pitch;
+  };
+  auto side = [&](const double* X, int64_t ni, int64_t si, int64_t sk) {
+    Side d{X, ni, si, sk, false, sk == 1 && (q.k > 1 || si != 1), 0, 0, 0};
+    d.len = d.kfast ? q.k : ni;
+    d.rows = d.kfast ? ni : q.k;
+    const int64_t ld = d.kfast ? si : sk;
+    d.ok = ((uintptr_t)X & 15) == 0 && (d.rows == 1 || (ld > 0 && ld % 2 == 0));
+    d.pitch = (d.len + 1) / 2 * 2;
+    return d;
+  };
+  Side A = side(q.A, q.m, q.sam, q.sak), B = side(q.B, q.n, q.sbn, q.sbk);
+  // one index of each operand has unit stride, and its rows do not overlap
+  for (const Side* d : {&A, &B}) {
+    if ((d->kfast ? d->sk : d->si) != 1) return false;
+    if (!d->ok && (d->kfast ? d->si : d->sk) < d->len) return false;
+  }
+  Gemm t = q;
+  // strides only matter to the estimate through dgemm_tma_rule's sizes
+  int cfg, S;
+  double tma = dgemm_tma_rule(t, &cfg, &S);
+  size_t need = 0;
+  for (const Side* d : {&A, &B})
+    if (!d->ok) {
+      tma += 3.0 + 16.0 * (double)d->rows * (double)d->len / 4.0e6;
+      need += (size_t)(d->rows * d->pitch + 2) * sizeof(double);
+    }
+  const int64_t tiles = ((q.m + 63) / 64) * ((q.n + 63) / 64);
+  const PlainChoice c = default_plain(q, false);
+  const int64_t x = (tiles * c.S + 147) / 148;
+  const double eff = x == 1 ? 0.45 : x == 2 ? 0.6 : 0.66;
+  const double cp = 3.0 + 0.521 * (double)(((q.k + c.S - 1) / c.S + 15) / 16 * x) / eff +
+                    (c.S > 1 ? 3.0 : 0.0);
+  if (tma >= cp) return false;
+  double* buf = (double*)split_scratch(s, need);
+  if (!buf) return false;  // no scratch (stream capture, memory): cp.async takes it as it is
+  for (Side* d : {&A, &B})
+    if (!d->ok) {
+      if (repitch(s, d->len, d->rows, d->X, d->kfast ? d->si : d->sk, buf, d->pitch)) return false;
+      d->X = buf;
+      (d->kfast ? d->si : d->sk) = d->pitch;
+      buf += (d->rows * d->pitch + 1) / 2 * 2;
+    }
+  t.A = A.X; t.sam = A.si; t.sak = A.sk;
+  t.B = B.X; t.sbn = B.si; t.sbk = B.sk;
+  *out = t;
+  return true;
+}
+
+static int plain_gemm(stream_t s, const GemmArgs& g0, const Gemm& q0) {
+  GemmArgs g = g0;
+  Gemm q;
+  if (pack_for_tma(s, q0, &q)) {
+    g.A = q.A; g.sam = q.sam; g.sak = q.sak;
+    g.B = q.B; g.sbk = q.sbk; g.sbn = q.sbn;
+  } else {
+    q = q0;
+  }
   PlainChoice c = default_plain(q);
   const std::string key = "dgemmt " + std::to_string(q.m) + " " + std::to_string(q.n) + " " +
                           std::to_string(q.k) + " " + std::to_string(q.batch) + " " +
@@ -1156,6 +1228,37 @@ int permute(stream_t s, int nd, const int64_t* in_dims, const int* perm, double 
 }
 
 // ---------------------------------------------------------------- elementwise
+
+// A warp copies 128 elements of a row, its four loads in flight together;
+// odd pitches leave no wider alignment than one double.
+__global__ void repitch_kernel(uint32_t n, uint32_t rows, const double* __restrict__ src,
+                               int64_t lds, double* __restrict__ dst, int64_t ldd) {
+  const uint32_t chunks = (n + 127) / 128, lane = threadIdx.x & 31;
+  const uint64_t items = (uint64_t)rows * chunks;
+  for (uint64_t it = blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); it < items;
+       it += (uint64_t)gridDim.x * (blockDim.x >> 5)) {
+    const uint32_t r = (uint32_t)(it / chunks), c = (uint32_t)(it - (uint64_t)r * chunks);
+    const uint32_t x0 = c * 128 + lane;
+    const double* s = src + (int64_t)r * lds + x0;
+    double* d = dst + (int64_t)r * ldd + x0;
+    double v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = x0 + 32 * j < n ? s[32 * j] : 0.0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (x0 + 32 * j < n) d[32 * j] = v[j];
+  }
+}
+
+int repitch(stream_t s, int64_t n, int64_t rows, const double* src, int64_t lds, double* dst,
+            int64_t ldd) {
+  if (n <= 0 || rows <= 0) return 0;
+  if (n >= ((int64_t)1 << 31) || rows >= ((int64_t)1 << 31)) return (int)cudaErrorInvalidValue;
+  const int64_t warps = rows * ((n + 127) / 128);
+  repitch_kernel<<<(unsigned)std::min<int64_t>((warps + 7) / 8, 148 * 16), 256, 0,
+                   (cudaStream_t)s>>>((uint32_t)n, (uint32_t)rows, src, lds, dst, ldd);
+  return launched();
+}
 
 __global__ void axpby_kernel(int64_t n, double alpha, const double* x, double beta, double* y) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;

@@ -327,7 +327,7 @@ static double dgemm_tma_cost(const Gemm& q, int cfg, int64_t S) {
   return t;
 }
 
-void dgemm_tma_rule(const Gemm& q, int* cfg, int* nsplit) {
+double dgemm_tma_rule(const Gemm& q, int* cfg, int* nsplit) {
   *cfg = 0;
   *nsplit = 1;
   double best = -1.0;
@@ -344,6 +344,7 @@ void dgemm_tma_rule(const Gemm& q, int* cfg, int* nsplit) {
       }
     }
   }
+  return best;
 }
 
 int dgemm_tma(stream_t s, const Gemm& q, int cfg, int nsplit) {

@@ -107,7 +107,8 @@ void sync_scalars(Ctx& c, int count) {
 // a-block size of the symmetric ladder: Vblk holds v^2 na (v - a0) doubles.
 static int64_t ladder_na(int64_t nv) {
   const int64_t budget = (int64_t)1 << 28;  // doubles (2 GiB) for one V block
-  int64_t na = (nv + 7) / 8;
+  // an even block start keeps the block's rows of B on 16 bytes for TMA
+  int64_t na = ((nv + 7) / 8 + 1) / 2 * 2;
   na = std::min<int64_t>(na, std::max<int64_t>(1, budget / std::max<int64_t>(nv * nv * nv, 1)));
   return std::max<int64_t>(1, std::min(na, nv));
 }
@@ -347,6 +348,8 @@ void ladder(Ctx& c, const double* Bf, const double* BfT, const double* T2, doubl
   double* Vm = c.ws.get(std::max<int64_t>(ldm * maxpp, 1));
   double* Lp = c.ws.get(maxpp * nijp);
   double* Lm = c.ws.get(std::max<int64_t>(maxpp * nijm, 1));
+  const double* Bl = BfT;  // FP64 V builds read it in an even pitch
+  int64_t ldb = v * v;
   // Mixed precision: the operands shared by every a-block (BfT for the V
   // build, the packed T2 for the contractions) are split into BF16 slices once
   // per call, each block reads row ranges of them; the per-block V+/- are
@@ -379,6 +382,12 @@ void ladder(Ctx& c, const double* Bf, const double* BfT, const double* T2, doubl
     if (mp) check(dev::tc_split(s, Ts, nijp, ncdp, ldp, 1, NSL, pTs, &oTs), "split T+");
     if (mm) check(dev::tc_split(s, Ta, nijm, ncdm, ldm, 1, NSL, pTa, &oTa), "split T-");
   }
+  if (!mv && v % 2 == 1) {
+    ldb = v * v + 1;
+    double* t = c.ws.get(ldb * Q);
+    check(dev::repitch(s, v * v, Q, BfT, v * v, t, ldb), "pad BfT");
+    Bl = t;
+  }
   const bool fused = mp && mm;  // V+/- packed into BF16 slices directly
   const bool vf32 = fused && mv && Q <= dev::TC_ACC_K;
   for (auto& b : c.lblocks) {
@@ -393,8 +402,8 @@ void ladder(Ctx& c, const double* Bf, const double* BfT, const double* T2, doubl
       g.C = V; g.scm = 1; g.scn = v * b.na; g.f32 = vf32;
       check(dev::tc_gemm(s, g), "gemm ladder V");
     } else {
-      check(dev::gemm(s, 'N', 'T', v * b.na, v * nb, Q, 1.0, BfT + v * b.a0, v * v,
-                      BfT + v * b.a0, v * v, 0.0, V, v * b.na),
+      check(dev::gemm(s, 'N', 'T', v * b.na, v * nb, Q, 1.0, Bl + v * b.a0, ldb, Bl + v * b.a0,
+                      ldb, 0.0, V, v * b.na),
             "gemm ladder V");
     }
     const int* pairs = c.pairs + 2 * b.poff;

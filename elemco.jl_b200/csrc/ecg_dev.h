@@ -67,7 +67,8 @@ int gemm_strided(stream_t s, const Gemm& g);
 // beforehand.  dgemm_tma_rule picks cfg and nsplit by estimated time.
 constexpr int DTMA_CONFIGS = 4;
 bool dgemm_tma_usable(const Gemm& q);
-void dgemm_tma_rule(const Gemm& q, int* cfg, int* nsplit);
+// Returns that time (us).
+double dgemm_tma_rule(const Gemm& q, int* cfg, int* nsplit);
 int dgemm_tma(stream_t s, const Gemm& q, int cfg, int nsplit);
 // Time-out code of the TMA FP64 GEMM's bounded waits since the last call
 // (0 = none); reading clears it.
@@ -183,6 +184,10 @@ int tc_gemm_batched(stream_t s, const TcGemm& g, int batch, const void* mtab, in
 // perm[d].  beta == 0 never reads out.
 int permute(stream_t s, int nd, const int64_t* in_dims, const int* perm, double alpha,
             const double* in, double beta, double* out);
+
+// dst[x + ldd*r] = src[x + lds*r], x < n, r < rows: a copy between row pitches.
+int repitch(stream_t s, int64_t n, int64_t rows, const double* src, int64_t lds, double* dst,
+            int64_t ldd);
 
 // y = alpha * x + beta * y   (beta == 0: y = alpha * x)
 int axpby(stream_t s, int64_t n, double alpha, const double* x, double beta, double* y);

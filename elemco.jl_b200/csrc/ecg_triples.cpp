@@ -132,8 +132,8 @@ FpAmps fp_amps(Ctx& c, const double* T, const TriplesOps& ops) {
   if (v % 2 == 0 && ((uintptr_t)T & 15) == 0) return f;
   double* p = c.alloc(ops.vq * v * o * o, "(T) T^{xy} padded");
   double* ab = c.alloc(ops.v2p * o * o, "(T) T2 padded");
-  check(dev::geam(c.st, v, v * o * o, 1.0, T, v, 0.0, p, ops.vq), "pad T^{xy}");
-  check(dev::geam(c.st, v2, o * o, 1.0, T, v2, 0.0, ab, ops.v2p), "pad T2");
+  check(dev::repitch(c.st, v, v * o * o, T, v, p, ops.vq), "pad T^{xy}");
+  check(dev::repitch(c.st, v2, o * o, T, v2, ab, ops.v2p), "pad T2");
   f.pair = p;
   f.ab = ab;
   return f;
@@ -333,15 +333,15 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
       build_v(kk, d1);
       check(dev::permute(s, 3, d3, swap01, 1.0, d1, 0.0, d2), "vvvo perm");
       if (!pad) continue;
-      check(dev::geam(s, v2, v, 1.0, d1, v2, 0.0, V1 + slab * kk, ops.v2p), "pad vvvo");
-      check(dev::geam(s, v2, v, 1.0, d2, v2, 0.0, V2 + slab * kk, ops.v2p), "pad vvvo");
+      check(dev::repitch(s, v2, v, d1, v2, V1 + slab * kk, ops.v2p), "pad vvvo");
+      check(dev::repitch(s, v2, v, d2, v2, V2 + slab * kk, ops.v2p), "pad vvvo");
     }
     // -ovoo as [c,l,j,k]
     const int64_t dl[4] = {o, o, v, o};
     const int pl[4] = {2, 0, 1, 3};
     double* Oc = c.alloc(o * o * o * v, "(T) ovoo [c,l,j,k]");
     check(dev::permute(s, 4, dl, pl, -1.0, On, 0.0, Oc), "-ovoo");
-    check(dev::geam(s, v, o * o * o, 1.0, Oc, v, 0.0, Onp, ops.vq), "-ovoo pitch");
+    check(dev::repitch(s, v, o * o * o, Oc, v, Onp, ops.vq), "-ovoo pitch");
     ops.V1 = V1;
     ops.V2 = V2;
     ops.On = Onp;
