@@ -255,6 +255,7 @@ struct GemmArgs {
   double alpha, beta;
   int a_kfast, b_nfast;  // loader thread order follows the unit-stride index
   int64_t klast;         // split-K: depth of the last z-slice (0 = all slices use k)
+  int64_t tri = 0;       // Gemm::tri
 };
 
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool pred) {
@@ -335,6 +336,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, BK, WM, WN, STAGES>::THREADS, 
   double* C = g.C + bz * g.scb;
   const int64_t m0 = (int64_t)blockIdx.x * BM;
   const int64_t n0 = (int64_t)blockIdx.y * BN;
+  if (g.tri > 0 && (n0 + BN - 1) / g.tri < m0 / g.tri) return;
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
   const int wm0 = (warp % Cfg::WARPS_M) * WM;
@@ -811,12 +813,13 @@ int gemm_strided(stream_t s, const Gemm& q) {
   if (!g_timing || q.m <= 0 || q.n <= 0 || q.batch <= 0 || q.k <= 0) return gemm_launch(s, q);
   const int slot = ktime_begin(s, KT_DGEMM);
   int r = gemm_launch(s, q);
-  ktime_end(s, KT_DGEMM, slot, 2.0 * (double)q.m * (double)q.n * (double)q.k * (double)q.batch);
+  ktime_end(s, KT_DGEMM, slot, 2.0 * (double)q.m * (double)q.n * (double)q.k * (double)q.batch * gemm_kept(q));
   return r;
 }
 
 static int gemm_launch(stream_t s, const Gemm& q) {
   if (q.m <= 0 || q.n <= 0 || q.batch <= 0) return 0;
+  if (q.tri > 0 && (q.batch != 1 || q.beta != 0.0)) return (int)cudaErrorInvalidValue;
   if ((q.n + 63) / 64 > 65535 && (q.m + 63) / 64 <= 65535) {
     // more column tiles than the grid's y extent: C^T = B^T A^T puts the long
     // dimension on the grid's x axis
@@ -833,6 +836,7 @@ static int gemm_launch(stream_t s, const Gemm& q) {
     t.sbb = q.sab;
     t.scm = q.scn;
     t.scn = q.scm;
+    t.tri = 0;  // the transposed triangle is computed whole
     return gemm_launch(s, t);
   }
   if (q.k <= 0 || q.alpha == 0.0) {
@@ -857,7 +861,7 @@ static int gemm_launch(stream_t s, const Gemm& q) {
   }
   GemmArgs g{q.A, q.B, q.C, q.m, q.n, q.k, q.sam, q.sak, q.sab, q.sbk, q.sbn, q.sbb,
              q.scm, q.scn, q.scb, q.alpha, q.beta, (q.sam != 1 && q.sak == 1) ? 1 : 0,
-             (q.sbk != 1 && q.sbn == 1) ? 1 : 0, 0};
+             (q.sbk != 1 && q.sbn == 1) ? 1 : 0, 0, q.tri};
   return plain_gemm(s, g, q);
 }
 
@@ -896,7 +900,7 @@ static int launch_plain(stream_t s, const GemmArgs& g, const Gemm& q, PlainChoic
     if (e != -1) return e;
     c = default_plain(q, false);  // TMA cannot address an operand
   }
-  if (c.S > 1 && q.batch == 1) {
+  if (c.S > 1 && q.batch == 1 && q.tri == 0) {
     int64_t kc = (q.k + c.S - 1) / c.S;
     kc = (kc + 15) / 16 * 16;
     const int64_t S = (q.k + kc - 1) / kc;

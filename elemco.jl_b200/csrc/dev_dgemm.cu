@@ -69,6 +69,7 @@ struct DOut {
   double* C;
   int64_t m, n, scn, scb;
   double alpha, beta;
+  int tri = 0;  // > 0: blocks whose elements all have j / tri < i / tri do nothing
 };
 
 template <int BM, int BN, int WM, int WN, int STAGES, int MINB, bool AKF, bool BKF>
@@ -86,6 +87,7 @@ __global__ void __launch_bounds__(DCfg<BM, BN, WM, WN, STAGES>::THREADS, MINB)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int z = blockIdx.z;
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+  if (out.tri > 0 && (n0 + BN - 1) / out.tri < m0 / out.tri) return;
   const int64_t kbeg = split ? (int64_t)z * kslice : 0;
   const int64_t kend = split ? (kbeg + kslice < k ? kbeg + kslice : k) : k;
   const int KT = kend > kbeg ? (int)((kend - kbeg + DK - 1) / DK) : 0;
@@ -319,7 +321,8 @@ bool dgemm_tma_usable(const Gemm& q) {
 static double dgemm_tma_cost(const Gemm& q, int cfg, int64_t S) {
   const int64_t bm = CFG_BM[cfg], bn = CFG_BN[cfg];
   const int64_t kt = ((q.k + S - 1) / S + DK - 1) / DK;
-  const int64_t ctas = ((q.m + bm - 1) / bm) * ((q.n + bn - 1) / bn) * q.batch * S;
+  int64_t ctas = ((q.m + bm - 1) / bm) * ((q.n + bn - 1) / bn) * q.batch * S;
+  if (q.tri > 0) ctas = (int64_t)((double)ctas * gemm_kept(q)) + 1;
   const int64_t x = (ctas + 147) / 148;
   const double eff = CFG_EFF[cfg][std::min<int64_t>(x, CFG_OCC[cfg]) - 1];
   double t = 3.0 + 0.521 * (double)(bm * bn) / 4096.0 * (double)(kt * x) / eff;
@@ -335,7 +338,7 @@ double dgemm_tma_rule(const Gemm& q, int* cfg, int* nsplit) {
     if ((q.n + CFG_BN[c] - 1) / CFG_BN[c] > 65535) continue;
     for (int64_t S : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64}) {
       // partial products within 128 MiB of scratch
-      if (S > 1 && (q.batch != 1 || q.k / S < 64 || S * q.m * q.n > ((int64_t)1 << 24))) break;
+      if (S > 1 && (q.batch != 1 || q.tri > 0 || q.k / S < 64 || S * q.m * q.n > ((int64_t)1 << 24))) break;
       const double t = dgemm_tma_cost(q, c, S);
       if (best < 0.0 || t < best) {
         best = t;
@@ -350,6 +353,7 @@ double dgemm_tma_rule(const Gemm& q, int* cfg, int* nsplit) {
 int dgemm_tma(stream_t s, const Gemm& q, int cfg, int nsplit) {
   if (cfg < 0 || cfg >= DTMA_CONFIGS) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)s;
+  if (q.tri > 0) nsplit = 1;  // the reduction of partial products covers all of C
   if (q.scm != 1 || (nsplit > 1 && q.batch != 1)) return (int)cudaErrorInvalidValue;
   CUtensorMap ma, mb;
   bool akf = false, bkf = false;
@@ -359,7 +363,7 @@ int dgemm_tma(stream_t s, const Gemm& q, int cfg, int nsplit) {
   DtmaLaunch f = akf ? (bkf ? pick<true, true>(cfg) : pick<true, false>(cfg))
                      : (bkf ? pick<false, true>(cfg) : pick<false, false>(cfg));
   if (nsplit <= 1) {
-    DOut o{q.C, q.m, q.n, q.scn, q.scb, q.alpha, q.beta};
+    DOut o{q.C, q.m, q.n, q.scn, q.scb, q.alpha, q.beta, (int)q.tri};
     return f(st, ma, mb, o, q.k, q.k, (int)q.batch, 0);
   }
   int64_t kc = (q.k + nsplit - 1) / nsplit;

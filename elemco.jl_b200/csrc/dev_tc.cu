@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
                       double alpha, double beta, const TcSegs segs, int kb_per_split,
                       int kblocks_total,
                       int64_t split_stride, int mtiles, int ntiles, int nsplit,
-                      const TcMaps* __restrict__ mtab, unsigned long long wait_ns) {
+                      const TcMaps* __restrict__ mtab, unsigned long long wait_ns, int tri) {
   using Cfg = TcCfg<NSL, TN>;
   constexpr int STAGES = Cfg::STAGES, STAGE_BYTES = Cfg::STAGE_BYTES;
   constexpr int TILE_BYTES_B = Cfg::TILE_BYTES_B;
@@ -278,6 +278,10 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
     }
     z = (int)(it / ((int64_t)mtiles * ntiles));
   };
+  // tri > 0: tiles whose elements all have n / tri < m / tri are not needed
+  auto skip = [&](int mt, int nt) {
+    return tri > 0 && (nt * TN + TN - 1) / tri < mt * TM / tri;
+  };
   // z is a K slice (mtab == nullptr) or a batch item with its own operand maps
   // (mtab[z]), each covering all k-blocks
   auto item_kblocks = [&](int z) {
@@ -290,6 +294,7 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
       for (int64_t it = blockIdx.x; it < items && !*(volatile int*)abort_flag; it += gridDim.x) {
         int mt, nt, z;
         item_coords(it, mt, nt, z);
+        if (skip(mt, nt)) continue;
         const int nk = item_kblocks(z), kb0 = mtab ? 0 : z * kb_per_split;
         const TcMaps* mp = mtab ? mtab + z : &maps;
         for (int kb = 0; kb < nk; ++kb, ++g) {
@@ -326,6 +331,10 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
            it += gridDim.x, ++lt) {
         int mt, nt, z;
         item_coords(it, mt, nt, z);
+        if (skip(mt, nt)) {
+          --lt;
+          continue;
+        }
         const int nk = item_kblocks(z), kb0 = mtab ? 0 : z * kb_per_split;
         const int acc = (int)(lt & 1);
         const int64_t ua = lt >> 1;
@@ -379,6 +388,10 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
     for (int64_t it = blockIdx.x; it < items; it += gridDim.x, ++lt) {
       int mt, nt, z;
       item_coords(it, mt, nt, z);
+      if (skip(mt, nt)) {
+        --lt;
+        continue;
+      }
       const int acc = (int)(lt & 1);
       const int64_t row = (int64_t)mt * TM + q * 32 + lane;
       int64_t rowoff = (int64_t)z * split_stride;
@@ -659,7 +672,7 @@ unsigned long long wait_bound(cudaStream_t st) {
 template <int NSL, int TN>
 int launch_tc(cudaStream_t st, const TcMaps& maps, const TcSegs& segs, int kbt, int64_t m,
               int64_t n, int64_t mp, int64_t np, double alpha, double beta, const TcOut& out,
-              int S) {
+              int S, int tri = 0) {
   using Cfg = TcCfg<NSL, TN>;
   set_smem_attr<NSL, TN>();
   const int mt = (int)(mp / TM), nt = (int)(np / TN);
@@ -669,11 +682,12 @@ int launch_tc(cudaStream_t st, const TcMaps& maps, const TcSegs& segs, int kbt, 
   const unsigned grid = (unsigned)(items < 148 ? items : 148);
   const unsigned long long wns = wait_bound(st);
   // useful BF16 products: 2 m n K per slice pair (zero padding not counted)
-  const double work = 2.0 * (double)m * (double)n * (double)seg_depth(segs) * Cfg::NPAIR;
+  const double work = 2.0 * (double)m * (double)n * (double)seg_depth(segs) * Cfg::NPAIR *
+                      gemm_kept(m, n, tri);
   const int slot = ktime_begin((stream_t)st, KT_TCGEMM);
   if (S == 1) {
     mgemm_bf16_kernel<NSL, TN><<<grid, THREADS_TC, Cfg::SMEM_BYTES, st>>>(
-        maps, out, m, n, alpha, beta, segs, kps, kbt, 0, mt, nt, 1, nullptr, wns);
+        maps, out, m, n, alpha, beta, segs, kps, kbt, 0, mt, nt, 1, nullptr, wns, tri);
     note_launches(1);
     ktime_end((stream_t)st, KT_TCGEMM, slot, work);
     return (int)cudaGetLastError();
@@ -685,7 +699,7 @@ int launch_tc(cudaStream_t st, const TcMaps& maps, const TcSegs& segs, int kbt, 
   if (!P) return (int)cudaErrorMemoryAllocation;
   TcOut po{P, 1, m, 0, 0, 0, 0, 1};
   mgemm_bf16_kernel<NSL, TN><<<grid, THREADS_TC, Cfg::SMEM_BYTES, st>>>(
-      maps, po, m, n, 1.0, 0.0, segs, kps, kbt, m * n, mt, nt, S, nullptr, wns);
+      maps, po, m, n, 1.0, 0.0, segs, kps, kbt, m * n, mt, nt, S, nullptr, wns, 0);
   note_launches(1);
   int e = (int)cudaGetLastError();
   if (e) return e;
@@ -929,19 +943,20 @@ static int tc_gemm_run(cudaStream_t st, const TcGemm& g, int ns, const TcSegs& s
   }
   TcOut out{g.C, g.scm, g.scn, g.dn, g.scn2, g.dm, g.scm2, g.f32 ? 1 : 0};
   const int64_t mp = pad_rows(g.m), np = (g.n + tn - 1) / tn * tn;
+  const int tri = (int)g.tri;
   if (nsl == 3)
     return tn == TN_WIDE
                ? launch_tc<3, TN_WIDE>(st, maps, segs, kbt, g.m, g.n, mp, np, g.alpha, g.beta,
-                                       out, S)
+                                       out, S, tri)
                : launch_tc<3, 128>(st, maps, segs, kbt, g.m, g.n, mp, np, g.alpha, g.beta, out,
-                                   S);
+                                   S, tri);
   if (tn == TN_XWIDE)
     return launch_tc<2, TN_XWIDE>(st, maps, segs, kbt, g.m, g.n, mp, np, g.alpha, g.beta, out,
-                                  S);
-  return tn == TN_WIDE
-             ? launch_tc<2, TN_WIDE>(st, maps, segs, kbt, g.m, g.n, mp, np, g.alpha, g.beta, out,
-                                     S)
-             : launch_tc<2, 128>(st, maps, segs, kbt, g.m, g.n, mp, np, g.alpha, g.beta, out, S);
+                                  S, tri);
+  return tn == TN_WIDE ? launch_tc<2, TN_WIDE>(st, maps, segs, kbt, g.m, g.n, mp, np, g.alpha,
+                                               g.beta, out, S, tri)
+                       : launch_tc<2, 128>(st, maps, segs, kbt, g.m, g.n, mp, np, g.alpha, g.beta,
+                                           out, S, tri);
 }
 
 // Split counts a plain FP64 output allows: at least enough K slices that no
@@ -952,7 +967,9 @@ int tc_gemm(stream_t s, const TcGemm& g) {
   if (g.m <= 0 || g.n <= 0) return 0;
   int64_t k[TC_MAX_SEG];
   const int ns = gemm_segments(g, k);
-  if (ns == 0) return (int)cudaErrorInvalidValue;
+  if (ns == 0 || (g.tri > 0 && (g.beta != 0.0 || g.m >= (int64_t)1 << 30 ||
+                                g.n >= (int64_t)1 << 30)))
+    return (int)cudaErrorInvalidValue;
   const int nsl = g.A[0]->slices;
   const TcSegs segs = make_segs(ns, k);
   const int kbt = segs.kb_end[TC_MAX_SEG - 1];
@@ -1045,7 +1062,7 @@ void launch_batched(cudaStream_t st, const TcOut& out, const TcGemm& g, const Tc
   const int slot = ktime_begin((stream_t)st, KT_TCGEMM);
   mgemm_bf16_kernel<NSL, TN><<<grid, THREADS_TC, Cfg::SMEM_BYTES, st>>>(
       dummy, out, g.m, g.n, g.alpha, g.beta, segs, kbt, kbt, c_stride, mt, nt, batch,
-      (const TcMaps*)mtab, wait_bound(st));
+      (const TcMaps*)mtab, wait_bound(st), 0);
   ktime_end((stream_t)st, KT_TCGEMM, slot,
             2.0 * (double)g.m * (double)g.n * (double)seg_depth(segs) * Cfg::NPAIR * batch);
 }

@@ -105,10 +105,16 @@ void sync_scalars(Ctx& c, int count) {
 // --------------------------------------------------------------- setup
 
 // a-block size of the symmetric ladder: Vblk holds v^2 na (v - a0) doubles.
+// An eighth of the virtual space, but as much of it as 256 MiB of V hold: at
+// small v a block's five launches cost more than they compute (CCSD iteration
+// of o=12, v=57 with 256 / 64 / 32 MiB: 1.76 / 1.80 / 1.84 ms, eight blocks
+// 2.01; o=14, v=100: 5.78 / 5.97 / 5.98, eight blocks 6.05), and the tiles with
+// b < a are skipped inside a block.
 static int64_t ladder_na(int64_t nv) {
   const int64_t budget = (int64_t)1 << 28;  // doubles (2 GiB) for one V block
   // an even block start keeps the block's rows of B on 16 bytes for TMA
   int64_t na = ((nv + 7) / 8 + 1) / 2 * 2;
+  na = std::max(na, (((int64_t)1 << 25) / (nv * nv * nv)) / 2 * 2);
   na = std::min<int64_t>(na, std::max<int64_t>(1, budget / std::max<int64_t>(nv * nv * nv, 1)));
   return std::max<int64_t>(1, std::min(na, nv));
 }
@@ -200,7 +206,7 @@ void setup_system(Ctx& c, int no, int nv, int nq, const double* B, const double*
 
   const int64_t n2 = c.n2(), na = ladder_na(v);
   int64_t wsn = 16 * n2 + 6 * v * o * Q + 3 * v * v * Q + 2 * n * n * Q + 4 * o * o * o * o +
-                3 * na * v * v * v + 8 * n * n + (1 << 16);
+                2 * na * v * v * v + 8 * n * n + (1 << 16);
   c.ws_base = c.alloc(wsn, "workspace");
   c.ws.init(c.ws_base, wsn);
 
@@ -392,19 +398,22 @@ void ladder(Ctx& c, const double* Bf, const double* BfT, const double* T2, doubl
   const bool vf32 = fused && mv && Q <= dev::TC_ACC_K;
   for (auto& b : c.lblocks) {
     const int64_t nb = v - b.a0;
-    // V[c,a',d,b''] = sum_Q BfT[c,a0+a',Q] BfT[d,a0+b'',Q]
+    // V[c,a',d,b''] = sum_Q BfT[c,a0+a',Q] BfT[d,a0+b'',Q], needed for b >= a only
     if (mv) {
       dev::TcOperand a, bb;
       check(dev::tc_view(oB, v * b.a0, v * b.na, &a), "view BfT");
       check(dev::tc_view(oB, v * b.a0, v * nb, &bb), "view BfT");
       dev::TcGemm g;
       g.m = v * b.na; g.n = v * nb; g.A[0] = &a; g.B[0] = &bb;
-      g.C = V; g.scm = 1; g.scn = v * b.na; g.f32 = vf32;
+      g.C = V; g.scm = 1; g.scn = v * b.na; g.f32 = vf32; g.tri = v;
       check(dev::tc_gemm(s, g), "gemm ladder V");
     } else {
-      check(dev::gemm(s, 'N', 'T', v * b.na, v * nb, Q, 1.0, Bl + v * b.a0, ldb, Bl + v * b.a0,
-                      ldb, 0.0, V, v * b.na),
-            "gemm ladder V");
+      dev::Gemm g;
+      g.m = v * b.na; g.n = v * nb; g.k = Q;
+      g.A = Bl + v * b.a0; g.sam = 1; g.sak = ldb;
+      g.B = Bl + v * b.a0; g.sbn = 1; g.sbk = ldb;
+      g.C = V; g.scn = v * b.na; g.tri = v;
+      check(dev::gemm_strided(s, g), "gemm ladder V");
     }
     const int* pairs = c.pairs + 2 * b.poff;
     if (fused) {

@@ -46,7 +46,9 @@ int gemm(stream_t s, char ta, char tb, int64_t m, int64_t n, int64_t k, double a
 // Fully strided batched GEMM: C(m,n) = alpha sum_k A(m,k) B(k,n) + beta C(m,n)
 // with A(m,k) = A[b*sab + m*sam + k*sak], B(k,n) = B[b*sbb + k*sbk + n*sbn],
 // C(m,n) = C[b*scb + m*scm + n*scn] for batch b.  Batches must not write
-// overlapping C elements.
+// overlapping C elements.  tri > 0 (batch 1, beta 0): elements with
+// n / tri < m / tri are not needed, and tiles that hold nothing else are
+// skipped (such elements of C may keep their old values or get their product).
 struct Gemm {
   int64_t m = 0, n = 0, k = 0, batch = 1;
   double alpha = 1.0, beta = 0.0;
@@ -56,8 +58,17 @@ struct Gemm {
   int64_t sbk = 1, sbn = 0, sbb = 0;
   double* C = nullptr;
   int64_t scm = 1, scn = 0, scb = 0;
+  int64_t tri = 0;
 };
 int gemm_strided(stream_t s, const Gemm& g);
+// Share of C's elements that g computes (1 unless tri > 0; counted by tri x tri
+// squares).
+inline double gemm_kept(int64_t m, int64_t n, int64_t tri) {
+  if (tri <= 0) return 1.0;
+  const double a = (double)((m + tri - 1) / tri), b = (double)((n + tri - 1) / tri);
+  return a <= b ? 1.0 - (a - 1.0) / (2.0 * b) : (b + 1.0) / (2.0 * a);
+}
+inline double gemm_kept(const Gemm& g) { return gemm_kept(g.m, g.n, g.tri); }
 // FP64 GEMM with TMA-staged operands (dev_dgemm.cu): C with unit row stride,
 // each operand contiguous along its row index or along k with its other
 // strides even (16-byte multiples) and a 16-byte-aligned base.  cfg selects the
@@ -166,6 +177,8 @@ struct TcGemm {
   void* C = nullptr;
   bool f32 = false;
   int64_t scm = 1, scn = 0, dn = 0, scn2 = 0, dm = 0, scm2 = 0;
+  // tri > 0 (tc_gemm): as Gemm::tri
+  int64_t tri = 0;
 };
 int tc_gemm(stream_t s, const TcGemm& g);
 // Batched form: `batch` GEMMs of the shape of g (g.A/g.B give the segments
