@@ -1,7 +1,7 @@
 // dev_ints.cu — Gaussian integrals over contracted Cartesian shells on the GPU
 // (McMurchie-Davidson): overlap, kinetic energy, nuclear attraction, dipole
-// (one-electron), and two-/three-centre Coulomb integrals (P|Q), (mn|P) for
-// density fitting.  Replaces ElemCo.jl's libcint calls (src/system/libcint5.jl,
+// (one-electron), and the two-centre Coulomb integrals (P|Q) of density fitting
+// (the three-centre ones: dev_int3c.cu).  Replaces ElemCo.jl's libcint calls (src/system/libcint5.jl,
 // integrals_2idx.jl, integrals_2e3idx.jl).
 //
 // A Cartesian function of shell s is (x-X)^i (y-Y)^j (z-Z)^k exp(-a r_s^2)
@@ -244,37 +244,6 @@ __device__ void coulomb_block(const Sh& a, const Sh* b, const Sh& c, const Sh* d
     }
 }
 
-// (mn|P): item -> (shell a, shell b <= a, aux shell P); Cartesian output
-// out[m + nm*(n + nm*P)] (both orders of m, n written).
-__global__ void int3c_kernel(const IntShell* __restrict__ ao, int nao_sh,
-                             const IntShell* __restrict__ aux, int naux_sh,
-                             const double* __restrict__ ex, const double* __restrict__ co,
-                             int64_t nm, double* out) {
-  const int64_t npair = (int64_t)nao_sh * (nao_sh + 1) / 2;
-  const int64_t items = npair * naux_sh;
-  for (int64_t it = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; it < items;
-       it += (int64_t)gridDim.x * blockDim.x) {
-    const int P = (int)(it % naux_sh);
-    int64_t pr = it / naux_sh;
-    int ia = (int)((sqrt(8.0 * (double)pr + 1.0) - 1.0) / 2.0);
-    while ((int64_t)ia * (ia + 1) / 2 > pr) --ia;
-    while ((int64_t)(ia + 1) * (ia + 2) / 2 <= pr) ++ia;
-    const int ib = (int)(pr - (int64_t)ia * (ia + 1) / 2);
-    const Sh a = load_shell(ao, ia), b = load_shell(ao, ib), c = load_shell(aux, P);
-    double* o = out + a.boff + nm * (b.boff + nm * (int64_t)c.boff);
-    coulomb_block(a, &b, c, nullptr, ex, co, o, 1, nm, nm * nm, 0);
-    if (ia != ib) {
-      // mirror: out[n, m, P] = out[m, n, P]
-      const int na = ncart(a.l), nb = ncart(b.l), nc = ncart(c.l);
-      double* o2 = out + b.boff + nm * (a.boff + nm * (int64_t)c.boff);
-      for (int k = 0; k < nc; ++k)
-        for (int j = 0; j < nb; ++j)
-          for (int i = 0; i < na; ++i)
-            o2[j + nm * (i + nm * (int64_t)k)] = o[i + nm * (j + nm * (int64_t)k)];
-    }
-  }
-}
-
 // (P|Q): item -> (P, Q <= P); out[P + np*Q] (both orders written).
 __global__ void int2c_kernel(const IntShell* __restrict__ aux, int naux_sh,
                              const double* __restrict__ ex, const double* __restrict__ co,
@@ -415,15 +384,6 @@ int int2c2e_cart(stream_t s, const IntShell* aux, int nsh, const double* ex, con
                  int64_t np_, double* out) {
   const int64_t items = (int64_t)nsh * (nsh + 1) / 2;
   int2c_kernel<<<grid_of(items, 64), 64, 0, (cudaStream_t)s>>>(aux, nsh, ex, co, np_, out);
-  note_launches(1);
-  return (int)cudaGetLastError();
-}
-
-int int3c2e_cart(stream_t s, const IntShell* ao, int nao_sh, const IntShell* aux, int naux_sh,
-                 const double* ex, const double* co, int64_t nm, double* out) {
-  const int64_t items = (int64_t)nao_sh * (nao_sh + 1) / 2 * naux_sh;
-  int3c_kernel<<<grid_of(items, 64), 64, 0, (cudaStream_t)s>>>(ao, nao_sh, aux, naux_sh, ex, co,
-                                                               nm, out);
   note_launches(1);
   return (int)cudaGetLastError();
 }

@@ -6,6 +6,7 @@
 #pragma once
 #include <cstddef>
 #include <cstdint>
+#include <vector>
 
 namespace ecg {
 namespace dev {
@@ -385,9 +386,41 @@ int int1e_cart(stream_t s, int kind, const IntShell* sh, int nsh, const double* 
 // (P|Q), out[P + np*Q]
 int int2c2e_cart(stream_t s, const IntShell* aux, int nsh, const double* ex, const double* co,
                  int64_t np, double* out);
-// (mn|P), out[m + nm*(n + nm*P)]; ex/co hold both bases' primitives
-int int3c2e_cart(stream_t s, const IntShell* ao, int nao_sh, const IntShell* aux, int naux_sh,
-                 const double* ex, const double* co, int64_t nm, double* out);
+// (mn|P) over real solid harmonics, normalised: out[m + n*(m' + n*P)].  build()
+// collects on the host the AO shell pairs by class with their primitive pairs,
+// and the fitting shells by degree (boff: first spherical function; exponents
+// and coefficients as for the other integrals, each basis with its own
+// arrays); it returns -1 for a function of zero norm.  run() uploads them to
+// `tables` (table_doubles(), 16-byte aligned) and launches.
+struct IntPair {
+  int pp0, npp, aoff, boff;  // primitive pairs, first functions (la >= lb)
+  int64_t hoff;              // its first Hermite expansion
+};
+struct IntPrimPair {
+  double p, x, y, z;
+};
+struct IntPairPrimSrc {
+  double p, pa[3], pb[3], f;
+  int64_t hoff;
+  int la, lb;
+};
+struct Int3cPlan {
+  std::vector<IntPair> pairs;
+  std::vector<IntPrimPair> prims;
+  std::vector<IntPairPrimSrc> src;
+  std::vector<IntShell> aux;
+  std::vector<double> ex, co;
+  // by class la*(INT_LMAX+1) + lb: first pair, pairs, and how many of them (the
+  // first ones) are contracted
+  int pair0[(INT_LMAX + 1) * (INT_LMAX + 1)] = {}, npair[(INT_LMAX + 1) * (INT_LMAX + 1)] = {};
+  int nsplit[(INT_LMAX + 1) * (INT_LMAX + 1)] = {};
+  int aux0[INT_LMAX + 1] = {}, naux[INT_LMAX + 1] = {};
+  int64_t hlen = 0;
+  int build(const IntShell* ao, int nao_sh, const double* aoex, const double* aoco,
+            const IntShell* fit, int nfit_sh, const double* fex, const double* fco);
+  int64_t table_doubles() const;
+  int run(stream_t s, double* tables, int64_t n, double* out) const;
+};
 
 // Count of kernels launched through this layer in this process.
 int64_t launches();

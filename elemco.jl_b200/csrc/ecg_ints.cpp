@@ -232,49 +232,22 @@ void check_ltot(const Basis& a, const Basis* b, const Basis& c) {
 }
 
 // (mn|P) of ao x ao x fit on the device, spherical and normalised, as
-// Z[m + nao*(n + nao*P)] in an allocation of c's stack (with the
-// intermediates below it: the caller's scope releases them all).
+// Z[m + nao*(n + nao*P)] in an allocation of c's stack (with its tables: the
+// caller's scope releases them).
 double* int3c2e_device(Ctx& c, const ecg_shells* ao, const ecg_shells* fit, int64_t* nao,
                        int64_t* naux) {
-  const Basis A = make_basis(ao, 0, 0);
-  // P0: the fitting basis on its own (normalisation, transform); P: the same
-  // shells with primitive offsets past A's, for the kernel's joint arrays
-  const Basis P0 = make_basis(fit, 0, 0);
-  const Basis P = make_basis(fit, (int)A.ex.size(), 0);
+  Basis A = make_basis(ao, 0, 0), P = make_basis(fit, 0, 0);
   check_ltot(A, &A, P);
-  const std::vector<double> dA = norms(c, A), dP = norms(c, P0);
-  std::vector<double> TA = sph_transform(A), TP = sph_transform(P0);
-  for (int64_t k = 0; k < A.ncart; ++k)
-    for (int64_t i = 0; i < A.nsph; ++i) TA[i + A.nsph * k] *= dA[i];
-  for (int64_t k = 0; k < P.ncart; ++k)
-    for (int64_t i = 0; i < P.nsph; ++i) TP[i + P.nsph * k] *= dP[i];
-  const int64_t na = A.ncart, np = P.ncart, sa = A.nsph, sp = P.nsph;
-  std::vector<double> ex(A.ex), co(A.co);
-  ex.insert(ex.end(), P.ex.begin(), P.ex.end());
-  co.insert(co.end(), P.co.begin(), P.co.end());
-  DevBasis dao = upload(c, A.sh, ex, co);
-  DevBasis daux = upload(c, P.sh, {}, {});
-  double* X = c.alloc(na * na * np, "int3c cart");
-  check(dev::memset0(X, na * na * np * 8, c.st), "memset");
-  check(dev::int3c2e_cart(c.st, dao.sh, (int)A.sh.size(), daux.sh, (int)P.sh.size(), dao.ex,
-                          dao.co, na, X),
-        "int3c2e");
-  double* dTA = c.alloc(sa * na, "TA");
-  double* dTP = c.alloc(sp * np, "TP");
-  check(dev::h2d(dTA, TA.data(), TA.size() * 8, c.st), "h2d");
-  check(dev::h2d(dTP, TP.data(), TP.size() * 8, c.st), "h2d");
-  // Y1[m,n,P] = sum_Pc X[m,n,Pc] TP[P,Pc]
-  double* Y1 = c.alloc(na * na * sp, "int3c 1");
-  check(dev::gemm(c.st, 'N', 'T', na * na, sp, np, 1.0, X, na * na, dTP, sp, 0.0, Y1, na * na),
-        "gemm P");
-  // Y2[m,n',P] = sum_n Y1[m,n,P] TA[n',n]  (batched over P)
-  double* Y2 = c.alloc(na * sa * sp, "int3c 2");
-  check(dev::gemm(c.st, 'N', 'T', na, sa, na, 1.0, Y1, na, dTA, sa, 0.0, Y2, na, sp, na * na, 0,
-                  na * sa),
-        "gemm n");
-  // Z[m',n',P] = sum_m TA[m',m] Y2[m,n',P]
-  double* Z = c.alloc(sa * sa * sp, "int3c 3");
-  check(dev::gemm(c.st, 'N', 'N', sa, sa * sp, na, 1.0, dTA, sa, Y2, na, 0.0, Z, sa), "gemm m");
+  for (Basis* b : {&A, &P})  // first spherical functions
+    for (size_t s = 0; s < b->sh.size(); ++s) b->sh[s].boff = b->sph_off[s];
+  const int64_t sa = A.nsph, sp = P.nsph;
+  dev::Int3cPlan plan;
+  if (plan.build(A.sh.data(), (int)A.sh.size(), A.ex.data(), A.co.data(), P.sh.data(),
+                 (int)P.sh.size(), P.ex.data(), P.co.data()))
+    throw Error(ECG_ERR_ARG, "basis function of zero norm");
+  double* tab = c.alloc(plan.table_doubles(), "int3c tables");
+  double* Z = c.alloc(sa * sa * sp, "int3c");
+  check(plan.run(c.st, tab, sa, Z), "int3c2e");
   *nao = sa;
   *naux = sp;
   return Z;
