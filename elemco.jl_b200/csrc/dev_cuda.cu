@@ -1989,14 +1989,22 @@ __global__ void final_sum_pairs_kernel(int nparts, const double* part, double* o
   if (threadIdx.x == 0) out[q] = r;
 }
 
+// Blocks per item: one block is resident per SM (128 registers a thread keep
+// the evaluation free of spills), and each fills and drains its pipeline of
+// staged orbits, so a block takes about 16 orbits rather than its share of 148
+// (at v = 76 that share had been 1.5 orbits, one or two of which the block
+// waited for and 26% of whose rounds were empty).  Measured, largest batch: v =
+// 76 1332 -> 1090 us; v = 318, capped at 148 blocks either way, 4152 us.  Of nv
+// alone, so that the sums group alike in every batch.
 int64_t triples_energy_grid(int nv) {
-  // one resident block per SM: 128 registers a thread keep the evaluation free
-  // of spills; the double-buffered loads overlap it with the next orbit
   const int64_t ntri = triples_cube_count(nv);
-  return ntri < 148 ? ntri : 148;
+  const int64_t per = std::max<int64_t>(2, std::min<int64_t>(16, ntri / 8));
+  return std::max<int64_t>(1, std::min<int64_t>((ntri + per - 1) / per, 148));
 }
 
-int64_t triples_energy_scratch_len(int nv, int nitems) { return 2 * triples_energy_grid(nv) * nitems; }
+int64_t triples_energy_scratch_len(int nv, int nitems) {
+  return 2 * std::max(triples_energy_grid(nv), triples_energy_f32_grid(nv)) * nitems;
+}
 
 int triples_energy_batched(stream_t s, int nv, int nitems, const void* K, const void* KU,
                            int64_t kstride, bool k_f32, const double* eijk_tab, const double* ev,

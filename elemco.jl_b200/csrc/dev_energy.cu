@@ -362,6 +362,18 @@ int launch_energy(cudaStream_t st, dim3 grid, const CUtensorMap* maps, int nv,
 
 }  // namespace
 
+// Blocks per item: about 16 orbits for each of a block's eight warps, which
+// start and drain a block at a cost of more than an orbit and share orbits out
+// evenly only when each has many (at v = 209 148 blocks had 3.1 orbits a warp).
+// Measured, largest batch: v = 129 1750 -> 1375 us, v = 209 2673 -> 2300 us; v =
+// 318 unchanged (1.8 ms).
+// Of nv alone, so that the sums group alike in every batch.
+int64_t triples_energy_f32_grid(int nv) {
+  const int64_t ntri = triples_cube_count(nv), w = EnergyWarpSmem<false>::WARPS;
+  const int64_t per = std::max<int64_t>(2, std::min<int64_t>(16, ntri / 64));
+  return std::max<int64_t>(1, std::min<int64_t>((ntri + w * per - 1) / (w * per), 148));
+}
+
 int64_t triples_mn_elems(int nv, int64_t npairs) {
   return (int64_t)((nv + 1) / 2 * 2) * nv * npairs;
 }
@@ -410,7 +422,7 @@ int triples_energy_f32_batched(stream_t s, int nv, int vp, int nitems, int nslot
     if (int e = encode(&maps[2], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, mn, dm, sm, bm)) return e;
     if (int e = encode(&maps[3], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, mt, dm, sm, bm)) return e;
   }
-  const int g = (int)triples_energy_grid(nv);
+  const int g = (int)triples_energy_f32_grid(nv);
   cudaStream_t st = (cudaStream_t)s;
   const dim3 grid((unsigned)g, (unsigned)nitems);
   const int slot = ktime_begin(s, KT_TRIPLES);

@@ -274,7 +274,9 @@ void triples_cube_table(int nv, int* tri);
 // summed in a fixed order.  One launch (plus one fixed-order reduction
 // launch).  k_f32 must be false (FP32 K: triples_energy_f32_batched).
 int64_t triples_energy_scratch_len(int nv, int nitems);
-int64_t triples_energy_grid(int nv);  // blocks per batch item of the energy kernels
+// blocks per batch item of the FP64 / FP32 energy kernels
+int64_t triples_energy_grid(int nv);
+int64_t triples_energy_f32_grid(int nv);
 int triples_energy_batched(stream_t s, int nv, int nitems, const void* K, const void* KU,
                            int64_t kstride, bool k_f32, const double* eijk_tab, const double* ev,
                            const TriplesTerms* tt_tab, const int* tri, double* scratch,
