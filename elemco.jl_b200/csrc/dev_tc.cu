@@ -32,6 +32,7 @@
 #include "ecg_dev.h"
 #include "ecg_tune.h"
 #include "tma_util.cuh"
+#include "umma.cuh"
 
 namespace ecg {
 namespace dev {
@@ -61,6 +62,7 @@ using tma::mbar_init;
 using tma::mbar_wait;
 using tma::smem_u32;
 using tma::tma_load_3d;
+using namespace umma_ops;
 
 template <int NSL, int TN>
 struct TcCfg {
@@ -78,38 +80,7 @@ struct TcCfg {
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
   static_assert(TILE_BYTES_B % 1024 == 0, "128-byte-swizzle tiles start on 1024 bytes");
 };
-// slice pairs (a, b): hi*hi, hi*mid, mid*hi, mid*mid, hi*lo, lo*hi (the first
-// three for NSL = 2)
-__host__ __device__ constexpr int pair_a(int p) { return p == 2 || p == 3 ? 1 : p == 5 ? 2 : 0; }
-__host__ __device__ constexpr int pair_b(int p) { return p == 1 || p == 3 ? 1 : p == 4 ? 2 : 0; }
-
 __device__ int g_tc_error = 0;
-
-// UMMA shared-memory descriptor, K-major operand in the 128-byte-swizzled
-// canonical layout: 128-byte rows, 8-row (1024-byte) groups.
-__device__ __forceinline__ uint64_t umma_desc(const void* p) {
-  const uint32_t a = smem_u32(p);
-  uint64_t d = (uint64_t)((a & 0x3FFFF) >> 4);  // start address
-  d |= (uint64_t)1 << 16;                        // leading byte offset (unused for SW128 K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;              // stride byte offset: 8-row group
-  d |= (uint64_t)1 << 46;                        // descriptor version (sm_100)
-  d |= (uint64_t)2 << 61;                        // layout: SWIZZLE_128B
-  return d;
-}
-
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc,
-                                     uint32_t acc) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(da), "l"(db), "r"(idesc), "r"(acc));
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-          smem_u32(bar)));
-}
 
 // Persistent, warp-specialised kernel: gridDim.x CTAs (one per SM) loop over
 // work items (m-tile, n-tile, k-slice).  Warp 0 lane 0: TMA producer over a
@@ -149,13 +120,12 @@ __device__ __forceinline__ SegPos seg_of(const TcSegs& sg, int kg) {
   return p;
 }
 
-// Output element (m, n) lives at C[rowoff(m) + coloff(n)] (FP64, or FP32 when
-// f32) with rowoff(m) = (m % dm)*scm + (m / dm)*scm2 (dm = 0: m*scm) and
-// coloff(n) = (n % dn)*scn + (n / dn)*scn2 (dn = 0: n*scn).  Lanes of an
-// epilogue warp hold consecutive rows, so scm == 1 gives coalesced stores.
+// Output element (m, n) lives at C[m*scm + n*scn] (FP64, or FP32 when f32).
+// Lanes of an epilogue warp hold consecutive rows, so scm == 1 gives coalesced
+// stores.
 struct TcOut {
   void* C;
-  int64_t scm, scn, dn, scn2, dm, scm2;
+  int64_t scm, scn;
   int f32;
 };
 
@@ -170,25 +140,9 @@ __device__ __forceinline__ void epi_chunk(CT* __restrict__ C, int64_t rowoff, co
                                           int64_t col0, int64_t N, const TcOut& out,
                                           double alpha, double beta, bool f32math) {
   int64_t off[16];
-  if (out.dn == 0) {
-    const int64_t b = rowoff + col0 * out.scn;
+  const int64_t b0 = rowoff + col0 * out.scn;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) off[j] = b + j * out.scn;
-  } else {
-    const uint32_t dn = (uint32_t)out.dn, nq = (uint32_t)col0 / dn;
-    int64_t nr = (uint32_t)col0 - nq * dn;
-    int64_t coff = nr * out.scn + (int64_t)nq * out.scn2;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      off[j] = rowoff + coff;
-      ++nr;
-      coff += out.scn;
-      if (nr == out.dn) {
-        nr = 0;
-        coff += out.scn2 - out.dn * out.scn;
-      }
-    }
-  }
+  for (int j = 0; j < 16; ++j) off[j] = b0 + j * out.scn;
   if (sizeof(CT) == 4 && f32math) {
     const float a = (float)alpha;
     if (beta != 0.0) {  // beta == 1
@@ -224,7 +178,7 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
                       double alpha, double beta, const TcSegs segs, int kb_per_split,
                       int kblocks_total,
                       int64_t split_stride, int mtiles, int ntiles, int nsplit,
-                      const TcMaps* __restrict__ mtab, unsigned long long wait_ns, int tri) {
+                      unsigned long long wait_ns, int tri) {
   using Cfg = TcCfg<NSL, TN>;
   constexpr int STAGES = Cfg::STAGES, STAGE_BYTES = Cfg::STAGE_BYTES;
   constexpr int TILE_BYTES_B = Cfg::TILE_BYTES_B;
@@ -282,11 +236,7 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
   auto skip = [&](int mt, int nt) {
     return tri > 0 && (nt * TN + TN - 1) / tri < mt * TM / tri;
   };
-  // z is a K slice (mtab == nullptr) or a batch item with its own operand maps
-  // (mtab[z]), each covering all k-blocks
-  auto item_kblocks = [&](int z) {
-    return mtab ? kblocks_total : min(kb_per_split, kblocks_total - z * kb_per_split);
-  };
+  auto item_kblocks = [&](int z) { return min(kb_per_split, kblocks_total - z * kb_per_split); };
 
   if (warp == 0) {
     if (lane == 0) {
@@ -295,8 +245,7 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
         int mt, nt, z;
         item_coords(it, mt, nt, z);
         if (skip(mt, nt)) continue;
-        const int nk = item_kblocks(z), kb0 = mtab ? 0 : z * kb_per_split;
-        const TcMaps* mp = mtab ? mtab + z : &maps;
+        const int nk = item_kblocks(z), kb0 = z * kb_per_split;
         for (int kb = 0; kb < nk; ++kb, ++g) {
           const int s = (int)(g % STAGES);
           const int64_t u = g / STAGES;
@@ -308,8 +257,8 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
           uint8_t* st = tiles + s * STAGE_BYTES;
           const int kg = kb0 + kb;
           const SegPos sp = seg_of(segs, kg);
-          const CUtensorMap* ma = &mp->a[sp.s];
-          const CUtensorMap* mb = &mp->b[sp.s];
+          const CUtensorMap* ma = &maps.a[sp.s];
+          const CUtensorMap* mb = &maps.b[sp.s];
           const int kx = (kg - sp.start) * TK;
           mbar_expect_tx(&full[s], STAGE_BYTES);
           for (int t = 0; t < NSL; ++t) {
@@ -335,7 +284,7 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
           --lt;
           continue;
         }
-        const int nk = item_kblocks(z), kb0 = mtab ? 0 : z * kb_per_split;
+        const int nk = item_kblocks(z), kb0 = z * kb_per_split;
         const int acc = (int)(lt & 1);
         const int64_t ua = lt >> 1;
         if (ua > 0 && !mbar_wait(&tempty[acc], (uint32_t)((ua - 1) & 1), wait_ns)) {
@@ -394,13 +343,7 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
       }
       const int acc = (int)(lt & 1);
       const int64_t row = (int64_t)mt * TM + q * 32 + lane;
-      int64_t rowoff = (int64_t)z * split_stride;
-      if (out.dm > 0) {
-        const int64_t mq = row / out.dm;
-        rowoff += (row - mq * out.dm) * out.scm + mq * out.scm2;
-      } else {
-        rowoff += row * out.scm;
-      }
+      const int64_t rowoff = (int64_t)z * split_stride + row * out.scm;
       // every lane waits; the warp goes on only if all lanes saw the
       // accumulator ready and no time-out was recorded, so the warp-wide
       // tcgen05.ld below always runs converged
@@ -417,14 +360,7 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
 #pragma unroll 1
       for (int c = hw * (TN / 2); c < (hw + 1) * (TN / 2); c += 16) {
         uint32_t r[16];
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,"
-            "%13,%14,%15}, [%16];\n"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-              "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-              "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-            : "r"(tmem + lane_base + (uint32_t)(acc * TN + c)));
-        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::);
+        tmem_ld16(tmem + lane_base + (uint32_t)(acc * TN + c), r);
         if (row < M) {
           const int64_t col0 = (int64_t)nt * TN + c;
           if (out.f32)
@@ -453,13 +389,22 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
 // coalesced whichever of sr / sk is the unit stride.
 __global__ void split_kernel(const double* __restrict__ src, int64_t R, int64_t K, int64_t sr,
                              int64_t sk, int64_t Rp, int64_t Kp, int nsl,
-                             __nv_bfloat16* __restrict__ dst) {
+                             __nv_bfloat16* __restrict__ dst, uint32_t dr, int64_t d, int64_t s0,
+                             int64_t s1) {
   __shared__ double tile[32][33];
   // tile indices in 32 bits (an operand whose BF16 slices fit in device
   // memory has fewer than 2^25 tiles): one 64-bit division per tile would
   // cost more instructions than its 1024 elements
   const uint32_t tk = (uint32_t)((Kp + 31) / 32), ntile = tk * (uint32_t)((Rp + 31) / 32);
-  const bool rfast = (sr == 1);
+  const bool rfast = (sr == 1 || dr > 0);
+  // item blockIdx.y of a stack (TcStack; one item: d = 1)
+  src += ((int64_t)blockIdx.y % d) * s0 + ((int64_t)blockIdx.y / d) * s1;
+  dst += (int64_t)blockIdx.y * nsl * Rp * Kp;
+  auto rowoff = [&](int64_t r) {
+    if (dr == 0) return r * sr;
+    const uint32_t q = (uint32_t)r / dr;
+    return (int64_t)((uint32_t)r - q * dr) + (int64_t)q * sr;
+  };
   for (uint32_t t = blockIdx.x; t < ntile; t += gridDim.x) {
     const int64_t r0 = (int64_t)(t / tk) * 32, k0 = (int64_t)(t % tk) * 32;
     // the four loads of a thread are issued before any of them is used
@@ -469,7 +414,7 @@ __global__ void split_kernel(const double* __restrict__ src, int64_t R, int64_t 
       const int j = threadIdx.y + 8 * jj;
       int64_t r, k;
       if (rfast) { r = r0 + threadIdx.x; k = k0 + j; } else { r = r0 + j; k = k0 + threadIdx.x; }
-      xs[jj] = (r < R && k < K) ? src[r * sr + k * sk] : 0.0;
+      xs[jj] = (r < R && k < K) ? src[rowoff(r) + k * sk] : 0.0;
     }
 #pragma unroll
     for (int jj = 0; jj < 4; ++jj) {
@@ -629,7 +574,7 @@ void launch_split(cudaStream_t st, const double* src, int64_t R, int64_t K, int6
                   int64_t sk, int64_t Rp, int64_t Kp, int nsl, __nv_bfloat16* dst) {
   const int64_t tiles = ((Rp + 31) / 32) * ((Kp + 31) / 32);
   const unsigned g = (unsigned)(tiles < 148 * 16 ? tiles : 148 * 16);
-  split_kernel<<<g, dim3(32, 8), 0, st>>>(src, R, K, sr, sk, Rp, Kp, nsl, dst);
+  split_kernel<<<g, dim3(32, 8), 0, st>>>(src, R, K, sr, sk, Rp, Kp, nsl, dst, 0, 1, 0, 0);
   note_launches(1);
 }
 
@@ -687,19 +632,19 @@ int launch_tc(cudaStream_t st, const TcMaps& maps, const TcSegs& segs, int kbt, 
   const int slot = ktime_begin((stream_t)st, KT_TCGEMM);
   if (S == 1) {
     mgemm_bf16_kernel<NSL, TN><<<grid, THREADS_TC, Cfg::SMEM_BYTES, st>>>(
-        maps, out, m, n, alpha, beta, segs, kps, kbt, 0, mt, nt, 1, nullptr, wns, tri);
+        maps, out, m, n, alpha, beta, segs, kps, kbt, 0, mt, nt, 1, wns, tri);
     note_launches(1);
     ktime_end((stream_t)st, KT_TCGEMM, slot, work);
     return (int)cudaGetLastError();
   }
-  if (out.f32 || out.dn > 0 || out.dm > 0) return (int)cudaErrorInvalidValue;
+  if (out.f32) return (int)cudaErrorInvalidValue;
   // partial products in FP32, exactly as tensor memory accumulated them (one
   // accumulation each), summed in FP64 by the reduction
   float* P = reinterpret_cast<float*>(splitk_buffer((stream_t)st, ((size_t)S * m * n + 1) / 2));
   if (!P) return (int)cudaErrorMemoryAllocation;
-  TcOut po{P, 1, m, 0, 0, 0, 0, 1};
+  TcOut po{P, 1, m, 1};
   mgemm_bf16_kernel<NSL, TN><<<grid, THREADS_TC, Cfg::SMEM_BYTES, st>>>(
-      maps, po, m, n, 1.0, 0.0, segs, kps, kbt, m * n, mt, nt, S, nullptr, wns, 0);
+      maps, po, m, n, 1.0, 0.0, segs, kps, kbt, m * n, mt, nt, S, wns, 0);
   note_launches(1);
   int e = (int)cudaGetLastError();
   if (e) return e;
@@ -735,6 +680,24 @@ int tc_split(stream_t s, const double* src, int64_t rows, int64_t k, int64_t sr,
   e = (int)cudaGetLastError();
   if (e) return e;
   return encode_operand(enc, op, op->rows_p);
+}
+
+int tc_split_stack(stream_t s, const double* src, int64_t rows, int64_t k, int64_t sr, int64_t sk,
+                   int64_t dr, int64_t items, int64_t d, int64_t s0, int64_t s1, void* dst,
+                   TcStack* out) {
+  if (rows <= 0 || k <= 0 || items <= 0 || items > 65535 || d <= 0 || dr < 0 || !src || !dst ||
+      !out || rows >= ((int64_t)1 << 31))
+    return (int)cudaErrorInvalidValue;
+  if (((uintptr_t)dst & 15) != 0) return (int)cudaErrorMisalignedAddress;
+  const int64_t Rp = pad_rows(rows), Kp = pad_k(k);
+  const int64_t tiles = ((Rp + 31) / 32) * ((Kp + 31) / 32);
+  const dim3 g((unsigned)std::min<int64_t>(tiles, 148 * 16), (unsigned)items);
+  split_kernel<<<g, dim3(32, 8), 0, (cudaStream_t)s>>>(src, rows, k, sr, sk, Rp, Kp, 2,
+                                                       (__nv_bfloat16*)dst, (uint32_t)dr, d, s0,
+                                                       s1);
+  note_launches(1);
+  *out = TcStack{dst, rows, k, items};
+  return (int)cudaGetLastError();
 }
 
 int64_t tc_pad_rows(int64_t rows) { return pad_rows(rows); }
@@ -941,7 +904,7 @@ static int tc_gemm_run(cudaStream_t st, const TcGemm& g, int ns, const TcSegs& s
     std::memcpy(&maps.a[t], g.A[t < ns ? t : 0]->map, sizeof(CUtensorMap));
     std::memcpy(&maps.b[t], b_map(g.B[t < ns ? t : 0], tn), sizeof(CUtensorMap));
   }
-  TcOut out{g.C, g.scm, g.scn, g.dn, g.scn2, g.dm, g.scm2, g.f32 ? 1 : 0};
+  TcOut out{g.C, g.scm, g.scn, g.f32 ? 1 : 0};
   const int64_t mp = pad_rows(g.m), np = (g.n + tn - 1) / tn * tn;
   const int tri = (int)g.tri;
   if (nsl == 3)
@@ -973,7 +936,7 @@ int tc_gemm(stream_t s, const TcGemm& g) {
   const int nsl = g.A[0]->slices;
   const TcSegs segs = make_segs(ns, k);
   const int kbt = segs.kb_end[TC_MAX_SEG - 1];
-  const bool plain = !g.f32 && g.dn == 0 && g.dm == 0;
+  const bool plain = !g.f32;
   // tile widths every B operand has a descriptor for
   auto usable = [&](int tn) {
     for (int t = 0; t < ns; ++t)
@@ -1000,7 +963,7 @@ int tc_gemm(stream_t s, const TcGemm& g) {
       tn = tw;
       S = plain ? std::max(enc / 4, tc_min_split(kbt)) : 1;
     }
-  } else if (tuning() && g.dn == 0 && g.dm == 0 && g.scm == 1 && !stream_capturing(s)) {
+  } else if (tuning() && g.scm == 1 && !stream_capturing(s)) {
     struct Cand {
       int tn, S;
     };
@@ -1030,76 +993,6 @@ int tc_gemm(stream_t s, const TcGemm& g) {
   return tc_gemm_run(st, g, ns, segs, kbt, tn, S);
 }
 
-size_t tc_maps_bytes() { return sizeof(TcMaps); }
-
-int tc_maps_fill(int nseg, const TcOperand* const* A, const TcOperand* const* B, int64_t n,
-                 void* dst) {
-  if (nseg < 1 || nseg > TC_MAX_SEG || !A || !B || !dst || n <= 0)
-    return (int)cudaErrorInvalidValue;
-  for (int t = 0; t < nseg; ++t)
-    if (!A[t] || !B[t]) return (int)cudaErrorInvalidValue;
-  const int tn = tile_n(n, A[0]->slices);
-  for (int t = 0; t < nseg; ++t)
-    if (!b_map(B[t], tn)) return (int)cudaErrorInvalidValue;
-  TcMaps* m = reinterpret_cast<TcMaps*>(dst);
-  for (int t = 0; t < TC_MAX_SEG; ++t) {
-    std::memcpy(&m->a[t], A[t < nseg ? t : 0]->map, sizeof(CUtensorMap));
-    std::memcpy(&m->b[t], b_map(B[t < nseg ? t : 0], tn), sizeof(CUtensorMap));
-  }
-  return 0;
-}
-
-namespace {
-template <int NSL, int TN>
-void launch_batched(cudaStream_t st, const TcOut& out, const TcGemm& g, const TcSegs& segs,
-                    int kbt, int64_t c_stride, int mt, int nt, int batch, const void* mtab) {
-  using Cfg = TcCfg<NSL, TN>;
-  set_smem_attr<NSL, TN>();
-  const int64_t items = (int64_t)mt * nt * batch;
-  const unsigned grid = (unsigned)(items < 148 ? items : 148);
-  TcMaps dummy;
-  std::memset(&dummy, 0, sizeof(dummy));
-  const int slot = ktime_begin((stream_t)st, KT_TCGEMM);
-  mgemm_bf16_kernel<NSL, TN><<<grid, THREADS_TC, Cfg::SMEM_BYTES, st>>>(
-      dummy, out, g.m, g.n, g.alpha, g.beta, segs, kbt, kbt, c_stride, mt, nt, batch,
-      (const TcMaps*)mtab, wait_bound(st), 0);
-  ktime_end((stream_t)st, KT_TCGEMM, slot,
-            2.0 * (double)g.m * (double)g.n * (double)seg_depth(segs) * Cfg::NPAIR * batch);
-}
-}  // namespace
-
-int tc_gemm_batched(stream_t s, const TcGemm& g, int batch, const void* mtab, int64_t c_stride) {
-  if (g.m <= 0 || g.n <= 0 || batch <= 0) return 0;
-  int64_t k[TC_MAX_SEG];
-  const int ns = gemm_segments(g, k);
-  if (ns == 0 || !mtab || ((uintptr_t)mtab & 63) != 0) return (int)cudaErrorInvalidValue;
-  // the tables were filled by tc_maps_fill with the same tile-width rule
-  const int nsl = g.A[0]->slices;
-  const int tn = tile_n(g.n, nsl);
-  for (int t = 0; t < ns; ++t)
-    if (!b_map(g.B[t], tn)) return (int)cudaErrorInvalidValue;
-  const TcSegs segs = make_segs(ns, k);
-  const int kbt = segs.kb_end[TC_MAX_SEG - 1];
-  const int64_t mp = pad_rows(g.m), np = (g.n + tn - 1) / tn * tn;
-  const int mt = (int)(mp / TM), nt = (int)(np / tn);
-  TcOut out{g.C, g.scm, g.scn, g.dn, g.scn2, g.dm, g.scm2, g.f32 ? 1 : 0};
-  cudaStream_t st = (cudaStream_t)s;
-  if (nsl == 3) {
-    if (tn == TN_WIDE)
-      launch_batched<3, TN_WIDE>(st, out, g, segs, kbt, c_stride, mt, nt, batch, mtab);
-    else
-      launch_batched<3, 128>(st, out, g, segs, kbt, c_stride, mt, nt, batch, mtab);
-  } else if (tn == TN_XWIDE) {
-    launch_batched<2, TN_XWIDE>(st, out, g, segs, kbt, c_stride, mt, nt, batch, mtab);
-  } else if (tn == TN_WIDE) {
-    launch_batched<2, TN_WIDE>(st, out, g, segs, kbt, c_stride, mt, nt, batch, mtab);
-  } else {
-    launch_batched<2, 128>(st, out, g, segs, kbt, c_stride, mt, nt, batch, mtab);
-  }
-  note_launches(1);
-  return (int)cudaGetLastError();
-}
-
 // C(m,n) = alpha sum_k A(m,k) B(k,n) + beta C(m,n) with the strided operands of
 // gemm_strided (batch 1): split both operands into three slices, run the
 // tensor-core kernel.
@@ -1125,7 +1018,7 @@ int gemm_strided_mixed(stream_t s, const Gemm& q) {
   // (n >= 160 then; rows past np read as zero)
   const TcSegs segs = make_segs(1, &k);
   const int kbt = (int)(kp / TK);
-  TcOut out{q.C, q.scm, q.scn, 0, 0, 0, 0, 0};
+  TcOut out{q.C, q.scm, q.scn, 0};
   auto run = [&](int tn, int S) {
     const int64_t npt = (n + tn - 1) / tn * tn;
     TcMaps maps;
@@ -1202,11 +1095,12 @@ int tc_error(int* code) {
     int zero = 0;
     cudaMemcpyToSymbol(g_tc_error, &zero, sizeof(int));
   }
-  int d = 0, en = 0, kb = 0;
+  int d = 0, en = 0, kb = 0, tk = 0;
   if (int r = dtma_error(&d)) return r;
   if (int r = energy_error(&en)) return r;
   if (int r = kbuild_error(&kb)) return r;
-  *code = h ? h : d ? 16 + d : en ? 32 + en : (kb ? 48 + kb : 0);
+  if (int r = tckbuild_error(&tk)) return r;
+  *code = h ? h : d ? 16 + d : en ? 32 + en : kb ? 48 + kb : (tk ? 64 + tk : 0);
   return 0;
 }
 

@@ -159,12 +159,10 @@ int ladder_pack_v_split(stream_t s, int nv, int a0, int na, int npairs, const in
 // C(m,n) = alpha sum_k A(m,k) B(k,n) + beta C(m,n) over pre-split operands
 // (all with the same slice count): the K sum runs over up to TC_MAX_SEG
 // segments A[s]/B[s], s = 0, 1, ... (the first null A[s] ends the list), each
-// with its own K depth and operands.  A plain FP64 C (no index maps) may be
-// computed in K slices summed in FP64 (to fill the GPU and to bound the FP32
-// accumulation length).  C is FP64, or FP32 when f32, at
-// C[rowoff(m) + coloff(n)] with rowoff(m) = (m % dm)*scm + (m / dm)*scm2
-// (dm = 0: m*scm) and coloff(n) = (n % dn)*scn + (n / dn)*scn2 (dn = 0:
-// n*scn).  Stores are coalesced when scm == 1.
+// with its own K depth and operands.  An FP64 C may be computed in K slices
+// summed in FP64 (to fill the GPU and to bound the FP32 accumulation length).
+// C is FP64, or FP32 when f32, at C[m*scm + n*scn]; stores are coalesced when
+// scm == 1.
 constexpr int TC_MAX_SEG = 4;
 // Longest K one FP32 tensor-memory accumulator sums: FP64 outputs with a
 // longer K are computed in K slices whose partial products are added in FP64;
@@ -177,21 +175,38 @@ struct TcGemm {
   const TcOperand* B[TC_MAX_SEG] = {nullptr, nullptr, nullptr, nullptr};
   void* C = nullptr;
   bool f32 = false;
-  int64_t scm = 1, scn = 0, dn = 0, scn2 = 0, dm = 0, scm2 = 0;
-  // tri > 0 (tc_gemm): as Gemm::tri
+  int64_t scm = 1, scn = 0;
+  // tri > 0: as Gemm::tri
   int64_t tri = 0;
 };
 int tc_gemm(stream_t s, const TcGemm& g);
-// Batched form: `batch` GEMMs of the shape of g (g.A/g.B give the segments
-// and operand shapes), item b reading the operand descriptors mtab[b] (device
-// memory, 64-byte aligned, tc_maps_bytes() each, written by tc_maps_fill on
-// the host from nseg segments A[s]/B[s]) and writing C + b*c_stride through
-// g's index map.  One launch.
-size_t tc_maps_bytes();
-// n: the GEMM's column count (it selects the tile width, as in tc_gemm_batched).
-int tc_maps_fill(int nseg, const TcOperand* const* A, const TcOperand* const* B, int64_t n,
-                 void* host_dst);
-int tc_gemm_batched(stream_t s, const TcGemm& g, int batch, const void* mtab, int64_t c_stride);
+// A stack of `items` operands of equal shape, each as tc_split writes one (two
+// slices), back to back.  tc_split_stack fills it: item i's X(r,k) sits at
+// src[(i % d)*s0 + (i / d)*s1 + rowoff(r) + k*sk], rowoff(r) = (r % dr) + (r /
+// dr)*sr (dr = 0: r*sr).
+struct TcStack {
+  const void* base = nullptr;
+  int64_t rows = 0, k = 0, items = 0;
+};
+int tc_split_stack(stream_t s, const double* src, int64_t rows, int64_t k, int64_t sr, int64_t sk,
+                   int64_t dr, int64_t items, int64_t d, int64_t s0, int64_t s1, void* dst,
+                   TcStack* out);
+// The (T) K builds on the tensor cores (dev_tckbuild.cu): kbuild's products
+// with FP32 C and BF16-split operands; beta adds to C.  pad4: rows of C are
+// followed by room for whole groups of four columns (scn == 1), and every item
+// starts on 16 bytes.  Items run in chunks of `chunk` consecutive ones, which
+// should share operands A.
+struct TcKbuild {
+  int64_t m = 0, n = 0;
+  int nseg = 0;
+  TcStack A[KB_MAX_SEG], B[KB_MAX_SEG];
+  bool beta = false, pad4 = false;
+  float* C = nullptr;
+  int64_t scm = 1, dm = 0, scm2 = 0, scn = 0;
+};
+int tc_kbuild(stream_t s, const TcKbuild& g, int nitems, const KbItem* items, int chunk);
+// Time-out code of its bounded waits (0 = none); reading clears it.
+int tckbuild_error(int* code);
 
 // out = alpha * permute(in) + beta * out.  in has rank nd with dims
 // in_dims (column-major, first fastest); out dimension d is in dimension
@@ -316,7 +331,8 @@ int gemm_splitk_noalloc(stream_t s, char ta, char tb, int64_t m, int64_t n, int6
 // Split-BF16 tensor-core GEMM (tcgen05, FP32 accumulate, ~FP32 accuracy),
 // same interface as gemm().  tc_error() returns and clears the time-out code
 // of the kernels with bounded mbarrier waits (0 = none; 1-4 tensor-core GEMM,
-// 17 TMA-staged FP64 GEMM, 33 FP32 (T) energy kernel, 49 FP64 K builds).
+// 17 TMA-staged FP64 GEMM, 33 FP32 (T) energy kernel, 49 FP64 K builds,
+// 65-68 tensor-core K builds).
 int gemm_mixed(stream_t s, char ta, char tb, int64_t m, int64_t n, int64_t k, double alpha,
                const double* A, int64_t lda, const double* B, int64_t ldb, double beta,
                double* C, int64_t ldc);

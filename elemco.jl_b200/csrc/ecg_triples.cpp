@@ -15,23 +15,21 @@
 // ovoo GEMMs pair up too, and each ovoo pair writes K through the same index
 // map, with the same rows and columns, as one vvvo pair, so every K
 // orientation is one GEMM of four K segments (v, v, o, o; ovoo held negated):
-// three launches per batch of triplets, each with a single pass over K.  The
-// FP64 builds run their rows over the pair index and their columns over a'.
-// On the tensor cores, whose epilogue lanes run along the GEMM rows, the
-// orientation whose a' index is the unit stride of K runs its rows over a'.
-// A fused kernel forms
+// three launches per batch of triplets, each with a single pass over K, with
+// rows over the pair index and columns over a'.  A fused kernel forms
 // X and both energy sums (sum K X and the singles/Fock term sum X Y,
 // cc_triples.jl:113-156); per-triplet energies are summed on the host in
 // triplet order, so the result is deterministic.
 //
 // Mixed precision: every operand is split into two BF16 slices once per call
 // (vvvo in both layouts, T^{xy} per pair, T2[:,:,x,:] and T2[:,:,:,x] per
-// occupied index, -ovoo per pair), the GEMMs run on the tensor cores and K is
+// occupied index, -ovoo per pair; each kind one stack), the GEMMs run on the tensor cores and K is
 // kept in FP32.
 #include "ecg_triples.h"
 
 #include <algorithm>
 #include <cmath>
+#include <tuple>
 #include <vector>
 
 namespace ecg {
@@ -43,41 +41,53 @@ namespace {
 // within ~1e-8 relative of FP64, since the element errors average out.
 constexpr int kTriplesSlices = 2;
 
-// One W GEMM of K = P[W]: amplitudes T^{xy}, integrals of occupied z in the
-// [b,c,d] (l2 = false) or [c,b,d] (l2 = true) layout, and where W[a',n] lands
-// in K: K[a'*scm + (n % dn)*scn + (n / dn)*scn2] (dn = 0: n*scn).
+// One W of K = P[W]: amplitudes T^{xy} and the integrals of occupied z in the
+// [b,c,d] (l2 = false) or [c,b,d] (l2 = true) layout.
 struct PermW {
   int x, y, z;
   bool l2;
-  int64_t scm, scn, dn, scn2;
 };
 
-// n = b' + v c' in the [b,c,d] layout, n = c' + v b' in the [c,b,d] layout.
-// K[a,b,c] sits at a + vp b + vp v c (vp >= v: the padded pitch of the a
-// index; vp = v for FP64 K, a multiple of 4 for FP32 K so that the energy
-// kernel's TMA copies start on 16 bytes).
-void perm_table(int i, int j, int k, int64_t v, int64_t vp, PermW* P) {
-  const int64_t pv = vp * v;
-  P[1] = {j, i, k, false, vp, 1, v, pv};   // W^{jik} -> K[b',a',c'] = vp a' + b' + vp v c'
-  P[4] = {j, k, i, true, vp, 1, v, pv};    // W^{jki} -> K[c',a',b'] = vp a' + c' + vp v b'
-  if (vp == v) {  // unpadded: the column index n maps with one stride
-    P[0] = {i, j, k, false, 1, v, 0, 0};   // W^{ijk} -> K[a',b',c'] = a' + v n
-    P[2] = {i, k, j, true, 1, v, 0, 0};    // W^{ikj} -> K[a',c',b'] = a' + v n
-    P[3] = {k, j, i, true, pv, 1, 0, 0};   // W^{kji} -> K[c',b',a'] = v^2 a' + n
-    P[5] = {k, i, j, false, pv, 1, 0, 0};  // W^{kij} -> K[b',c',a'] = v^2 a' + n
-  } else {
-    P[0] = {i, j, k, false, 1, vp, v, pv};  // K[a',b',c'] = a' + vp b' + vp v c'
-    P[2] = {i, k, j, true, 1, vp, v, pv};   // K[a',c',b'] = a' + vp c' + vp v b'
-    P[3] = {k, j, i, true, pv, 1, v, vp};   // K[c',b',a'] = c' + vp b' + vp v a'
-    P[5] = {k, i, j, false, pv, 1, v, vp};  // K[b',c',a'] = b' + vp c' + vp v a'
-  }
+// W[a',n], n = b' + v c' in the [b,c,d] layout, n = c' + v b' in the [c,b,d]
+// layout.  W^{ijk} and W^{ikj} land at K[a',n], W^{jik} and W^{jki} at K[b',a',c'],
+// W^{kji} and W^{kij} at K[n,a'] (see k_map).
+void perm_table(int i, int j, int k, PermW* P) {
+  P[0] = {i, j, k, false};
+  P[1] = {j, i, k, false};
+  P[2] = {i, k, j, true};
+  P[3] = {k, j, i, true};
+  P[4] = {j, k, i, true};
+  P[5] = {k, i, j, false};
 }
 
-// BF16 operands of one amplitude tensor (T2 or covariant U2).
+constexpr int kGemms = 3;
+// the permutations whose W land in K through one index map
+constexpr int kPairs[kGemms][2] = {{0, 2}, {1, 4}, {3, 5}};
+
+// Where orientation q puts (row n = n0 + v n1, column a') in K[a,b,c], which sits
+// at a + vp b + vp v c (vp >= v: the padded pitch of the a index; vp = v for FP64
+// K, a multiple of 4 for FP32 K so that the energy kernel's TMA copies start on
+// 16 bytes): (n % dm)*scm + (n / dm)*scm2 + a'*scn (dm = 0: n*scm + a'*scn).
+struct KMap {
+  int64_t scm, dm, scm2, scn;
+};
+KMap k_map(int q, int64_t v, int64_t vp) {
+  if (q == 0) return {vp, 0, 0, 1};                      // K[a',n0,n1]
+  if (q == 1) return {1, v, vp * v, vp};                 // K[n0,a',n1]
+  return vp == v ? KMap{1, 0, 0, vp * v} : KMap{1, v, vp, vp * v};  // K[n0,n1,a']
+}
+
+// Consecutive triplets whose tensor-core tiles are interleaved (two that share
+// j and k read a row tile of their vvvo slabs together), and the block of (i, j)
+// the sweep takes triplets in: eight i of four j need 13 slabs of one k, which L2
+// can hold part of, where i running fastest over all needs one slab each.
+constexpr int kChunk = 2, kBlockI = 8, kBlockJ = 4;
+
+// BF16 operands of one amplitude tensor (T2 or covariant U2), as stacks.
 struct SplitAmps {
-  std::vector<dev::TcOperand> pair;  // T^{xy}[a,d]: rows a, k d        (x + o*y)
-  std::vector<dev::TcOperand> G;     // T2[:,:,x,l]: rows (a,b), k l    (x)
-  std::vector<dev::TcOperand> C;     // T2[:,:,l,x]: rows (a,b), k l    (x)
+  dev::TcStack pair;  // T^{xy}[a,d]: rows a, k d        (x + o*y)
+  dev::TcStack G;     // T2[:,:,x,l]: rows (a,b), k l    (x)
+  dev::TcStack C;     // T2[:,:,l,x]: rows (a,b), k l    (x)
 };
 
 uint16_t* alloc_bf16(Ctx& c, size_t elems, const char* what) {
@@ -87,25 +97,15 @@ uint16_t* alloc_bf16(Ctx& c, size_t elems, const char* what) {
 void split_amps(Ctx& c, const double* T, SplitAmps& S) {
   const int64_t o = c.no, v = c.nv, v2 = v * v;
   dev::stream_t s = c.st;
-  S.pair.resize(o * o);
-  S.G.resize(o);
-  S.C.resize(o);
   const size_t ep = dev::tc_operand_elems(v, v, kTriplesSlices);
   const size_t eg = dev::tc_operand_elems(v2, o, kTriplesSlices);
   uint16_t* bp = alloc_bf16(c, ep * o * o, "(T) T^{xy} BF16");
   uint16_t* bg = alloc_bf16(c, 2 * eg * o, "(T) T2 slices BF16");
-  for (int64_t y = 0; y < o; ++y)
-    for (int64_t x = 0; x < o; ++x)
-      check(dev::tc_split(s, T + v2 * (x + o * y), v, v, 1, v, kTriplesSlices,
-                          bp + ep * (x + o * y), &S.pair[x + o * y]),
-            "split T^{xy}");
-  for (int64_t x = 0; x < o; ++x) {
-    check(dev::tc_split(s, T + v2 * x, v2, o, 1, v2 * o, kTriplesSlices, bg + eg * x, &S.G[x]),
-          "split T2 G");
-    check(dev::tc_split(s, T + v2 * o * x, v2, o, 1, v2, kTriplesSlices, bg + eg * (o + x),
-                        &S.C[x]),
-          "split T2 C");
-  }
+  check(dev::tc_split_stack(s, T, v, v, 1, v, 0, o * o, o, v2, v2 * o, bp, &S.pair),
+        "split T^{xy}");
+  check(dev::tc_split_stack(s, T, v2, o, 1, v2 * o, 0, o, o, v2, 0, bg, &S.G), "split T2 G");
+  check(dev::tc_split_stack(s, T, v2, o, 1, v2, 0, o, o, v2 * o, 0, bg + eg * o, &S.C),
+        "split T2 C");
 }
 
 // Everything the K builds read: FP64 integrals, or their BF16 splits.  The
@@ -116,7 +116,7 @@ struct TriplesOps {
   const double* V1 = nullptr;  // [b,c,d,k], (b,c) in pitch v2p
   const double* V2 = nullptr;  // [c,b,d,k], (c,b) in pitch v2p
   const double* On = nullptr;  // -(lj|ck) as [c,l,j,k], c in pitch vq
-  std::vector<dev::TcOperand> V1s, V2s, Ons;
+  dev::TcStack V1s, V2s, Ons;  // rows (b,c) / (c,b), k d (item k); rows c, k l (j + o*k)
 };
 
 // FP64 amplitudes (T2 or covariant U2) as the K builds read them.
@@ -146,99 +146,42 @@ struct Trip {
   double f, eijk;
 };
 
-// Host-built tables of one amplitude tensor's K builds for the whole sweep,
-// uploaded once: FP64 item tables [3 GEMMs][triplet] (the C offset is the
-// triplet's slot in its batch) or tensor-core descriptor tables [3 GEMMs]
-// [triplet][maps of 4 segments].
-struct KTables {
-  std::vector<dev::KbItem> items;
-  std::vector<unsigned char> mtab;
-  dev::KbItem* items_d = nullptr;
-  unsigned char* mtab_d = nullptr;
-};
-
-constexpr int kGemms = 3;
-// the permutations whose W land in K through one index map
-constexpr int kPairs[kGemms][2] = {{0, 2}, {1, 4}, {3, 5}};
-
-void fill_tables(Ctx& c, const TriplesOps& ops, const SplitAmps* Sp, const std::vector<Trip>& tr,
-                 int NB, int64_t kstride, int64_t vp, KTables& kt) {
-  const int64_t o = c.no, v = c.nv, v2 = v * v;
-  const int64_t nt = (int64_t)tr.size();
-  if (!ops.mixed) {
-    kt.items.resize(kGemms * nt);
-    for (int64_t t = 0; t < nt; ++t) {
-      const int i = tr[t].i, j = tr[t].j, k = tr[t].k;
-      PermW P[6];
-      perm_table(i, j, k, v, vp, P);
-      auto on = [&](int y, int z) { return (int32_t)(y + o * z); };
-      // ovoo segments: the occupied index of the T2 slices (see build_K_batch)
-      // and the pair of -ovoo
-      const int32_t ov[3][4] = {{k, j, on(j, i), on(k, i)},
-                                {i, k, on(k, j), on(i, j)},
-                                {i, j, on(j, k), on(i, k)}};
-      for (int q = 0; q < kGemms; ++q) {
-        const PermW &p0 = P[kPairs[q][0]], &p1 = P[kPairs[q][1]];
-        kt.items[q * nt + t] = {{p0.z, p1.z, ov[q][0], ov[q][1]},
-                                {(int32_t)(p0.x + o * p0.y), (int32_t)(p1.x + o * p1.y),
-                                 ov[q][2], ov[q][3]},
-                                (t % NB) * kstride};
-      }
-    }
-    return;
-  }
-  const size_t mb = dev::tc_maps_bytes();
-  kt.mtab.assign(kGemms * nt * mb, 0);
-  auto op = [&](int y, int z) { return &ops.Ons[y + o * z]; };
+// Items of the K builds, [orientation][triplet]: the operand items of the four
+// segments (alike for FP64 arrays and BF16 stacks) and the K slot.
+std::vector<dev::KbItem> k_items(Ctx& c, const std::vector<Trip>& tr, int NB,
+                                 int64_t kstride) {
+  const int64_t o = c.no, nt = (int64_t)tr.size();
+  std::vector<dev::KbItem> items(kGemms * nt);
   for (int64_t t = 0; t < nt; ++t) {
     const int i = tr[t].i, j = tr[t].j, k = tr[t].k;
     PermW P[6];
-    perm_table(i, j, k, v, vp, P);
-    // ovoo pairs (A of both segments, B of both segments) in the order of
-    // the vvvo pairs they share K's index map with
-    const dev::TcOperand* ovoo[3][4] = {
-        {op(j, i), op(k, i), &Sp->C[k], &Sp->G[j]},   // rows a, columns (b,c)
-        {&Sp->G[i], &Sp->C[k], op(k, j), op(i, j)},   // rows (a,c), columns b
-        {&Sp->G[i], &Sp->C[j], op(j, k), op(i, k)}};  // rows (a,b), columns c
+    perm_table(i, j, k, P);
+    auto on = [&](int y, int z) { return (int32_t)(y + o * z); };
+    // ovoo segments: the occupied index of the T2 slices (see build_K_batch)
+    // and the pair of -ovoo
+    const int32_t ov[3][4] = {{k, j, on(j, i), on(k, i)},
+                              {i, k, on(k, j), on(i, j)},
+                              {i, j, on(j, k), on(i, k)}};
     for (int q = 0; q < kGemms; ++q) {
-      const PermW& p0 = P[kPairs[q][0]];
-      const PermW& p1 = P[kPairs[q][1]];
-      const dev::TcOperand* T0 = &Sp->pair[p0.x + o * p0.y];
-      const dev::TcOperand* T1 = &Sp->pair[p1.x + o * p1.y];
-      const dev::TcOperand* V0 = p0.l2 ? &ops.V2s[p0.z] : &ops.V1s[p0.z];
-      const dev::TcOperand* V1 = p1.l2 ? &ops.V2s[p1.z] : &ops.V1s[p1.z];
-      const bool rows_a = p0.scm == 1;
-      const dev::TcOperand* A[4] = {rows_a ? T0 : V0, rows_a ? T1 : V1, ovoo[q][0], ovoo[q][1]};
-      const dev::TcOperand* B[4] = {rows_a ? V0 : T0, rows_a ? V1 : T1, ovoo[q][2], ovoo[q][3]};
-      check(dev::tc_maps_fill(4, A, B, rows_a ? v2 : v, kt.mtab.data() + (q * nt + t) * mb),
-            "maps");
+      const PermW &p0 = P[kPairs[q][0]], &p1 = P[kPairs[q][1]];
+      items[q * nt + t] = {{p0.z, p1.z, ov[q][0], ov[q][1]},
+                           {(int32_t)(p0.x + o * p0.y), (int32_t)(p1.x + o * p1.y), ov[q][2],
+                            ov[q][3]},
+                           (t % NB) * kstride};
     }
   }
-}
-
-void upload_tables(Ctx& c, KTables& kt) {
-  dev::stream_t s = c.st;
-  if (!kt.items.empty()) {
-    const size_t bytes = kt.items.size() * sizeof(dev::KbItem);
-    kt.items_d = reinterpret_cast<dev::KbItem*>(c.alloc((int64_t)(bytes / 8), "(T) item table"));
-    check(dev::h2d(kt.items_d, kt.items.data(), bytes, s), "h2d");
-  }
-  if (!kt.mtab.empty()) {
-    kt.mtab_d = reinterpret_cast<unsigned char*>(
-        c.alloc((int64_t)((kt.mtab.size() + 7) / 8), "(T) descriptor table"));
-    check(dev::h2d(kt.mtab_d, kt.mtab.data(), kt.mtab.size(), s), "h2d");
-  }
+  return items;
 }
 
 // K^{ijk} = P[W] for triplets t0 .. t0+nb-1 into K slots 0 .. nb-1 (FP64 or
 // FP32), one launch per K orientation.
-void build_K_batch(Ctx& c, const TriplesOps& ops, const FpAmps& F, const SplitAmps* Sp,
-                   const KTables& kt, int64_t nt, int64_t t0, int nb, void* K, int64_t kstride,
-                   int64_t vp) {
+void build_K_batch(Ctx& c, const TriplesOps& ops, const FpAmps& F, const SplitAmps& S,
+                   const dev::KbItem* items, int64_t nt, int64_t t0, int nb, void* K,
+                   int64_t kstride, int64_t vp) {
   const int64_t o = c.no, v = c.nv, v2 = v * v;
   dev::stream_t s = c.st;
   PermW P[6];
-  perm_table(0, 0, 0, v, vp, P);  // output maps and layouts do not depend on i, j, k
+  perm_table(0, 0, 0, P);  // the layouts do not depend on i, j, k
   if (!ops.mixed) {
     const int64_t v2p = ops.v2p, vq = ops.vq;
     const dev::KbOperand V1{ops.V1, v2, v2p, o, v2p * v}, V2{ops.V2, v2, v2p, o, v2p * v};
@@ -258,33 +201,27 @@ void build_K_batch(Ctx& c, const TriplesOps& ops, const FpAmps& F, const SplitAm
       g.B[0] = g.B[1] = Tp; g.B[2] = g.B[3] = On;
       g.beta = q ? 1.0 : 0.0;
       g.C = (double*)K;
-      g.scm = p0.scn; g.dm = p0.dn; g.scm2 = p0.scn2; g.scn = p0.scm;
+      const KMap m = k_map(q, v, vp);
+      g.scm = m.scm; g.dm = m.dm; g.scm2 = m.scm2; g.scn = m.scn;
       g.even_items = kstride % 2 == 0;
-      check(dev::kbuild(s, g, nb, kt.items_d + q * nt + t0), "W");
+      check(dev::kbuild(s, g, nb, items + q * nt + t0), "W");
     }
     return;
   }
-  const size_t mb = dev::tc_maps_bytes();
-  auto tab = [&](int q) { return kt.mtab_d + (q * nt + t0) * mb; };
-  // shape representatives (every triplet's operands have the same shapes)
-  const dev::TcOperand* Tp = &Sp->pair[0];
-  const dev::TcOperand* Vp = &ops.V1s[0];
-  const dev::TcOperand* Op = &ops.Ons[0];
-  const dev::TcOperand* Gp = &Sp->G[0];
+  const dev::TcStack* ab[kGemms][2] = {{&S.C, &S.G}, {&S.G, &S.C}, {&S.G, &S.C}};
   for (int q = 0; q < kGemms; ++q) {
-    const PermW& p0 = P[kPairs[q][0]];
-    dev::TcGemm g;
-    g.alpha = 1.0; g.beta = q ? 1.0 : 0.0; g.C = K; g.f32 = true;
-    if (p0.scm == 1) {  // rows a', columns (b',c'); ovoo rows a
-      g.m = v; g.n = v2;
-      g.A[0] = g.A[1] = Tp; g.B[0] = g.B[1] = Vp; g.A[2] = g.A[3] = Op; g.B[2] = g.B[3] = Gp;
-      g.scm = 1; g.scn = p0.scn; g.dn = p0.dn; g.scn2 = p0.scn2;
-    } else {            // rows (b',c'), columns a'; ovoo rows (a,b) or (a,c)
-      g.m = v2; g.n = v;
-      g.A[0] = g.A[1] = Vp; g.B[0] = g.B[1] = Tp; g.A[2] = g.A[3] = Gp; g.B[2] = g.B[3] = Op;
-      g.scm = p0.scn; g.dm = p0.dn; g.scm2 = p0.scn2; g.scn = p0.scm;
-    }
-    check(dev::tc_gemm_batched(s, g, nb, tab(q), kstride), "W");
+    const PermW &p0 = P[kPairs[q][0]], &p1 = P[kPairs[q][1]];
+    dev::TcKbuild g;
+    g.m = v2; g.n = v; g.nseg = 4;
+    g.A[0] = p0.l2 ? ops.V2s : ops.V1s; g.A[1] = p1.l2 ? ops.V2s : ops.V1s;
+    g.A[2] = *ab[q][0]; g.A[3] = *ab[q][1];
+    g.B[0] = g.B[1] = S.pair; g.B[2] = g.B[3] = ops.Ons;
+    g.beta = q > 0;
+    g.C = (float*)K;
+    const KMap m = k_map(q, v, vp);
+    g.scm = m.scm; g.dm = m.dm; g.scm2 = m.scm2; g.scn = m.scn;
+    g.pad4 = vp % 4 == 0 && kstride % 4 == 0;
+    check(dev::tc_kbuild(s, g, nb, items + q * nt + t0, kChunk), "W");
   }
 }
 
@@ -309,34 +246,64 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
   double* On = c.alloc(o * o * o * v, "(T) ovoo");
   Contractor con = c.con();
   con(1.0, c.Boo, "ljQ", c.Bvo, "ckQ", 0.0, On, "ljck");
-  // vvvo[b,c,d,k] = (bd|ck): per k, a GEMM batched over d; [c,b,d,k] by permutation
+  // vvvo[b,c,d,k] = (bd|ck): per k one GEMM over rows (b,d) into a slab
+  // [b,d,c], whose orders [b,c,d] and [c,b,d] the K builds read
   const int64_t d3[3] = {v, v, v};
-  const int swap01[3] = {1, 0, 2};
-  auto build_v = [&](int64_t kk, double* out) {
+  const int bcd[3] = {0, 2, 1}, cbd[3] = {2, 0, 1};
+  const bool pad = ops.v2p != v2;  // odd v: factors and integrals in an even pitch
+  uint16_t *bv = nullptr, *bo = nullptr;
+  double *V1 = nullptr, *V2 = nullptr, *Onp = nullptr;
+  const size_t evs = dev::tc_operand_elems(v2, v, kTriplesSlices);
+  const size_t eos = dev::tc_operand_elems(v, o, kTriplesSlices);
+  const int64_t slab = ops.v2p * v;
+  if (mixed) {
+    bv = alloc_bf16(c, 2 * evs * o, "(T) vvvo BF16");
+    bo = alloc_bf16(c, eos * o * o, "(T) ovoo BF16");
+  } else {
+    V1 = c.alloc(slab * o, "(T) vvvo [b,c,d,k]");
+    V2 = c.alloc(slab * o, "(T) vvvo [c,b,d,k]");
+    Onp = c.alloc(ops.vq * o * o * o, "(T) -ovoo");
+  }
+  const size_t mark = c.allocs.size();
+  double* D = c.alloc(v3, "(T) vvvo slab");
+  double* Dt = mixed || pad ? c.alloc(v3, "(T) vvvo slab") : nullptr;
+  const double* Bl = c.Bvv;
+  if (pad) {
+    double* t = c.alloc(ops.v2p * c.nq, "(T) padded Bvv");
+    check(dev::repitch(s, v2, c.nq, c.Bvv, v2, t, ops.v2p), "pad Bvv");
+    Bl = t;
+  }
+  for (int64_t kk = 0; kk < o; ++kk) {
     dev::Gemm g;
-    g.m = v; g.n = v; g.k = c.nq; g.batch = v; g.alpha = 1.0; g.beta = 0.0;
-    g.A = c.Bvv; g.sam = 1; g.sak = v * v; g.sab = v;
-    g.B = c.Bvo + v * kk; g.sbk = v * o; g.sbn = 1; g.sbb = 0;
-    g.C = out; g.scm = 1; g.scn = v; g.scb = v * v;
+    g.m = v2; g.n = v; g.k = c.nq;
+    g.A = Bl; g.sam = 1; g.sak = ops.v2p;
+    g.B = c.Bvo + v * kk; g.sbn = 1; g.sbk = v * o;
+    g.C = D; g.scn = v2;
     check(dev::gemm_strided(s, g), "vvvo");
-  };
-  if (!mixed) {
-    const int64_t slab = ops.v2p * v;
-    double* V1 = c.alloc(slab * o, "(T) vvvo [b,c,d,k]");
-    double* V2 = c.alloc(slab * o, "(T) vvvo [c,b,d,k]");
-    double* Onp = c.alloc(ops.vq * o * o * o, "(T) -ovoo");
-    const bool pad = ops.v2p != v2;  // dense slabs first, then copies in the even pitch
-    double* Vt = pad ? c.alloc(2 * v3, "(T) vvvo slabs") : nullptr;
-    for (int64_t kk = 0; kk < o; ++kk) {
-      double* d1 = pad ? Vt : V1 + slab * kk;
-      double* d2 = pad ? Vt + v3 : V2 + slab * kk;
-      build_v(kk, d1);
-      check(dev::permute(s, 3, d3, swap01, 1.0, d1, 0.0, d2), "vvvo perm");
-      if (!pad) continue;
-      check(dev::repitch(s, v2, v, d1, v2, V1 + slab * kk, ops.v2p), "pad vvvo");
-      check(dev::repitch(s, v2, v, d2, v2, V2 + slab * kk, ops.v2p), "pad vvvo");
+    if (mixed) {
+      check(dev::tc_split_stack(s, D, v2, v, v2, v, v, 1, 1, 0, 0, bv + evs * kk, &ops.V1s),
+            "split vvvo");
+      check(dev::permute(s, 3, d3, cbd, 1.0, D, 0.0, Dt), "vvvo perm");
+      check(dev::tc_split_stack(s, Dt, v2, v, 1, v2, 0, 1, 1, 0, 0, bv + evs * (o + kk),
+                                &ops.V2s),
+            "split vvvo");
+      continue;
     }
-    // -ovoo as [c,l,j,k]
+    for (int w = 0; w < 2; ++w) {
+      double* V = (w ? V2 : V1) + slab * kk;
+      check(dev::permute(s, 3, d3, w ? cbd : bcd, 1.0, D, 0.0, pad ? Dt : V), "vvvo perm");
+      if (pad) check(dev::repitch(s, v2, v, Dt, v2, V, ops.v2p), "pad vvvo");
+    }
+  }
+  // -ovoo: the ovoo segments share the vvvo segments' sign
+  if (mixed) {
+    check(dev::axpby(s, o * o * o * v, -1.0, On, 0.0, On), "-ovoo");
+    check(dev::tc_split_stack(s, On, v, o, o * o, 1, 0, o * o, o, o, o * o * v, bo, &ops.Ons),
+          "split ovoo");
+    ops.V1s.base = bv;
+    ops.V2s.base = bv + evs * o;
+    ops.V1s.items = ops.V2s.items = o;
+  } else {  // as [c,l,j,k]
     const int64_t dl[4] = {o, o, v, o};
     const int pl[4] = {2, 0, 1, 3};
     double* Oc = c.alloc(o * o * o * v, "(T) ovoo [c,l,j,k]");
@@ -345,37 +312,8 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
     ops.V1 = V1;
     ops.V2 = V2;
     ops.On = Onp;
-  } else {
-    const size_t evs = dev::tc_operand_elems(v2, v, kTriplesSlices);
-    const size_t eos = dev::tc_operand_elems(v, o, kTriplesSlices);
-    uint16_t* bv = alloc_bf16(c, 2 * evs * o, "(T) vvvo BF16");
-    uint16_t* bo = alloc_bf16(c, eos * o * o, "(T) ovoo BF16");
-    const size_t mark = c.allocs.size();
-    double* Vt = c.alloc(v3, "(T) vvvo slab");
-    double* Vt2 = c.alloc(v3, "(T) vvvo slab");
-    ops.V1s.resize(o);
-    ops.V2s.resize(o);
-    ops.Ons.resize(o * o);
-    for (int64_t kk = 0; kk < o; ++kk) {
-      build_v(kk, Vt);
-      check(dev::tc_split(s, Vt, v2, v, 1, v2, kTriplesSlices, bv + evs * kk, &ops.V1s[kk]),
-            "split vvvo");
-      check(dev::permute(s, 3, d3, swap01, 1.0, Vt, 0.0, Vt2), "vvvo perm");
-      check(dev::tc_split(s, Vt2, v2, v, 1, v2, kTriplesSlices, bv + evs * (o + kk),
-                          &ops.V2s[kk]),
-            "split vvvo");
-    }
-    // -ovoo: the ovoo segments share the vvvo GEMMs' alpha = 1 (the BF16
-    // split of -x is the negated split of x)
-    check(dev::axpby(s, o * o * o * v, -1.0, On, 0.0, On), "-ovoo");
-    for (int64_t z = 0; z < o; ++z)
-      for (int64_t y = 0; y < o; ++y)
-        check(dev::tc_split(s, On + o * y + o * o * v * z, v, o, o * o, 1, kTriplesSlices,
-                            bo + eos * (y + o * z), &ops.Ons[y + o * z]),
-              "split ovoo");
-    check(dev::sync(s), "sync");
-    c.release_to(mark);
   }
+  c.release_to(mark);
 
   double* U2c = nullptr;
   if (lam) {
@@ -397,16 +335,20 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
     if (lam) split_amps(c, U2c, SU);
   }
 
-  // the sweep: triplet order and weights of cc_triples.jl:62-72
+  // the sweep: triplet weights of cc_triples.jl:62-72, taken in blocks of (i, j)
+  // that share integrals; energies are summed in the reference's order (k, j,
+  // i outermost first)
   const double* eps = c.fock_host.data();
   std::vector<Trip> tr;
   for (int k = 0; k < o; ++k)
-    for (int j = 0; j <= k; ++j)
-      for (int i = 0; i <= j; ++i) {
-        if (i == j && j == k) continue;
-        const double f = (i == j) ? 1.0 : (j == k ? 1.0 : 2.0);
-        tr.push_back({i, j, k, f, eps[i + i * n] + eps[j + j * n] + eps[k + k * n]});
-      }
+    for (int j0 = 0; j0 <= k; j0 += kBlockJ)
+      for (int i0 = 0; i0 <= std::min(j0 + kBlockJ - 1, k); i0 += kBlockI)
+        for (int j = j0; j < std::min(j0 + kBlockJ, k + 1); ++j)
+          for (int i = i0; i < std::min(i0 + kBlockI, j + 1); ++i) {
+            if (i == j && j == k) continue;
+            const double f = (i == j) ? 1.0 : (j == k ? 1.0 : 2.0);
+            tr.push_back({i, j, k, f, eps[i + i * n] + eps[j + j * n] + eps[k + k * n]});
+          }
   const int64_t nt = (int64_t)tr.size();
   if (nt == 0) {
     *et = *etb = 0.0;
@@ -414,7 +356,7 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
   }
   // batches of NB triplets, one K slot each, within a 4 GiB budget
   const int64_t esz = mixed ? 4 : 8;
-  const int64_t vp = mixed ? (v + 3) / 4 * 4 : v;  // K's a pitch (see perm_table)
+  const int64_t vp = mixed ? (v + 3) / 4 * 4 : v;  // K's a pitch (see k_map)
   const int64_t kstride = (vp * v2 + 31) / 32 * 32;
   const int64_t per = kstride * esz * (lam ? 2 : 1);
   int64_t nbmax = std::min<int64_t>({256, nt, ((int64_t)4 << 30) / per});
@@ -422,13 +364,11 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
   const int NB = (int)std::max<int64_t>(1, nbmax);
   void* K = c.alloc((NB * kstride * esz + 7) / 8, "(T) K slots");
   void* KU = lam ? (void*)c.alloc((NB * kstride * esz + 7) / 8, "(T) K(Lambda) slots") : nullptr;
-  KTables KT, KUt;
-  fill_tables(c, ops, &ST, tr, NB, kstride, vp, KT);
-  upload_tables(c, KT);
-  if (lam) {
-    fill_tables(c, ops, &SU, tr, NB, kstride, vp, KUt);
-    upload_tables(c, KUt);
-  }
+  const std::vector<dev::KbItem> items = k_items(c, tr, NB, kstride);
+  static_assert(sizeof(dev::KbItem) % 8 == 0, "whole doubles");
+  dev::KbItem* items_d = reinterpret_cast<dev::KbItem*>(
+      c.alloc((int64_t)(items.size() * sizeof(dev::KbItem) / 8), "(T) item table"));
+  check(dev::h2d(items_d, items.data(), items.size() * sizeof(dev::KbItem), s), "h2d");
 
   // energy terms per triplet: g = T1 (or U1/2), f[a,i] = fock[i, o+a], <ij|ab>, T2 (or U2c)
   std::vector<double> gh(v * o), fh(v * o);
@@ -515,8 +455,8 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
       if (bi == 1) check(dev::graph_capture_begin(s), "graph capture");
       const int64_t t0 = bi * NB;
       const int nb = (int)std::min<int64_t>(NB, nt - t0);
-      build_K_batch(c, ops, FT, &ST, KT, nt, t0, nb, K, kstride, vp);
-      if (lam) build_K_batch(c, ops, FU, &SU, KUt, nt, t0, nb, KU, kstride, vp);
+      build_K_batch(c, ops, FT, ST, items_d, nt, t0, nb, K, kstride, vp);
+      if (lam) build_K_batch(c, ops, FU, SU, items_d, nt, t0, nb, KU, kstride, vp);
       if (mixed)
         check(dev::triples_energy_f32_batched(s, (int)v, (int)vp, nb, NB,
                                               static_cast<const float*>(K),
@@ -545,7 +485,12 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
   if (tc) throw Error(ECG_ERR_TIMEOUT, "GEMM wait timed out in (T) (code " + std::to_string(tc) + ")");
   // sum K X, and the singles / Fock term sum X Y (cc_triples.jl:143-156 / :286-294)
   double Enb3 = 0.0, Esf = 0.0;
-  for (int64_t q = 0; q < nt; ++q) {
+  std::vector<int64_t> order(nt);
+  for (int64_t q = 0; q < nt; ++q) order[q] = q;
+  std::sort(order.begin(), order.end(), [&](int64_t x, int64_t y) {
+    return std::tie(tr[x].k, tr[x].j, tr[x].i) < std::tie(tr[y].k, tr[y].j, tr[y].i);
+  });
+  for (int64_t q : order) {
     Enb3 += tr[q].f * Eh[2 * q];
     Esf += tr[q].f * Eh[2 * q + 1];
   }

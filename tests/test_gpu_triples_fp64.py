@@ -47,3 +47,25 @@ def test_pert_t_matches_restatement(ctx, no, nv, nq):
     got = ctx.pert_t(T1, np.asfortranarray(d.T2))
     # sums of ~nv^3 terms of either sign: 1e-12 of the energy's size
     assert abs(got[0] - ref[0]) < 1e-12 and abs(got[1] - ref[1]) < 1e-12
+
+
+@pytest.mark.parametrize("no,nv,nq", [(2, 9, 30), (4, 33, 60), (3, 64, 80), (3, 129, 90),
+                                      (7, 100, 110), (2, 257, 60), (2, 300, 60)])
+def test_mixed_pert_t_matches_fp64(ctx, no, nv, nq):
+    """Tensor-core tile widths at their edges (one tile of 16 to 256 columns, two
+    beyond), chunks of triplets that are full and not."""
+    import ecgpu
+    B, h1, e0 = _system(no, nv, nq)
+    ctx.set_system(B, h1, e0, no)
+    _, T1, T2 = ctx.mp2()
+    T1 = 0.02 * np.random.default_rng(nv).standard_normal((nv, no))
+    ref = ctx.pert_t(T1, T2)
+    ctx.set_precision(ecgpu.ECG_PREC_MIXED)
+    try:
+        got = ctx.pert_t(T1, T2)
+        assert ctx.pert_t(T1, T2) == got
+    finally:
+        ctx.set_precision(ecgpu.ECG_PREC_FP64)
+    # two-slice products, 2^-16 of each term, averaging over v^3 of them
+    for x, y in zip(got, ref):
+        assert abs(x - y) < 2e-5 * abs(y)
