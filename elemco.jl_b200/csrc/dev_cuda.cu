@@ -1388,13 +1388,56 @@ int update_singles(stream_t s, int nv, int no, const double* eo, const double* e
   return launched();
 }
 
+// T and R are vectors [singles | doubles]; one pass reads both once and writes
+// T, and the copies that the DIIS keeps (four launches before: two updates and
+// two copies, which read T and R again).
+__global__ void update_save_kernel(int nv, int no, const double* __restrict__ eo,
+                                   const double* __restrict__ ev, double shifts, double shiftp,
+                                   const double* __restrict__ R, double* __restrict__ T,
+                                   double* __restrict__ Ts, double* __restrict__ Rs) {
+  const uint32_t v = nv, o = no, n1 = v * o;
+  const int64_t n = n1 + (int64_t)n1 * n1;
+  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < n;
+       idx += (int64_t)gridDim.x * blockDim.x) {
+    double den;
+    if (idx < n1) {
+      const uint32_t i = (uint32_t)idx / v, a = (uint32_t)idx - i * v;
+      den = ev[a] - eo[i] + shifts;
+    } else {
+      const int64_t x = idx - n1;
+      // x = a + v (b + v (i + o j)): split in halves that fit 32 bits
+      const uint32_t ij = (uint32_t)(x / ((int64_t)v * v));
+      const uint32_t ab = (uint32_t)(x - (int64_t)ij * v * v);
+      const uint32_t b = ab / v, a = ab - b * v, j = ij / o, i = ij - j * o;
+      den = ev[a] + ev[b] - eo[i] - eo[j] + shiftp;
+    }
+    const double r = R[idx], t = T[idx] - r / den;
+    T[idx] = t;
+    Ts[idx] = t;
+    Rs[idx] = r;
+  }
+}
+
+int update_save(stream_t s, int nv, int no, const double* eo, const double* ev, double shifts,
+                double shiftp, const double* R, double* T, double* Tsave, double* Rsave) {
+  if (nv <= 0 || no <= 0 || (int64_t)nv * nv >= ((int64_t)1 << 31))
+    return (int)cudaErrorInvalidValue;
+  const int64_t n1 = (int64_t)nv * no;
+  update_save_kernel<<<grid_for(n1 + n1 * n1), 256, 0, (cudaStream_t)s>>>(
+      nv, no, eo, ev, shifts, shiftp, R, T, Tsave, Rsave);
+  return launched();
+}
+
 // ---------------------------------------------------------------- reductions
 //
-// Fixed grid (RED_BLOCKS x 256) + a single-block final pass in a fixed order:
-// results are bitwise reproducible run to run.
+// A fixed number of blocks per job leaves partial sums, and the job's last
+// block adds them in a fixed order: results are bitwise reproducible run to
+// run.  All dots of a step share one launch: a CCSD iteration needed 46 launches
+// (partial and final sums one by one), which at small sizes cost as much as its
+// products.
 
 static constexpr int RED_BLOCKS = 592;
-int64_t reduce_scratch_len() { return 2 * RED_BLOCKS; }
+int64_t reduce_scratch_len() { return (int64_t)DOT_MAX * 2 * RED_BLOCKS + DOT_MAX; }
 
 __device__ __forceinline__ double block_sum(double v, double* sh) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -1410,93 +1453,276 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
   return r;
 }
 
-__global__ void dot_partial_kernel(int64_t n, const double* x, const double* y, double* part) {
-  __shared__ double sh[32];
-  double acc = 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    acc += x[i] * y[i];
-  double r = block_sum(acc, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = r;
-}
+struct DotJobs {
+  DotJob j[DOT_MAX];
+  int blocks[DOT_MAX];
+};
 
-// Partial sums of <X|Y> and <X^T|Y> (X^T[a,b,i,j] = X[b,a,i,j]) over 32 x 32
-// tiles of each (a,b) slice: the block reads the tile of X and Y and the
-// mirrored tile of X, all coalesced, and takes the transposed elements from
-// shared memory.  Tiles go to blocks in a fixed order, so the sums are
-// deterministic.
-__global__ void cs_dot_partial_kernel(int nv, int no, const double* X, const double* Y,
-                                      double* part) {
+// <X|Y> and <X^T|Y> (X^T[a,b,i,j] = X[b,a,i,j]) over 32 x 32 tiles of each (a,b)
+// slice: the block reads the tile of X and Y and the mirrored tile of X, all
+// coalesced, and takes the transposed elements from shared memory.
+__global__ void dots_kernel(int nv, int no, DotJobs jobs, double* part, unsigned* done) {
   __shared__ double sh[32];
   __shared__ double xt[32][33];
-  const int64_t vv = (int64_t)nv * nv;
-  const uint32_t T = (uint32_t)(nv + 31) / 32, ntile = T * T * (uint32_t)no * (uint32_t)no;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
+  __shared__ bool last;
+  const int q = blockIdx.y, nb = jobs.blocks[q];
+  if ((int)blockIdx.x >= nb) return;
+  const DotJob J = jobs.j[q];
   double d = 0.0, ex = 0.0;
-  for (uint32_t t = blockIdx.x; t < ntile; t += gridDim.x) {
-    const uint32_t ta = t % T, tb = (t / T) % T, ij = t / (T * T);
-    const double* Xs = X + ij * vv;
-    const double* Ys = Y + ij * vv;
-    const int a0 = ta * 32, b0 = tb * 32;
-    // all twelve loads of a thread are issued before any of them is used:
-    // xt[j][tx] = X[b0 + tx, a0 + j], and X, Y at (a0 + tx, b0 + j)
-    double rt[4], rx[4], ry[4];
+  if (J.type == DOT_PLAIN) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < J.n;
+         i += (int64_t)nb * blockDim.x)
+      d += J.X[i] * J.Y[i];
+  } else {
+    const int64_t vv = (int64_t)nv * nv;
+    const uint32_t T = (uint32_t)(nv + 31) / 32, ntile = T * T * (uint32_t)no * (uint32_t)no;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
+    const bool t1 = J.type == DOT_CS_T1;
+    for (uint32_t t = blockIdx.x; t < ntile; t += nb) {
+      const uint32_t ta = t % T, tb = (t / T) % T, ij = t / (T * T);
+      const double* Xs = t1 ? J.X : J.X + ij * vv;
+      const double* Ys = J.Y + ij * vv;
+      const int a0 = ta * 32, b0 = tb * 32;
+      // the products' singles columns i, j of a T1 job
+      const double* ti = J.X + (int64_t)nv * (ij % no);
+      const double* tj = J.X + (int64_t)nv * (ij / no);
+      // all twelve loads of a thread are issued before any of them is used:
+      // xt[j][tx] = X[b0 + tx, a0 + j], and X, Y at (a0 + tx, b0 + j)
+      double rt[4], rx[4], ry[4];
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
-      const int j = ty + 8 * jj, a = a0 + tx, b = b0 + j;
-      rt[jj] = (b0 + tx < nv && a0 + j < nv) ? Xs[(b0 + tx) + (int64_t)nv * (a0 + j)] : 0.0;
-      const bool in = a < nv && b < nv;
-      const int64_t i = a + (int64_t)nv * b;
-      rx[jj] = in ? Xs[i] : 0.0;
-      ry[jj] = in ? Ys[i] : 0.0;
+      for (int jj = 0; jj < 4; ++jj) {
+        const int j = ty + 8 * jj, a = a0 + tx, b = b0 + j;
+        const bool tr = b0 + tx < nv && a0 + j < nv, in = a < nv && b < nv;
+        const int64_t i = a + (int64_t)nv * b;
+        if (t1) {
+          rt[jj] = tr ? ti[b0 + tx] * tj[a0 + j] : 0.0;
+          rx[jj] = in ? ti[a] * tj[b] : 0.0;
+        } else {
+          rt[jj] = tr ? Xs[(b0 + tx) + (int64_t)nv * (a0 + j)] : 0.0;
+          rx[jj] = in ? Xs[i] : 0.0;
+        }
+        ry[jj] = in ? Ys[i] : 0.0;
+      }
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) xt[ty + 8 * jj][tx] = rt[jj];
+      __syncthreads();
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        d += rx[jj] * ry[jj];
+        ex += xt[tx][ty + 8 * jj] * ry[jj];  // X[b, a]
+      }
+      __syncthreads();
     }
-#pragma unroll
-    for (int jj = 0; jj < 4; ++jj) xt[ty + 8 * jj][tx] = rt[jj];
-    __syncthreads();
-#pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
-      d += rx[jj] * ry[jj];
-      ex += xt[tx][ty + 8 * jj] * ry[jj];  // X[b, a]
-    }
-    __syncthreads();
   }
-  double r0 = block_sum(d, sh);
-  double r1 = block_sum(ex, sh);
+  const int nout = J.type == DOT_PLAIN ? 1 : 2;
+  double* pq = part + (int64_t)q * 2 * RED_BLOCKS;
+  const double r0 = block_sum(d, sh);
+  const double r1 = nout > 1 ? block_sum(ex, sh) : 0.0;
   if (threadIdx.x == 0) {
-    part[blockIdx.x] = r0;
-    part[RED_BLOCKS + blockIdx.x] = r1;
+    pq[blockIdx.x] = r0;
+    if (nout > 1) pq[RED_BLOCKS + blockIdx.x] = r1;
+    __threadfence();
+    last = atomicAdd(&done[q], 1u) == (unsigned)(nb - 1);
   }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int c = 0; c < nout; ++c) {
+    double acc = 0.0;
+    for (int i = threadIdx.x; i < nb; i += blockDim.x)
+      acc += *(volatile double*)&pq[c * RED_BLOCKS + i];
+    const double r = block_sum(acc, sh);
+    if (threadIdx.x == 0) J.out[c] = r;
+  }
+  if (threadIdx.x == 0) done[q] = 0;  // ready for the next launch
 }
 
-__global__ void final_sum_kernel(int nparts, int nout, const double* part, double* out) {
-  __shared__ double sh[32];
-  for (int o = 0; o < nout; ++o) {
-    double acc = 0.0;
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x) acc += part[o * RED_BLOCKS + i];
-    double r = block_sum(acc, sh);
-    if (threadIdx.x == 0) out[o] = r;
+int dots(stream_t s, int nv, int no, int njobs, const DotJob* jobs, double* scratch) {
+  if (njobs <= 0) return 0;
+  if (njobs > DOT_MAX) return (int)cudaErrorInvalidValue;
+  const uint64_t T = ((uint64_t)nv + 31) / 32, tiles = T * T * (uint64_t)no * (uint64_t)no;
+  DotJobs a{};
+  int most = 1;
+  for (int q = 0; q < njobs; ++q) {
+    a.j[q] = jobs[q];
+    if (jobs[q].type != DOT_PLAIN && tiles >= ((uint64_t)1 << 32) - RED_BLOCKS)
+      return (int)cudaErrorInvalidValue;  // tile index beyond 32 bits
+    const int64_t w = jobs[q].type == DOT_PLAIN ? (jobs[q].n + 1023) / 1024 : (int64_t)tiles;
+    a.blocks[q] = (int)std::max<int64_t>(1, std::min<int64_t>(w, RED_BLOCKS));
+    most = std::max(most, a.blocks[q]);
   }
+  dots_kernel<<<dim3((unsigned)most, (unsigned)njobs), 256, 0, (cudaStream_t)s>>>(
+      nv, no, a, scratch, (unsigned*)(scratch + (int64_t)DOT_MAX * 2 * RED_BLOCKS));
+  return launched();
 }
 
 int dot(stream_t s, int64_t n, const double* x, const double* y, double* scratch, double* out) {
-  cudaStream_t st = (cudaStream_t)s;
-  dot_partial_kernel<<<RED_BLOCKS, 256, 0, st>>>(n, x, y, scratch);
-  int e = launched();
-  if (e) return e;
-  final_sum_kernel<<<1, 256, 0, st>>>(RED_BLOCKS, 1, scratch, out);
-  return launched();
+  const DotJob j{DOT_PLAIN, x, y, n, out};
+  return dots(s, 1, 1, 1, &j, scratch);
 }
 
 int cs_dot(stream_t s, int nv, int no, const double* X, const double* Y, double* scratch,
            double* out) {
-  cudaStream_t st = (cudaStream_t)s;
-  const uint64_t T = ((uint64_t)nv + 31) / 32;
-  if (T * T * (uint64_t)no * (uint64_t)no >= ((uint64_t)1 << 32) - RED_BLOCKS)
-    return (int)cudaErrorInvalidValue;  // tile index beyond 32 bits
-  cs_dot_partial_kernel<<<RED_BLOCKS, 256, 0, st>>>(nv, no, X, Y, scratch);
-  int e = launched();
-  if (e) return e;
-  final_sum_kernel<<<1, 256, 0, st>>>(RED_BLOCKS, 2, scratch, out);
+  const DotJob j{DOT_CS, X, Y, 0, out};
+  return dots(s, nv, no, 1, &j, scratch);
+}
+
+// ---------------------------------------------------------------- ring terms
+
+// A warp per row a of (b, i, j): both orders of i, j are read and four rows
+// written, all contiguous.  Bound by memory: 2 reads (the second hits L2 where
+// two pairs' slices fit) and 4 writes of n2.
+__global__ void ring_split_kernel(int nv, int no, const double* __restrict__ T2,
+                                  double* __restrict__ X1, double* __restrict__ X2,
+                                  double* __restrict__ Xt, double* __restrict__ Tt) {
+  const uint32_t v = nv, o = no, rows = v * o * o, lane = threadIdx.x & 31;
+  const uint32_t nwarp = gridDim.x * (blockDim.x >> 5);
+  for (uint32_t r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += nwarp) {
+    const uint32_t b = r % v, ij = r / v, j = ij / o, i = ij - j * o;
+    const double* s1 = T2 + (int64_t)r * v;
+    const double* s2 = T2 + (int64_t)(b + v * (j + o * i)) * v;
+    const int64_t x0 = (int64_t)(i + o * (b + v * j)) * v;
+    double* tt = Tt + (int64_t)r * v;
+    for (uint32_t a = lane; a < v; a += 32) {
+      const double p = s1[a], q = s2[a], m = 2.0 * p - q;
+      X1[x0 + a] = p;
+      X2[x0 + a] = q;
+      Xt[x0 + a] = m;
+      tt[a] = m;
+    }
+  }
+}
+
+int ring_split(stream_t s, int nv, int no, const double* T2, double* X1, double* X2, double* Xt,
+               double* Tt) {
+  const int64_t rows = (int64_t)nv * no * no;
+  if (rows <= 0) return 0;
+  if (rows >= ((int64_t)1 << 32) - 8 * 148 * 16) return (int)cudaErrorInvalidValue;
+  ring_split_kernel<<<(unsigned)std::min<int64_t>((rows + 7) / 8, 148 * 16), 256, 0,
+                      (cudaStream_t)s>>>(nv, no, T2, X1, X2, Xt, Tt);
+  return launched();
+}
+
+__global__ void ring_combine_kernel(int64_t n, double* __restrict__ W, double* __restrict__ Y,
+                                    double* __restrict__ Z, const double* __restrict__ Q) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const double w = W[i], z = Z[i], y = Q ? Y[i] : 0.0, q = Q ? Q[i] : 0.0;
+    W[i] = y - w;
+    Y[i] = 2.0 * w - y - z;
+    Z[i] = 0.5 * q - z;
+  }
+}
+
+int ring_combine(stream_t s, int64_t n, double* W, double* Y, double* Z, const double* Q) {
+  if (n <= 0) return 0;
+  ring_combine_kernel<<<grid_for(n), 256, 0, (cudaStream_t)s>>>(n, W, Y, Z, Q);
+  return launched();
+}
+
+// 32 x 32 tiles of (a, b) for one (i, j): the terms with a as their fastest index
+// are read as they lie, those with b through shared memory.
+__global__ void ring_add_kernel(int nv, int no, const double* __restrict__ D,
+                                const double* __restrict__ E, double* __restrict__ R2) {
+  __shared__ double tr[32][33];
+  const uint32_t v = nv, o = no, T = (v + 31) / 32, ntile = T * T * o * o;
+  const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
+  const int64_t vo = (int64_t)v * o, vvo = vo * v;
+  for (uint32_t t = blockIdx.x; t < ntile; t += gridDim.x) {
+    const uint32_t ta = t % T, tb = (t / T) % T, ij = t / (T * T), j = ij / o, i = ij - j * o;
+    const uint32_t a0 = ta * 32, b0 = tb * 32;
+    const double* D1 = D + (int64_t)v * i + vvo * j;  // a + vo b
+    const double* D2 = D + (int64_t)v * j + vvo * i;  // b + vo a
+    const double* E1 = E + (int64_t)v * i + vvo * j;  // b + vo a
+    const double* E2 = E + (int64_t)v * j + vvo * i;  // a + vo b
+    double p[4], q[4], x[4], y[4], r[4];
+    double* R = R2 + (int64_t)ij * v * v;
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) {
+      const uint32_t y0 = ty + 8 * jj;
+      const bool tin = b0 + tx < v && a0 + y0 < v, in = a0 + tx < v && b0 + y0 < v;
+      const int64_t f = (int64_t)(b0 + tx) + vo * (a0 + y0), g = (int64_t)(a0 + tx) + vo * (b0 + y0);
+      p[jj] = tin ? D2[f] : 0.0;
+      q[jj] = tin ? E1[f] : 0.0;
+      x[jj] = in ? D1[g] : 0.0;
+      y[jj] = in ? E2[g] : 0.0;
+      r[jj] = in ? R[(a0 + tx) + (int64_t)v * (b0 + y0)] : 0.0;
+    }
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) tr[ty + 8 * jj][tx] = p[jj] + q[jj];  // [a - a0][b - b0]
+    __syncthreads();
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) {
+      const uint32_t y0 = ty + 8 * jj;
+      if (a0 + tx < v && b0 + y0 < v)
+        R[(a0 + tx) + (int64_t)v * (b0 + y0)] = r[jj] + (x[jj] + y[jj] + tr[tx][y0]);
+    }
+    __syncthreads();
+  }
+}
+
+int ring_add(stream_t s, int nv, int no, const double* D, const double* E, double* R2) {
+  const int64_t T = ((int64_t)nv + 31) / 32, tiles = T * T * no * no;
+  if (tiles <= 0) return 0;
+  if (tiles >= ((int64_t)1 << 32) - 148 * 16) return (int)cudaErrorInvalidValue;
+  ring_add_kernel<<<(unsigned)std::min<int64_t>(tiles, 148 * 16), dim3(32, 8), 0,
+                    (cudaStream_t)s>>>(nv, no, D, E, R2);
+  return launched();
+}
+
+// 32 elements a block, their sums over Q shared by its eight warps (added in a
+// fixed order): one launch for the Coulomb sums, the exchange sums' addition
+// and the block copies of all four blocks.
+__global__ void fock_blocks_kernel(int no, int nv, int nq, const double* __restrict__ dh,
+                                   const double* __restrict__ Boo, const double* __restrict__ Bvo,
+                                   const double* __restrict__ Bov, const double* __restrict__ Bvv,
+                                   const double* __restrict__ J, const double* __restrict__ G,
+                                   double* __restrict__ f, double* __restrict__ foo,
+                                   double* __restrict__ fvo, double* __restrict__ fov,
+                                   double* __restrict__ fvv) {
+  __shared__ double sh[8][33];
+  const int64_t o = no, v = nv, n = o + v, oo = o * o, vo = v * o;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int64_t total = n * n;
+  for (int64_t e0 = (int64_t)blockIdx.x * 32; e0 < total; e0 += (int64_t)gridDim.x * 32) {
+    const int64_t e = e0 + tx;  // dense blocks oo, vo, ov, vv back to back
+    const int k = e < oo ? 0 : e < oo + vo ? 1 : e < oo + 2 * vo ? 2 : 3;
+    const int64_t x = k == 0 ? e : k == 1 ? e - oo : k == 2 ? e - oo - vo : e - oo - 2 * vo;
+    const double* B = k == 0 ? Boo : k == 1 ? Bvo : k == 2 ? Bov : Bvv;
+    const int64_t rows = k == 0 || k == 2 ? o : v, len = k == 0 ? oo : k == 3 ? v * v : vo;
+    double s0 = 0.0, s1 = 0.0;
+    if (e < total) {
+      int q = ty;
+      for (; q + 8 < nq; q += 16) {
+        s0 += B[x + len * q] * J[q];
+        s1 += B[x + len * (q + 8)] * J[q + 8];
+      }
+      if (q < nq) s0 += B[x + len * q] * J[q];
+    }
+    sh[ty][tx] = s0 + s1;
+    __syncthreads();
+    if (ty == 0 && e < total) {
+      double s = 0.0;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) s += sh[w][tx];
+      const int64_t c = x / rows, r = x - c * rows;
+      const int64_t i = r + (k & 1 ? o : 0), jn = c + (k >= 2 ? o : 0);
+      const double val = dh[i + n * jn] + 2.0 * s + G[e];
+      f[i + n * jn] = val;
+      if (k == 2) fov[c + v * r] = val;
+      else (k == 0 ? foo : k == 1 ? fvo : fvv)[x] = val;
+    }
+    __syncthreads();
+  }
+}
+
+int fock_blocks(stream_t s, int no, int nv, int nq, const double* dh, const double* Boo,
+                const double* Bvo, const double* Bov, const double* Bvv, const double* J,
+                const double* G, double* f, double* foo, double* fvo, double* fov, double* fvv) {
+  const int64_t n = (int64_t)no + nv, b = (n * n + 31) / 32;
+  fock_blocks_kernel<<<(unsigned)std::min<int64_t>(b, 148 * 64), dim3(32, 8), 0,
+                       (cudaStream_t)s>>>(no, nv, nq, dh, Boo, Bvo, Bov, Bvv, J, G, f,
+                                                  foo, fvo, fov, fvv);
   return launched();
 }
 
@@ -1542,13 +1768,14 @@ int outer(stream_t s, int64_t na, int64_t ni, int64_t nb, int64_t nj, double alp
 
 struct CombineArgs {
   const double* X[8];
+  double coef[8];
 };
 
-__global__ void combine_kernel(int64_t n, int m, CombineArgs a, const double* coef, double* out) {
+__global__ void combine_kernel(int64_t n, int m, CombineArgs a, double* out) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    double v = coef[0] * a.X[0][i];
-    for (int k = 1; k < m; ++k) v += coef[k] * a.X[k][i];
+    double v = a.coef[0] * a.X[0][i];
+    for (int k = 1; k < m; ++k) v += a.coef[k] * a.X[k][i];
     out[i] = v;
   }
 }
@@ -1558,8 +1785,11 @@ int combine(stream_t s, int64_t n, int m, const double* const* X, const double* 
   if (m < 1 || m > 8) return (int)cudaErrorInvalidValue;
   if (n <= 0) return 0;
   CombineArgs a{};
-  for (int k = 0; k < m; ++k) a.X[k] = X[k];
-  combine_kernel<<<grid_for(n), 256, 0, (cudaStream_t)s>>>(n, m, a, coef, out);
+  for (int k = 0; k < m; ++k) {
+    a.X[k] = X[k];
+    a.coef[k] = coef[k];
+  }
+  combine_kernel<<<grid_for(n), 256, 0, (cudaStream_t)s>>>(n, m, a, out);
   return launched();
 }
 

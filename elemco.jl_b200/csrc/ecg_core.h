@@ -50,11 +50,15 @@ struct Ctx {
   double* klcd = nullptr;  // [k,l,c,d] = <kl|cd>
   double* Kvvoo = nullptr; // [a,b,i,j] = <ij|ab>
   double* fvo_t = nullptr; // [a,i] = f[i,a]
+  // (kc|ld) as the ring terms' matrices, [c,k,d,l] and [c,l,d,k]
+  double *V1 = nullptr, *V2 = nullptr;
   std::vector<double> h_host, fock_host;
 
   // dressed quantities
   double *dBvv = nullptr, *dBvo = nullptr, *dBoo = nullptr, *dBvvT = nullptr;
   double *dh = nullptr, *dfock = nullptr, *J = nullptr;
+  // dense blocks of dfock: [i,j], [a,i], f[i,a] as [a,i], [a,b]
+  double *dfoo = nullptr, *dfvo = nullptr, *dfov = nullptr, *dfvv = nullptr;
 
   // amplitudes: T = [T1 (nv*no) | T2 (nv^2 no^2)], same for R
   double *T = nullptr, *R = nullptr;
@@ -66,7 +70,6 @@ struct Ctx {
   double* dscal = nullptr;
   double* red = nullptr;
   double* hscal = nullptr;
-  double* dcoef = nullptr;
 
   Arena ws;
   double* ws_base = nullptr;
@@ -117,8 +120,9 @@ struct IterResult {
 void cc_init_iterations(Ctx& c, const ecg_cc_opts& o);
 IterResult cc_iteration(Ctx& c, bool dc);
 void diis_reset(Ctx& c, DiisState& d, int maxdiis, double resthr, int64_t len, bool cs);
-// DIIS perform on device vectors (src/solvers/diis.jl:246-305)
-void diis_perform(Ctx& c, DiisState& d, double* amps, const double* res);
+// DIIS perform on device vectors (src/solvers/diis.jl:246-305); saved: amps and
+// res are already in the slots d.amp[d.next], d.res[d.next]
+void diis_perform(Ctx& c, DiisState& d, double* amps, const double* res, bool saved = false);
 double scal(Ctx& c, int i);
 void sync_scalars(Ctx& c, int count);
 

@@ -232,15 +232,49 @@ int update_doubles(stream_t s, int nv, int no, const double* eo, const double* e
 int update_singles(stream_t s, int nv, int no, const double* eo, const double* ev,
                    double shift, const double* R, double* T);
 
-// Deterministic reductions into out[slot...] (device scalars):
-//   dot:      out[0] = sum x*y over n
-//   cs_dot:   for nv x nv x no x no:  out[0] = sum X[a,b,i,j] Y[a,b,i,j],
-//             out[1] = sum X[b,a,i,j] Y[a,b,i,j]
-// `scratch` must hold at least reduce_scratch_len() doubles.
+// Deterministic reductions (fixed grouping and order), all jobs in one launch:
+//   DOT_PLAIN  out[0] = sum X*Y over n
+//   DOT_CS     for nv x nv x no x no:  out[0] = sum X[a,b,i,j] Y[a,b,i,j],
+//              out[1] = sum X[b,a,i,j] Y[a,b,i,j]
+//   DOT_CS_T1  DOT_CS of X[a,b,i,j] = X[a,i] X[b,j] (X nv x no)
+// `scratch` must hold at least reduce_scratch_len() doubles, zero before its
+// first use; calls that share it run on one stream.
+enum { DOT_PLAIN = 0, DOT_CS = 1, DOT_CS_T1 = 2 };
+constexpr int DOT_MAX = 16;
+struct DotJob {
+  int type;
+  const double* X;
+  const double* Y;
+  int64_t n;  // DOT_PLAIN
+  double* out;
+};
 int64_t reduce_scratch_len();
+int dots(stream_t s, int nv, int no, int njobs, const DotJob* jobs, double* scratch);
 int dot(stream_t s, int64_t n, const double* x, const double* y, double* scratch, double* out);
 int cs_dot(stream_t s, int nv, int no, const double* X, const double* Y, double* scratch,
            double* out);
+
+// Doubles amplitudes as the ring terms read them, in one pass over T2[a,b,i,j]:
+//   X1[a,i,b,j] = T2[a,b,i,j], X2[a,i,b,j] = T2[a,b,j,i], Xt = 2 X1 - X2,
+//   Tt[a,b,i,j] = 2 T2[a,b,i,j] - T2[a,b,j,i]
+int ring_split(stream_t s, int nv, int no, const double* T2, double* X1, double* X2, double* Xt,
+               double* Tt);
+// In place over n elements: W, Y, Z <- Y - W, 2 W - Y - Z, Q/2 - Z (Y and Q read
+// as zero, and Q not at all, when Q is null).
+int ring_combine(stream_t s, int64_t n, double* W, double* Y, double* Z, const double* Q);
+// R2[a,b,i,j] += D[a,i,b,j] + D[b,j,a,i] + E[b,i,a,j] + E[a,j,b,i]
+int ring_add(stream_t s, int nv, int no, const double* D, const double* E, double* R2);
+// Fock matrix blocks: f = dh + 2 sum_Q B[:,:,Q] J[Q] + G, written to f (n x n) and
+// as dense blocks foo [i,j], fvo [a,i], fov [a,i] (of f[i,a]) and fvv [a,b].  G
+// holds the dense blocks oo, vo [a,i], ov [i,a], vv back to back.
+int fock_blocks(stream_t s, int no, int nv, int nq, const double* dh, const double* Boo,
+                const double* Bvo, const double* Bov, const double* Bvv, const double* J,
+                const double* G, double* f, double* foo, double* fvo, double* fov, double* fvv);
+// Level-shifted update of T = [T1 | T2] by R = [R1 | R2], in place, with copies
+// of both at Tsave and Rsave:
+//   T1 -= R1 / (ev[a] - eo[i] + shifts), T2 -= R2 / (ev[a] + ev[b] - eo[i] - eo[j] + shiftp)
+int update_save(stream_t s, int nv, int no, const double* eo, const double* ev, double shifts,
+                double shiftp, const double* R, double* T, double* Tsave, double* Rsave);
 
 // C(i,j) = alpha * A(i,j) + beta * C(i,j) for an m x n column-major block
 // (leading dimensions lda, ldc); beta == 0 never reads C.
@@ -252,7 +286,7 @@ int geam(stream_t s, int64_t m, int64_t n, double alpha, const double* A, int64_
 int outer(stream_t s, int64_t na, int64_t ni, int64_t nb, int64_t nj, double alpha,
           const double* X, const double* Y, double beta, double* out);
 
-// out = sum_{k<m} coef[k] * X[k]   (coef on the device)
+// out = sum_{k<m} coef[k] * X[k]
 int combine(stream_t s, int64_t n, int m, const double* const* X, const double* coef,
             double* out);
 
