@@ -97,6 +97,7 @@ int stream_create(stream_t* s) {
   cudaStream_t st;
   int e = (int)cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
   *s = (stream_t)st;
+  if (!e && !wait_error()) e = (int)cudaErrorMemoryAllocation;  // before any capture
   return e;
 }
 
@@ -144,6 +145,37 @@ uint64_t tc_wait(stream_t s) {
   return stream_state_locked((cudaStream_t)s).tc_wait_ns;
 }
 int sync(stream_t s) { return (int)cudaStreamSynchronize((cudaStream_t)s); }
+
+// The kernels write the code straight into host memory, so that reading it after
+// a synchronisation costs a load: copying one device variable per kernel back
+// took four synchronous copies, 30 to 40 us each time, four times an iteration.
+int* wait_error() {
+  static std::atomic<int*> word{nullptr};
+  int* p = word.load(std::memory_order_acquire);
+  if (p) return p;
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lk(mu);
+  p = word.load(std::memory_order_relaxed);
+  if (!p) {
+    if (cudaHostAlloc((void**)&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    *p = 0;
+    word.store(p, std::memory_order_release);
+  }
+  return p;
+}
+
+int tc_error(int* code) {
+  int* p = wait_error();
+  if (!p) return (int)cudaErrorMemoryAllocation;
+  *code = *(volatile int*)p;
+  if (*code) *(volatile int*)p = 0;
+  return 0;
+}
+
 const char* error_string(int code) { return cudaGetErrorString((cudaError_t)code); }
 int check_launch() { return (int)cudaGetLastError(); }
 
@@ -705,6 +737,12 @@ namespace {
 std::mutex g_tune_mu;
 std::map<std::string, int> g_tune;
 std::atomic<bool> g_tuning{false};
+// whether the table has entries of FP64 GEMMs ("dgemmt ..."): without them a
+// launch need not spell out its key
+std::atomic<bool> g_tune_fp64{false};
+void note_key(const std::string& key) {
+  if (key.compare(0, 7, "dgemmt ") == 0) g_tune_fp64.store(true);
+}
 }  // namespace
 
 void set_tuning(bool on) { g_tuning.store(on); }
@@ -722,6 +760,7 @@ bool tune_get(const std::string& key, int* value) {
 void tune_put(const std::string& key, int value) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
   g_tune[key] = value;
+  note_key(key);
 }
 
 size_t tune_size() {
@@ -753,7 +792,10 @@ int tune_parse(const std::string& text) {
     add[line.substr(0, sp)] = (int)v;
   }
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  for (auto& kv : add) g_tune[kv.first] = kv.second;
+  for (auto& kv : add) {
+    g_tune[kv.first] = kv.second;
+    note_key(kv.first);
+  }
   return (int)add.size();
 }
 
@@ -1003,6 +1045,7 @@ static int plain_gemm(stream_t s, const GemmArgs& g0, const Gemm& q0) {
     q = q0;
   }
   PlainChoice c = default_plain(q);
+  if (!g_tune_fp64.load(std::memory_order_relaxed) && !tuning()) return launch_plain(s, g, q, c);
   const std::string key = "dgemmt " + std::to_string(q.m) + " " + std::to_string(q.n) + " " +
                           std::to_string(q.k) + " " + std::to_string(q.batch) + " " +
                           std::to_string(g.a_kfast) + std::to_string(g.b_nfast);

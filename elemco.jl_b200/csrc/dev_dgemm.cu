@@ -26,7 +26,7 @@
 //            (g&1) + 8((g>>1)&1) + 2(g>>2) + 4s
 //
 // Every mbarrier wait is bounded (the stream's tensor-core bound, default
-// 1 s): on time-out the kernel records an error code (read by dtma_error),
+// 1 s): on time-out the kernel records an error code (read by tc_error),
 // waits (bounded) for its own copies in flight and returns without writing C.
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -47,8 +47,6 @@ namespace {
 
 using namespace tma;
 using namespace dfrag;
-
-__device__ int g_dtma_error = 0;
 
 template <int BM, int BN, int WM, int WN, int STAGES>
 struct DCfg {
@@ -76,7 +74,7 @@ template <int BM, int BN, int WM, int WN, int STAGES, int MINB, bool AKF, bool B
 __global__ void __launch_bounds__(DCfg<BM, BN, WM, WN, STAGES>::THREADS, MINB)
     dgemm_tma_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ CUtensorMap mb,
                      DOut out, int64_t k, int64_t kslice, int split,
-                     unsigned long long wait_ns) {
+                     unsigned long long wait_ns, int* err) {
   using Cfg = DCfg<BM, BN, WM, WN, STAGES>;
   constexpr int MT = WM / 8, NTL = WN / 8;
   extern __shared__ uint8_t smem_raw[];
@@ -135,7 +133,7 @@ __global__ void __launch_bounds__(DCfg<BM, BN, WM, WN, STAGES>::THREADS, MINB)
       for (; t < KT; ++t) {
         if (t >= STAGES &&
             !mbar_wait(&empty[t % STAGES], (uint32_t)((t / STAGES - 1) & 1), wait_ns)) {
-          atomicExch(&g_dtma_error, 1);
+          *(volatile int*)err = 17;
           break;
         }
         issue(t);
@@ -162,7 +160,7 @@ __global__ void __launch_bounds__(DCfg<BM, BN, WM, WN, STAGES>::THREADS, MINB)
     const int s = t % STAGES;
     const bool ready = mbar_wait(&full[s], (uint32_t)((t / STAGES) & 1), wait_ns);
     if (!__all_sync(~0u, ready)) {
-      if (lane == 0) atomicExch(&g_dtma_error, 1);
+      if (lane == 0) *(volatile int*)err = 17;
       return;
     }
     // Release the stage of tile t-1 only now, past the wait on tile t: the
@@ -210,28 +208,43 @@ __global__ void __launch_bounds__(DCfg<BM, BN, WM, WN, STAGES>::THREADS, MINB)
   }
 }
 
-// The map of operand X(i, k) = X[i*si + k*sk + z*sz] (i < ni, k < nk, z <
-// nz): k-fast when sk == 1 (box 16 k x rows), else i-fast (si == 1; box
-// 16 i x 16 k).  Returns false when TMA cannot address it.
-bool operand_map(CUtensorMap* m, bool* kfast, const double* X, int64_t ni, int64_t nk,
-                 int64_t si, int64_t sk, int64_t nz, int64_t sz, int rows) {
-  if (((uintptr_t)X & 15) != 0) return false;
-  if (nz > 1 && !stride_ok(sz)) return false;
-  // a single item's map still needs a valid third stride: the item's extent
-  auto zs = [&](int64_t s1, int64_t d1) { return nz > 1 ? sz : (s1 * d1 + 1) / 2 * 2; };
+// Operand X(i, k) = X[i*si + k*sk + z*sz] (i < ni, k < nk, z < nz) as TMA would
+// address it: k-fast when sk == 1 (rows of k, s1 apart), else i-fast (si == 1).
+// ok is false when it cannot.  A single item's map still needs a valid third
+// stride: the item's extent.
+struct DOperand {
+  bool ok = false, kfast = false;
+  int64_t s1 = 0, sz = 0;
+};
+DOperand operand(const double* X, int64_t ni, int64_t nk, int64_t si, int64_t sk, int64_t nz,
+                 int64_t sz) {
+  DOperand d;
+  if (((uintptr_t)X & 15) != 0 || (nz > 1 && !stride_ok(sz))) return d;
+  int64_t rows;
   if (sk == 1 && (nk > 1 || si != 1)) {
-    const int64_t s1 = ni > 1 ? si : (nk + 1) / 2 * 2;
-    if (!stride_ok(s1)) return false;
-    *kfast = true;
-    return dmap(m, X, nk, ni, s1, nz, zs(s1, ni), rows) == 0;
+    d.kfast = true;
+    rows = ni;
+    d.s1 = ni > 1 ? si : (nk + 1) / 2 * 2;
+  } else if (si == 1) {
+    rows = nk;
+    d.s1 = nk > 1 ? sk : (ni + 1) / 2 * 2;
+  } else {
+    return d;
   }
-  if (si == 1) {
-    const int64_t s1 = nk > 1 ? sk : (ni + 1) / 2 * 2;
-    if (!stride_ok(s1)) return false;
-    *kfast = false;
-    return dmap(m, X, ni, nk, s1, nz, zs(s1, nk), 16) == 0;
-  }
-  return false;
+  d.sz = nz > 1 ? sz : (d.s1 * rows + 1) / 2 * 2;
+  d.ok = stride_ok(d.s1) && stride_ok(d.sz);
+  return d;
+}
+
+// Its map (box 16 k x box_rows rows, or 16 i x 16 k); false when TMA cannot
+// address it.
+bool operand_map(CUtensorMap* m, bool* kfast, const double* X, int64_t ni, int64_t nk,
+                 int64_t si, int64_t sk, int64_t nz, int64_t sz, int box_rows) {
+  const DOperand d = operand(X, ni, nk, si, sk, nz, sz);
+  if (!d.ok) return false;
+  *kfast = d.kfast;
+  return d.kfast ? dmap(m, X, nk, ni, d.s1, nz, d.sz, box_rows) == 0
+                 : dmap(m, X, ni, nk, d.s1, nz, d.sz, 16) == 0;
 }
 
 template <int BM, int BN, int WM, int WN, int STAGES, int MINB, bool AKF, bool BKF>
@@ -258,8 +271,10 @@ int launch_dtma(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap& mb, c
   if (gy > 65535 || nz > 65535) return (int)cudaErrorInvalidConfiguration;
   dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)nz);
   unsigned long long w = tc_wait((stream_t)st);
-  kern<<<grid, Cfg::THREADS, Cfg::SMEM, st>>>(ma, mb, out, k, kslice, split,
-                                              w ? w : WAIT_NS);
+  int* err = wait_error();
+  if (!err) return (int)cudaErrorMemoryAllocation;
+  kern<<<grid, Cfg::THREADS, Cfg::SMEM, st>>>(ma, mb, out, k, kslice, split, w ? w : WAIT_NS,
+                                              err);
   note_launches(1);
   return (int)cudaGetLastError();
 }
@@ -309,10 +324,8 @@ bool dgemm_tma_usable(const Gemm& q) {
   if (q.scm != 1 || q.m <= 0 || q.n <= 0 || q.k <= 0) return false;
   if (q.m >= ((int64_t)1 << 31) || q.n >= ((int64_t)1 << 31) || q.k >= ((int64_t)1 << 31))
     return false;
-  CUtensorMap m;
-  bool kf;
-  return operand_map(&m, &kf, q.A, q.m, q.k, q.sam, q.sak, q.batch, q.sab, 64) &&
-         operand_map(&m, &kf, q.B, q.n, q.k, q.sbn, q.sbk, q.batch, q.sbb, 64);
+  return operand(q.A, q.m, q.k, q.sam, q.sak, q.batch, q.sab).ok &&
+         operand(q.B, q.n, q.k, q.sbn, q.sbk, q.batch, q.sbb).ok;
 }
 
 // Estimated time (us) of configuration cfg with K in S slices: the busiest
@@ -374,18 +387,6 @@ int dgemm_tma(stream_t s, const Gemm& q, int cfg, int nsplit) {
   DOut o{P, q.m, q.n, q.m, q.m * q.n, 1.0, 0.0};
   if (int e = f(st, ma, mb, o, q.k, kc, (int)S, 1)) return e;
   return splitk_reduce(s, q.m, q.n, (int)S, P, q.alpha, q.beta, q.C, q.scm, q.scn);
-}
-
-int dtma_error(int* code) {
-  int h = 0;
-  cudaError_t e = cudaMemcpyFromSymbol(&h, g_dtma_error, sizeof(int));
-  if (e != cudaSuccess) return (int)e;
-  *code = h;
-  if (h) {
-    int zero = 0;
-    cudaMemcpyToSymbol(g_dtma_error, &zero, sizeof(int));
-  }
-  return 0;
 }
 
 }  // namespace dev

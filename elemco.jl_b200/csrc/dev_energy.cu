@@ -33,7 +33,7 @@
 // sums are reduced in a fixed order.
 //
 // Every mbarrier wait is bounded (the stream's tensor-core bound, default
-// 1 s); on time-out the warp records an error code (read by energy_error),
+// 1 s); on time-out the warp records an error code (read by tc_error),
 // waits (bounded) for its own copies and stops.
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -54,8 +54,6 @@ namespace {
 using namespace tma;
 
 constexpr int EC_CUBE = 512;  // floats per staged cube, [z][y][x]
-
-__device__ int g_energy_error = 0;
 
 template <bool HAS_U>
 struct EnergyWarpSmem {
@@ -110,7 +108,7 @@ __global__ void __launch_bounds__(EnergyWarpSmem<HAS_U>::THREADS, 1)
                               const double* __restrict__ eijk_tab, const double* __restrict__ ev,
                               const TriplesTermsF* __restrict__ tt_tab,
                               const int* __restrict__ tri, int ntri, double* part,
-                              unsigned long long wait_ns) {
+                              unsigned long long wait_ns, int* err) {
   using L = EnergyWarpSmem<HAS_U>;
   extern __shared__ unsigned char esm_raw[];
   __shared__ double red[2][L::WARPS];
@@ -184,7 +182,7 @@ __global__ void __launch_bounds__(EnergyWarpSmem<HAS_U>::THREADS, 1)
     asm volatile("cp.async.wait_group 0;\n" ::);
     const bool landed = mbar_wait(bar, phase, wait_ns);
     if (!__all_sync(~0u, landed)) {
-      if (lane == 0) atomicExch(&g_energy_error, 1);
+      if (lane == 0) *(volatile int*)err = 33;
       mbar_wait(bar, phase, WAIT_NS);  // nothing of this warp's may stay in flight
       break;
     }
@@ -354,8 +352,10 @@ int launch_energy(cudaStream_t st, dim3 grid, const CUtensorMap* maps, int nv,
     if (d >= 0 && d < 128) done[d].store(true, std::memory_order_release);
   }
   const unsigned long long w = tc_wait((stream_t)st);
+  int* err = wait_error();
+  if (!err) return (int)cudaErrorMemoryAllocation;
   kern<<<grid, L::THREADS, L::SMEM, st>>>(maps[0], maps[1], maps[2], maps[3], nv, eijk_tab, ev,
-                                          tt_tab, tri, ntri, scratch, w ? w : WAIT_NS);
+                                          tt_tab, tri, ntri, scratch, w ? w : WAIT_NS, err);
   note_launches(1);
   return (int)cudaGetLastError();
 }
@@ -436,18 +436,6 @@ int triples_energy_f32_batched(stream_t s, int nv, int vp, int nitems, int nslot
   energy_final_kernel<<<2 * nitems, 32, 0, st>>>(g, scratch, out);
   note_launches(1);
   return (int)cudaGetLastError();
-}
-
-int energy_error(int* code) {
-  int h = 0;
-  cudaError_t e = cudaMemcpyFromSymbol(&h, g_energy_error, sizeof(int));
-  if (e != cudaSuccess) return (int)e;
-  *code = h;
-  if (h) {
-    int zero = 0;
-    cudaMemcpyToSymbol(g_energy_error, &zero, sizeof(int));
-  }
-  return 0;
 }
 
 }  // namespace dev

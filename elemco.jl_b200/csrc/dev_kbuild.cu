@@ -37,8 +37,6 @@ namespace {
 using namespace tma;
 using namespace dfrag;
 
-__device__ int g_kbuild_error = 0;
-
 constexpr int KB_BM = 64, KB_WARPS = 4, KB_THREADS = 32 * KB_WARPS;
 
 template <int BN, int STAGES>
@@ -69,7 +67,7 @@ struct KbOut {
 template <int BN, int STAGES, int MINB>
 __global__ void __launch_bounds__(KB_THREADS, MINB)
     kbuild_kernel(const __grid_constant__ KbMaps maps, const KbOut out, const KbSegs segs,
-                  const KbItem* __restrict__ items, int ntn, unsigned long long wait_ns) {
+                  const KbItem* __restrict__ items, int ntn, unsigned long long wait_ns, int* err) {
   using Cfg = KbCfg<BN, STAGES>;
   constexpr int MT = 2, NTL = BN / 8;
   extern __shared__ uint8_t smem_raw[];
@@ -174,7 +172,7 @@ __global__ void __launch_bounds__(KB_THREADS, MINB)
     }
   }
   if (!ok) {
-    if (lane == 0) atomicExch(&g_kbuild_error, 1);
+    if (lane == 0) *(volatile int*)err = 49;
     // nothing of this CTA's may be in flight when it exits
     if (tid == 0)
       for (int t = consumed; t < issued; ++t)
@@ -233,7 +231,7 @@ __global__ void __launch_bounds__(KB_THREADS, MINB)
 
 template <int BN, int STAGES, int MINB>
 int launch_kbuild(cudaStream_t st, const KbMaps& maps, const KbOut& out, const KbSegs& segs,
-                  const KbItem* items, int nitems, unsigned long long wait_ns) {
+                  const KbItem* items, int nitems, unsigned long long wait_ns, int* err) {
   using Cfg = KbCfg<BN, STAGES>;
   auto kern = kbuild_kernel<BN, STAGES, MINB>;
   // cudaFuncSetAttribute acts on the current device only: one flag per device
@@ -252,7 +250,7 @@ int launch_kbuild(cudaStream_t st, const KbMaps& maps, const KbOut& out, const K
   const int64_t mt = (out.m + KB_BM - 1) / KB_BM, nt = (out.n + BN - 1) / BN;
   if (mt * nt >= ((int64_t)1 << 31)) return (int)cudaErrorInvalidConfiguration;
   kern<<<dim3((unsigned)(mt * nt), (unsigned)nitems), KB_THREADS, Cfg::SMEM, st>>>(
-      maps, out, segs, items, (int)nt, wait_ns);
+      maps, out, segs, items, (int)nt, wait_ns, err);
   note_launches(1);
   return (int)cudaGetLastError();
 }
@@ -309,30 +307,20 @@ int kbuild(stream_t s, const KbGemm& g, int nitems, const KbItem* items) {
   cudaStream_t st = (cudaStream_t)s;
   const uint64_t w = tc_wait(s);
   const unsigned long long wns = w ? (unsigned long long)w : WAIT_NS;
+  int* err = wait_error();
+  if (!err) return (int)cudaErrorMemoryAllocation;
   const int slot = ktime_begin(s, KT_DGEMM);
   int e;
   switch (kb_width(g.n)) {
-    case 112: e = launch_kbuild<112, 4, 2>(st, maps, out, segs, items, nitems, wns); break;
-    case 96: e = launch_kbuild<96, 4, 2>(st, maps, out, segs, items, nitems, wns); break;
-    case 80: e = launch_kbuild<80, 4, 3>(st, maps, out, segs, items, nitems, wns); break;
-    case 64: e = launch_kbuild<64, 4, 3>(st, maps, out, segs, items, nitems, wns); break;
-    case 48: e = launch_kbuild<48, 4, 3>(st, maps, out, segs, items, nitems, wns); break;
-    default: e = launch_kbuild<32, 4, 3>(st, maps, out, segs, items, nitems, wns); break;
+    case 112: e = launch_kbuild<112, 4, 2>(st, maps, out, segs, items, nitems, wns, err); break;
+    case 96: e = launch_kbuild<96, 4, 2>(st, maps, out, segs, items, nitems, wns, err); break;
+    case 80: e = launch_kbuild<80, 4, 3>(st, maps, out, segs, items, nitems, wns, err); break;
+    case 64: e = launch_kbuild<64, 4, 3>(st, maps, out, segs, items, nitems, wns, err); break;
+    case 48: e = launch_kbuild<48, 4, 3>(st, maps, out, segs, items, nitems, wns, err); break;
+    default: e = launch_kbuild<32, 4, 3>(st, maps, out, segs, items, nitems, wns, err); break;
   }
   ktime_end(s, KT_DGEMM, slot, 2.0 * (double)g.m * (double)g.n * depth * nitems);
   return e;
-}
-
-int kbuild_error(int* code) {
-  int h = 0;
-  cudaError_t e = cudaMemcpyFromSymbol(&h, g_kbuild_error, sizeof(int));
-  if (e != cudaSuccess) return (int)e;
-  *code = h;
-  if (h) {
-    int zero = 0;
-    cudaMemcpyToSymbol(g_kbuild_error, &zero, sizeof(int));
-  }
-  return 0;
 }
 
 }  // namespace dev

@@ -80,8 +80,6 @@ struct TcCfg {
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
   static_assert(TILE_BYTES_B % 1024 == 0, "128-byte-swizzle tiles start on 1024 bytes");
 };
-__device__ int g_tc_error = 0;
-
 // Persistent, warp-specialised kernel: gridDim.x CTAs (one per SM) loop over
 // work items (m-tile, n-tile, k-slice).  Warp 0 lane 0: TMA producer over a
 // STAGES-deep shared-memory ring (full/empty mbarriers).  Warp 1: owns the
@@ -178,7 +176,7 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
                       double alpha, double beta, const TcSegs segs, int kb_per_split,
                       int kblocks_total,
                       int64_t split_stride, int mtiles, int ntiles, int nsplit,
-                      unsigned long long wait_ns, int tri) {
+                      unsigned long long wait_ns, int tri, int* err) {
   using Cfg = TcCfg<NSL, TN>;
   constexpr int STAGES = Cfg::STAGES, STAGE_BYTES = Cfg::STAGE_BYTES;
   constexpr int TILE_BYTES_B = Cfg::TILE_BYTES_B;
@@ -250,7 +248,7 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
           const int s = (int)(g % STAGES);
           const int64_t u = g / STAGES;
           if (u > 0 && !mbar_wait(&empty[s], (uint32_t)((u - 1) & 1), wait_ns)) {
-            atomicExch(&g_tc_error, 1);
+            *(volatile int*)err = 1;
             atomicExch(abort_flag, 1);
             break;
           }
@@ -288,7 +286,7 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
         const int acc = (int)(lt & 1);
         const int64_t ua = lt >> 1;
         if (ua > 0 && !mbar_wait(&tempty[acc], (uint32_t)((ua - 1) & 1), wait_ns)) {
-          atomicExch(&g_tc_error, 4);
+          *(volatile int*)err = 4;
           atomicExch(abort_flag, 1);
           break;
         }
@@ -298,7 +296,7 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
         for (int kb = 0; kb < nk; ++kb, ++g) {
           const int s = (int)(g % STAGES);
           if (!mbar_wait(&full[s], (uint32_t)((g / STAGES) & 1), wait_ns)) {
-            atomicExch(&g_tc_error, 2);
+            *(volatile int*)err = 2;
             atomicExch(abort_flag, 1);
             ok = false;
             break;
@@ -350,7 +348,7 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
       const bool ready = mbar_wait(&tfull[acc], (uint32_t)((lt >> 1) & 1), wait_ns);
       if (!__all_sync(0xffffffffu, ready)) {
         if (lane == 0) {
-          atomicExch(&g_tc_error, 3);
+          *(volatile int*)err = 3;
           atomicExch(abort_flag, 1);
         }
         break;
@@ -626,13 +624,15 @@ int launch_tc(cudaStream_t st, const TcMaps& maps, const TcSegs& segs, int kbt, 
   const int64_t items = (int64_t)mt * nt * S;
   const unsigned grid = (unsigned)(items < 148 ? items : 148);
   const unsigned long long wns = wait_bound(st);
+  int* err = wait_error();
+  if (!err) return (int)cudaErrorMemoryAllocation;
   // useful BF16 products: 2 m n K per slice pair (zero padding not counted)
   const double work = 2.0 * (double)m * (double)n * (double)seg_depth(segs) * Cfg::NPAIR *
                       gemm_kept(m, n, tri);
   const int slot = ktime_begin((stream_t)st, KT_TCGEMM);
   if (S == 1) {
     mgemm_bf16_kernel<NSL, TN><<<grid, THREADS_TC, Cfg::SMEM_BYTES, st>>>(
-        maps, out, m, n, alpha, beta, segs, kps, kbt, 0, mt, nt, 1, wns, tri);
+        maps, out, m, n, alpha, beta, segs, kps, kbt, 0, mt, nt, 1, wns, tri, err);
     note_launches(1);
     ktime_end((stream_t)st, KT_TCGEMM, slot, work);
     return (int)cudaGetLastError();
@@ -644,7 +644,7 @@ int launch_tc(cudaStream_t st, const TcMaps& maps, const TcSegs& segs, int kbt, 
   if (!P) return (int)cudaErrorMemoryAllocation;
   TcOut po{P, 1, m, 1};
   mgemm_bf16_kernel<NSL, TN><<<grid, THREADS_TC, Cfg::SMEM_BYTES, st>>>(
-      maps, po, m, n, 1.0, 0.0, segs, kps, kbt, m * n, mt, nt, S, wns, 0);
+      maps, po, m, n, 1.0, 0.0, segs, kps, kbt, m * n, mt, nt, S, wns, 0, err);
   note_launches(1);
   int e = (int)cudaGetLastError();
   if (e) return e;
@@ -1085,23 +1085,6 @@ int gemm_mixed(stream_t s, char ta, char tb, int64_t m, int64_t n, int64_t k, do
   q.sbk = bt ? ldb : 1; q.sbn = bt ? 1 : ldb;
   q.scm = 1; q.scn = ldc;
   return gemm_strided_mixed(s, q);
-}
-
-int tc_error(int* code) {
-  int h = 0;
-  cudaError_t e = cudaMemcpyFromSymbol(&h, g_tc_error, sizeof(int));
-  if (e != cudaSuccess) return (int)e;
-  if (h) {
-    int zero = 0;
-    cudaMemcpyToSymbol(g_tc_error, &zero, sizeof(int));
-  }
-  int d = 0, en = 0, kb = 0, tk = 0;
-  if (int r = dtma_error(&d)) return r;
-  if (int r = energy_error(&en)) return r;
-  if (int r = kbuild_error(&kb)) return r;
-  if (int r = tckbuild_error(&tk)) return r;
-  *code = h ? h : d ? 16 + d : en ? 32 + en : kb ? 48 + kb : (tk ? 64 + tk : 0);
-  return 0;
 }
 
 }  // namespace dev

@@ -62,8 +62,6 @@ constexpr int EPI_WARPS = 8;  // two per lane quarter, alternate 16-column chunk
 constexpr int KT_THREADS = 32 * (2 + EPI_WARPS);
 constexpr uint32_t TMEM_COLS = 512, ACC_STRIDE = 256;
 
-__device__ int g_tckb_error = 0;
-
 struct KtMaps {
   CUtensorMap a[KB_MAX_SEG], b[KB_MAX_SEG];
 };
@@ -113,7 +111,7 @@ __device__ __forceinline__ SegPos seg_at(const KtSegs& g, int kb) {
 __global__ void __launch_bounds__(KT_THREADS, 1)
     tc_kbuild_kernel(const __grid_constant__ KtMaps maps, const KtOut out, const KtSegs segs,
                      const KtTiles tiles, const KbItem* __restrict__ items,
-                     unsigned long long wait_ns) {
+                     unsigned long long wait_ns, int* err) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int tn = tiles.tn, b_bytes = tn * TK * 2, stage_bytes = NSL * (A_BYTES + b_bytes);
@@ -164,7 +162,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1)
         for (int kb = 0; kb < nk; ++kb) {
           const SegPos sp = seg_at(segs, kb);
           if (issued >= stages && !mbar_wait(&empty[s], ph ^ 1u, wait_ns)) {
-            atomicExch(&g_tckb_error, 1);
+            *(volatile int*)err = 65;
             atomicExch(abort_flag, 1);
             break;
           }
@@ -212,7 +210,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1)
            it += gridDim.x, ++lt) {
         const int acc = lt & 1, ua = lt >> 1;
         if (ua > 0 && !mbar_wait(&tempty[acc], (uint32_t)((ua - 1) & 1), wait_ns)) {
-          atomicExch(&g_tckb_error, 4);
+          *(volatile int*)err = 68;
           atomicExch(abort_flag, 1);
           break;
         }
@@ -221,7 +219,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1)
         bool ok = true;
         for (int kb = 0; kb < nk; ++kb) {
           if (!mbar_wait(&full[s], ph, wait_ns)) {
-            atomicExch(&g_tckb_error, 2);
+            *(volatile int*)err = 66;
             atomicExch(abort_flag, 1);
             ok = false;
             break;
@@ -301,7 +299,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1)
           lane != 0 || mbar_wait(&tfull[acc], (uint32_t)((lt >> 1) & 1), wait_ns);
       if (!__all_sync(0xffffffffu, ready)) {
         if (lane == 0) {
-          atomicExch(&g_tckb_error, 3);
+          *(volatile int*)err = 67;
           atomicExch(abort_flag, 1);
         }
         break;
@@ -422,24 +420,14 @@ int tc_kbuild(stream_t s, const TcKbuild& g, int nitems, const KbItem* items, in
   }
   cudaStream_t st = (cudaStream_t)s;
   const uint64_t w = tc_wait(s);
+  int* err = wait_error();
+  if (!err) return (int)cudaErrorMemoryAllocation;
   const int slot = ktime_begin(s, KT_TCGEMM);
   tc_kbuild_kernel<<<(unsigned)std::min<int64_t>(total, 148), KT_THREADS, KT_SMEM, st>>>(
-      maps, out, segs, tiles, items, w ? (unsigned long long)w : WAIT_NS);
+      maps, out, segs, tiles, items, w ? (unsigned long long)w : WAIT_NS, err);
   note_launches(1);
   ktime_end(s, KT_TCGEMM, slot, 2.0 * (double)g.m * (double)g.n * depth * NPAIR * nitems);
   return (int)cudaGetLastError();
-}
-
-int tckbuild_error(int* code) {
-  int h = 0;
-  cudaError_t e = cudaMemcpyFromSymbol(&h, g_tckb_error, sizeof(int));
-  if (e != cudaSuccess) return (int)e;
-  *code = h;
-  if (h) {
-    int zero = 0;
-    cudaMemcpyToSymbol(g_tckb_error, &zero, sizeof(int));
-  }
-  return 0;
 }
 
 }  // namespace dev

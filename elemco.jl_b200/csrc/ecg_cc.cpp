@@ -614,25 +614,28 @@ static double diis_dot_value(Ctx& c, const DiisState& d, int slot) {
 
 // perform! (diis.jl:246-305) on device vectors; the B matrix and the small
 // linear solve live on the host in FP64.  `amps` is replaced by the
-// extrapolated vector.
-void diis_perform(Ctx& c, DiisState& d, double* amps, const double* res, bool saved) {
+// extrapolated vector.  In three parts, so that the CC iteration can read these
+// dots with its norms and energies in one synchronisation:
+// diis_dots queues the dots of `res` with every slot (slot i's at scalars
+// [128 + 3i, 130 + 3i], `res` itself standing in for the slot it will take),
+// diis_solve, once they are on the host, gives the coefficients and the next
+// slot (none: no extrapolation).
+static int diis_dots(Ctx& c, DiisState& d, const double* res) {
   if (d.ndim < d.maxdiis) d.ndim += 1;
-  const int ithis = d.next, nd = d.ndim, M = d.maxdiis + 1;
-  if (!saved) {
-    check(dev::d2d(d.amp[ithis], amps, d.len * 8, c.st), "diis save amps");
-    check(dev::d2d(d.res[ithis], res, d.len * 8, c.st), "diis save res");
-  }
-  // dots of `res` with every slot, slot i's at scalars [128 + 3i, 130 + 3i]
   dev::DotJob jobs[2 * 8];
   int nj = 0;
-  for (int i = 0; i < nd; ++i) {
-    const double* other = i == ithis ? res : d.res[i];
+  for (int i = 0; i < d.ndim; ++i) {
+    const double* other = i == d.next ? res : d.res[i];
     double* out = c.dscal + 128 + 3 * i;
     jobs[nj++] = {dev::DOT_PLAIN, res, other, d.cs ? c.n1() : d.len, out};
     if (d.cs) jobs[nj++] = {dev::DOT_CS, res + c.n1(), other + c.n1(), 0, out + 1};
   }
   check(dev::dots(c.st, c.nv, c.no, nj, jobs, c.red), "diis dots");
-  sync_scalars(c, 128 + 3 * nd);
+  return 128 + 3 * d.ndim;  // scalars to read
+}
+
+static std::vector<double> diis_solve(Ctx& c, DiisState& d) {
+  const int ithis = d.next, nd = d.ndim, M = d.maxdiis + 1;
   for (int i = 0; i < nd; ++i) {
     double dv = diis_dot_value(c, d, i);
     d.bmat[i * M + ithis] = dv;
@@ -649,7 +652,7 @@ void diis_perform(Ctx& c, DiisState& d, double* amps, const double* res, bool sa
   sym_pinv_solve(nd + 1, B, rhs, x);
   if (nd == 1 && d.next == 0 && thisdot > d.resthr) {
     d.ndim = 0;
-    return;
+    return {};
   } else if (nd < d.maxdiis) {
     d.next = nd;
   } else {
@@ -660,8 +663,21 @@ void diis_perform(Ctx& c, DiisState& d, double* amps, const double* res, bool sa
         d.next = i;
       }
   }
-  std::vector<const double*> X(d.amp.begin(), d.amp.begin() + nd);
-  check(dev::combine(c.st, d.len, nd, X.data(), x.data(), amps), "diis combine");
+  x.resize(nd);
+  return x;
+}
+
+static void diis_combine(Ctx& c, DiisState& d, const std::vector<double>& x, double* amps) {
+  if (x.empty()) return;
+  std::vector<const double*> X(d.amp.begin(), d.amp.begin() + x.size());
+  check(dev::combine(c.st, d.len, (int)x.size(), X.data(), x.data(), amps), "diis combine");
+}
+
+void diis_perform(Ctx& c, DiisState& d, double* amps, const double* res) {
+  check(dev::d2d(d.amp[d.next], amps, d.len * 8, c.st), "diis save amps");
+  check(dev::d2d(d.res[d.next], res, d.len * 8, c.st), "diis save res");
+  sync_scalars(c, diis_dots(c, d, res));
+  diis_combine(c, d, diis_solve(c, d), amps);
 }
 
 // --------------------------------------------------------------- iteration
@@ -694,14 +710,23 @@ IterResult cc_iteration(Ctx& c, bool dc) {
   jobs[nj++] = {dev::DOT_CS, c.T2(), c.R2(), 0, c.dscal + 8};
   jobs[nj++] = {dev::DOT_PLAIN, c.R1(), c.T1(), c.n1(), c.dscal + 10};
   check(dev::dots(s, c.nv, c.no, nj, jobs, c.red), "norms, energies");
-  sync_scalars(c, 11);
+  // a wait that ran out leaves T and the DIIS history as they were
+  const int ndim = c.diis.ndim;
+  try {
+    sync_scalars(c, diis_dots(c, c.diis, c.R));
+  } catch (...) {
+    c.diis.ndim = ndim;
+    throw;
+  }
   double sc[11];
   std::memcpy(sc, c.hscal, sizeof sc);
-  // update (cctools.jl:284-300)
+  // update (cctools.jl:284-300) and extrapolation
+  const int slot = c.diis.next;
+  const std::vector<double> x = diis_solve(c, c.diis);
   check(dev::update_save(s, c.nv, c.no, c.eps, c.eps + c.no, c.opts.shifts, c.opts.shiftp, c.R,
-                         c.T, c.diis.amp[c.diis.next], c.diis.res[c.diis.next]),
+                         c.T, c.diis.amp[slot], c.diis.res[slot]),
         "update");
-  diis_perform(c, c.diis, c.T, c.R, true);
+  diis_combine(c, c.diis, x, c.T);
   nj = energy_dots(c, 20, jobs);
   check(dev::dots(s, c.nv, c.no, nj, jobs, c.red), "energies");
   sync_scalars(c, 25);

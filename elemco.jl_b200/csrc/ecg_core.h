@@ -120,9 +120,8 @@ struct IterResult {
 void cc_init_iterations(Ctx& c, const ecg_cc_opts& o);
 IterResult cc_iteration(Ctx& c, bool dc);
 void diis_reset(Ctx& c, DiisState& d, int maxdiis, double resthr, int64_t len, bool cs);
-// DIIS perform on device vectors (src/solvers/diis.jl:246-305); saved: amps and
-// res are already in the slots d.amp[d.next], d.res[d.next]
-void diis_perform(Ctx& c, DiisState& d, double* amps, const double* res, bool saved = false);
+// DIIS perform on device vectors (src/solvers/diis.jl:246-305)
+void diis_perform(Ctx& c, DiisState& d, double* amps, const double* res);
 double scal(Ctx& c, int i);
 void sync_scalars(Ctx& c, int count);
 

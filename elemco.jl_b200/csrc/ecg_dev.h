@@ -82,9 +82,6 @@ bool dgemm_tma_usable(const Gemm& q);
 // Returns that time (us).
 double dgemm_tma_rule(const Gemm& q, int* cfg, int* nsplit);
 int dgemm_tma(stream_t s, const Gemm& q, int cfg, int nsplit);
-// Time-out code of the TMA FP64 GEMM's bounded waits since the last call
-// (0 = none); reading clears it.
-int dtma_error(int* code);
 
 // The (T) K builds in FP64 (dev_kbuild.cu): for each item z of a batch
 //   C_z(r,c) = beta C_z(r,c) + sum_{s < nseg} sum_{k < k[s]} A_s(r,k) B_s(c,k)
@@ -113,8 +110,6 @@ struct KbGemm {
   bool even_items = false;
 };
 int kbuild(stream_t s, const KbGemm& g, int nitems, const KbItem* items);
-// Time-out code of its bounded waits (0 = none); reading clears it.
-int kbuild_error(int* code);
 // Split-BF16 tensor-core version of gemm_strided (batch 1).
 int gemm_strided_mixed(stream_t s, const Gemm& g);
 
@@ -205,8 +200,6 @@ struct TcKbuild {
   int64_t scm = 1, dm = 0, scm2 = 0, scn = 0;
 };
 int tc_kbuild(stream_t s, const TcKbuild& g, int nitems, const KbItem* items, int chunk);
-// Time-out code of its bounded waits (0 = none); reading clears it.
-int tckbuild_error(int* code);
 
 // out = alpha * permute(in) + beta * out.  in has rank nd with dims
 // in_dims (column-major, first fastest); out dimension d is in dimension
@@ -350,9 +343,6 @@ int triples_energy_f32_batched(stream_t s, int nv, int vp, int nitems, int nslot
                                int64_t npairs, const double* eijk_tab, const double* ev,
                                const TriplesTermsF* tt_tab, const int* tri, double* scratch,
                                double* out);
-// Time-out code of the FP32 energy kernel's bounded waits (0 = none); reading
-// clears it.
-int energy_error(int* code);
 
 // Split-K GEMM (column-major, device pointers) whose partial products use a
 // fixed file-scope device array instead of allocated memory; m*n must not
@@ -371,6 +361,9 @@ int gemm_mixed(stream_t s, char ta, char tb, int64_t m, int64_t n, int64_t k, do
                const double* A, int64_t lda, const double* B, int64_t ldb, double beta,
                double* C, int64_t ldc);
 int tc_error(int* code);
+// Where those kernels leave it: one word of pinned host memory that every
+// device maps (nullptr: it could not be allocated).
+int* wait_error();
 // Split-K scratch of stream s on the current device (at least n doubles;
 // grown on demand, after s has drained, never during stream capture: nullptr
 // then, or when the allocation fails) and its fixed-order reduction
