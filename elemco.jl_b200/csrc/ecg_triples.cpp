@@ -23,8 +23,8 @@
 //
 // Mixed precision: every operand is split into two BF16 slices once per call
 // (vvvo in both layouts, T^{xy} per pair, T2[:,:,x,:] and T2[:,:,:,x] per
-// occupied index, -ovoo per pair; each kind one stack), the GEMMs run on the tensor cores and K is
-// kept in FP32.
+// occupied index, -ovoo per pair; each kind one stack), the GEMMs run on the
+// tensor cores and K is kept in FP32.
 #include "ecg_triples.h"
 
 #include <algorithm>
@@ -77,11 +77,13 @@ KMap k_map(int q, int64_t v, int64_t vp) {
   return vp == v ? KMap{1, 0, 0, vp * v} : KMap{1, v, vp, vp * v};  // K[n0,n1,a']
 }
 
-// Consecutive triplets whose tensor-core tiles are interleaved (two that share
-// j and k read a row tile of their vvvo slabs together), and the block of (i, j)
-// the sweep takes triplets in: eight i of four j need 13 slabs of one k, which L2
-// can hold part of, where i running fastest over all needs one slab each.
-constexpr int kChunk = 2, kBlockI = 8, kBlockJ = 4;
+// Consecutive triplets whose tensor-core tiles are interleaved, and the block of
+// (i, j) the sweep takes them in: a chunk of 32 shares one k, about four j and
+// eight i, so it reads 13 vvvo slabs where triplet by triplet it read 64 (and
+// holds 15 MB of T^{xy} at v = 209, well inside L2).  Measured at v = 209, all
+// triplets of 31 orbitals: chunks of 2 800 ms, 32 749, 64 747; at v = 129 and 318
+// within the runs' spread of one another.
+constexpr int kChunk = 32, kBlockI = 8, kBlockJ = 4;
 
 // BF16 operands of one amplitude tensor (T2 or covariant U2), as stacks.
 struct SplitAmps {
