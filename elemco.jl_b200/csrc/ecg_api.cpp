@@ -239,7 +239,7 @@ int ecg_mp2(ecg_ctx* c, double* T1, double* T2, double* e_mp2) {
     check(dev::cs_dot(s, c->nv, c->no, c->T2(), c->Kvvoo, c->red, c->dscal), "mp2 e");
     check(dev::dot(s, c->n1(), c->fvo_t, c->T1(), c->red, c->dscal + 2), "mp2 e1");
     if (T1) check(dev::d2h(T1, c->T1(), c->n1() * 8, s), "d2h");
-    if (T2) check(dev::d2h(T2, c->T2(), c->n2() * 8, s), "d2h");
+    if (T2) check(dev::d2h_large(T2, c->T2(), c->n2() * 8, s), "d2h");
     sync_scalars(*c, 3);
     c->t_resident = true;
     if (e_mp2) *e_mp2 = 2.0 * c->hscal[0] - c->hscal[1] + 2.0 * c->hscal[2];
@@ -254,7 +254,7 @@ int ecg_cc_residual(ecg_ctx* c, int dc, const double* T1, const double* T2, doub
     load_T(*c, T1, T2);
     cc_residual(*c, dc != 0);
     if (R1) check(dev::d2h(R1, c->R1(), c->n1() * 8, c->st), "d2h R1");
-    if (R2) check(dev::d2h(R2, c->R2(), c->n2() * 8, c->st), "d2h R2");
+    if (R2) check(dev::d2h_large(R2, c->R2(), c->n2() * 8, c->st), "d2h R2");
     check(dev::sync(c->st), "sync");
   });
 }
@@ -298,7 +298,7 @@ int ecg_cc_store(ecg_ctx* c, double* T1, double* T2) {
   return guarded(c, [&] {
     need_system(*c);
     if (T1) check(dev::d2h(T1, c->T1(), c->n1() * 8, c->st), "d2h T1");
-    if (T2) check(dev::d2h(T2, c->T2(), c->n2() * 8, c->st), "d2h T2");
+    if (T2) check(dev::d2h_large(T2, c->T2(), c->n2() * 8, c->st), "d2h T2");
     check(dev::sync(c->st), "sync");
   });
 }
@@ -339,7 +339,7 @@ int ecg_cc_solve(ecg_ctx* c, int dc, const ecg_cc_opts* opts, double* T1, double
     }
     if (it > o.maxit) it = o.maxit;
     check(dev::d2h(T1, c->T1(), c->n1() * 8, c->st), "d2h T1");
-    check(dev::d2h(T2, c->T2(), c->n2() * 8, c->st), "d2h T2");
+    check(dev::d2h_large(T2, c->T2(), c->n2() * 8, c->st), "d2h T2");
     check(dev::sync(c->st), "sync");
     if (out) {
       out[0] = r.E;
@@ -401,9 +401,11 @@ int ecg_lambda_residual(ecg_ctx* c, int dc, const double* T1, const double* T2, 
     need_ptr(U1, "U1");
     need_ptr(U2, "U2");
     check_finite(U1, c->n1(), "U1");
-    check_finite(U2, c->n2(), "U2");
     lambda_prepare(*c, dc != 0);
-    lambda_load_U(*c, U1, U2);
+    // checked on the device, in the residual's place: a refused U2 leaves U as it was
+    h2d_finite(*c, c->RU + c->n1(), U2, c->n2(), "U2");
+    lambda_load_U(*c, U1, nullptr);
+    check(dev::d2d(c->U + c->n1(), c->RU + c->n1(), c->n2() * 8, c->st), "d2d U2");
     lambda_residual(*c, dc != 0);
     lambda_store_R(*c, R1, R2);
   });
@@ -548,7 +550,7 @@ int ecg_cc_step_host(ecg_ctx* c, int dc, double* T1, double* T2, double* out) {
     if (T1 && T2) load_T(*c, T1, T2);
     IterResult r = cc_iteration(*c, dc != 0);
     if (T1) check(dev::d2h(T1, c->T1(), c->n1() * 8, c->st), "d2h T1");
-    if (T2) check(dev::d2h(T2, c->T2(), c->n2() * 8, c->st), "d2h T2");
+    if (T2) check(dev::d2h_large(T2, c->T2(), c->n2() * 8, c->st), "d2h T2");
     check(dev::sync(c->st), "sync");
     if (out) {
       out[0] = r.E;

@@ -29,6 +29,9 @@ void hfree_pinned(void* p);
 int h2d(void* dst, const void* src, size_t bytes, stream_t s);
 int d2h(void* dst, const void* src, size_t bytes, stream_t s);
 int d2d(void* dst, const void* src, size_t bytes, stream_t s);
+// d2h for results that may be large and go to pageable memory; the data has
+// arrived on return (where it was not staged: once the stream is synchronised).
+int d2h_large(void* dst, const void* src, size_t bytes, stream_t s);
 int memset0(void* dst, size_t bytes, stream_t s);
 // Record the launches issued on s after graph_capture_begin into a CUDA graph;
 // graph_capture_run ends the capture, runs the graph once, waits for it and

@@ -339,7 +339,7 @@ int ecg_int3c2e(ecg_ctx* ctx, const ecg_shells* ao, const ecg_shells* fit, doubl
     Scope scope{*c, c->allocs.size()};
     int64_t n = 0, naux = 0;
     const double* Z = int3c2e_device(*c, ao, fit, &n, &naux);
-    check(dev::d2h(out, Z, n * n * naux * 8, c->st), "d2h");
+    check(dev::d2h_large(out, Z, n * n * naux * 8, c->st), "d2h");
     check(dev::sync(c->st), "sync");
   });
 }
@@ -451,7 +451,7 @@ int ecg_df_mo(ecg_df* d, const double* C, int64_t nmo, double* B) {
     check(dev::gemm(c->st, 'N', 'N', nmo, nmo, n, 1.0, T1, nmo, dC, n, 0.0, dB, nmo, nL, nmo * n,
                     0, nmo * nmo),
           "gemm mmL");
-    check(dev::d2h(B, dB, nmo * nmo * nL * 8, c->st), "d2h");
+    check(dev::d2h_large(B, dB, nmo * nmo * nL * 8, c->st), "d2h");
     check(dev::sync(c->st), "sync");
   });
 }

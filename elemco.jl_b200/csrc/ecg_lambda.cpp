@@ -47,18 +47,18 @@ void lambda_prepare(Ctx& c, bool dc) {
 void lambda_load_U(Ctx& c, const double* U1h, const double* U2h) {
   ensure_lambda_buffers(c);
   check(dev::h2d(c.U, U1h, c.n1() * 8, c.st), "h2d U1");
-  check(dev::h2d(c.U + c.n1(), U2h, c.n2() * 8, c.st), "h2d U2");
+  if (U2h) check(dev::h2d(c.U + c.n1(), U2h, c.n2() * 8, c.st), "h2d U2");
 }
 
 void lambda_store_U(Ctx& c, double* U1h, double* U2h) {
   check(dev::d2h(U1h, c.U, c.n1() * 8, c.st), "d2h U1");
-  check(dev::d2h(U2h, c.U + c.n1(), c.n2() * 8, c.st), "d2h U2");
+  check(dev::d2h_large(U2h, c.U + c.n1(), c.n2() * 8, c.st), "d2h U2");
   check(dev::sync(c.st), "sync");
 }
 
 void lambda_store_R(Ctx& c, double* R1h, double* R2h) {
   if (R1h) check(dev::d2h(R1h, c.RU, c.n1() * 8, c.st), "d2h R1");
-  if (R2h) check(dev::d2h(R2h, c.RU + c.n1(), c.n2() * 8, c.st), "d2h R2");
+  if (R2h) check(dev::d2h_large(R2h, c.RU + c.n1(), c.n2() * 8, c.st), "d2h R2");
   check(dev::sync(c.st), "sync");
 }
 
