@@ -350,6 +350,35 @@ int graph_capture_run(stream_t s, int64_t* nodes) {
   return (int)e;
 }
 
+int graph_capture_keep(stream_t s, void** exec, int* kernels) {
+  cudaGraph_t g = nullptr;
+  cudaError_t e = cudaStreamEndCapture((cudaStream_t)s, &g);
+  if (e != cudaSuccess) return (int)e;
+  size_t n = 0;
+  cudaGraphGetNodes(g, nullptr, &n);
+  std::vector<cudaGraphNode_t> nodes(n);
+  cudaGraphGetNodes(g, nodes.data(), &n);
+  *kernels = 0;
+  for (cudaGraphNode_t q : nodes) {
+    cudaGraphNodeType t;
+    if (cudaGraphNodeGetType(q, &t) == cudaSuccess && t == cudaGraphNodeTypeKernel) ++*kernels;
+  }
+  cudaGraphExec_t x = nullptr;
+  e = cudaGraphInstantiate(&x, g, 0);
+  cudaGraphDestroy(g);
+  *exec = e == cudaSuccess ? x : nullptr;
+  return (int)e;
+}
+
+int graph_launch(stream_t s, void* exec, int kernels) {
+  note_launches(kernels);  // 0 where the recorded launches were counted
+  return (int)cudaGraphLaunch((cudaGraphExec_t)exec, (cudaStream_t)s);
+}
+
+void graph_free(void* exec) {
+  if (exec) cudaGraphExecDestroy((cudaGraphExec_t)exec);
+}
+
 void graph_capture_abort(stream_t s) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing((cudaStream_t)s, &cs) == cudaSuccess &&
@@ -862,6 +891,7 @@ void note_key(const std::string& key) {
 void set_tuning(bool on) { g_tuning.store(on); }
 bool tuning() { return g_tuning.load(); }
 bool stream_capturing(stream_t s) { return capturing((cudaStream_t)s); }
+bool graphs_usable(stream_t s) { return !g_timing && !tuning() && !stream_capturing(s); }
 
 bool tune_get(const std::string& key, int* value) {
   std::lock_guard<std::mutex> lk(g_tune_mu);

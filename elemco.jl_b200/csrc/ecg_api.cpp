@@ -325,11 +325,15 @@ int ecg_cc_solve(ecg_ctx* c, int dc, const ecg_cc_opts* opts, double* T1, double
       Ctx& c;
       ~Restore() { c.mixed_active = false; }
     } restore{*c};
+    IterGraph graph;
     for (it = 1; it <= o.maxit; ++it) {
       c->mixed_active = mixed_phase;
-      r = cc_iteration(*c, dc != 0);
+      r = cc_iteration(*c, dc != 0, &graph);
       if (mixed_phase) {
-        if (r.normR < 100.0 * o.thr) mixed_phase = false;
+        if (r.normR < 100.0 * o.thr) {
+          mixed_phase = false;
+          graph.reset();  // the recorded products are the mixed ones
+        }
         continue;
       }
       if (r.normR < o.thr && std::fabs(r.dE) < thren) {

@@ -118,7 +118,20 @@ struct IterResult {
   double E, ESS, EOS, normR, dE, En;
 };
 void cc_init_iterations(Ctx& c, const ecg_cc_opts& o);
-IterResult cc_iteration(Ctx& c, bool dc);
+// The launches of an iteration up to its first synchronisation, recorded by its
+// second run (the first one sizes scratch and sets kernels up).  For one solve:
+// precision, options and buffers must stay as they are, or reset() comes first.
+struct IterGraph {
+  void* exec = nullptr;
+  int kernels = 0, runs = 0;
+  void reset() {
+    dev::graph_free(exec);
+    exec = nullptr;
+    runs = 0;
+  }
+  ~IterGraph() { reset(); }
+};
+IterResult cc_iteration(Ctx& c, bool dc, IterGraph* graph = nullptr);
 void diis_reset(Ctx& c, DiisState& d, int maxdiis, double resthr, int64_t len, bool cs);
 // DIIS perform on device vectors (src/solvers/diis.jl:246-305)
 void diis_perform(Ctx& c, DiisState& d, double* amps, const double* res);

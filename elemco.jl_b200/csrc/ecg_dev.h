@@ -39,6 +39,13 @@ int memset0(void* dst, size_t bytes, stream_t s);
 int graph_capture_begin(stream_t s);
 int graph_capture_run(stream_t s, int64_t* nodes);
 void graph_capture_abort(stream_t s);  // end a capture in progress, discarding it
+// As graph_capture_run, but hands the graph to the caller (graph_free) instead
+// of running it; graph_launch queues it once more.
+int graph_capture_keep(stream_t s, void** exec, int* kernels);
+int graph_launch(stream_t s, void* exec, int kernels);
+void graph_free(void* exec);
+// Whether launches on s may be recorded: not while they are timed or tuned.
+bool graphs_usable(stream_t s);
 
 // C(m,n) = alpha * sum_k opA(A)(m,k) opB(B)(k,n) + beta * C(m,n), column-major;
 // ta/tb = 'N' or 'T'.  batch > 1 uses strides sa/sb/sc between instances.
