@@ -222,14 +222,16 @@ int d2d(void* dst, const void* src, size_t bytes, stream_t s) {
 // Device-to-host copies of tens of megabytes into pageable memory.  The driver's
 // own staging is one thread that also takes the page faults of a fresh array:
 // 234 MB (the factors of (H2O)4 cc-pVTZ) took 54 ms, ten times the transform that
-// made them.  Here the copy goes through a ring of pinned chunks (32 MiB a
-// stream, kept until the stream goes) that several host threads empty, so that
-// faults and host copies run side by side and beside the transfers.
-// Measured, the whole transform of that example with its copies: 65 -> 28 ms (23
-// on a second machine).
+// made them.  Here the copy goes through a ring of pinned chunks (8 MiB a stream,
+// kept until the stream goes) that several host threads empty, so that faults
+// and host copies run side by side and beside the transfers.  Measured, the whole
+// transform of that example with its copies: 65 -> 28 ms.  Pinning the ring is
+// part of a stream's first large copy: 32 MiB had cost it 30 to 40 ms (a first
+// Lambda residual at o = 16, v = 76 took 37 to 51 ms, now 10).  Below 32 MiB the
+// plain copy is as fast (12 MB results: 7.3 ms a residual either way).
 namespace {
-constexpr size_t CHUNK_BYTES = (size_t)1 << 20, NCHUNK = 32, STAGING_BYTES = CHUNK_BYTES * NCHUNK;
-constexpr size_t LARGE_COPY = (size_t)4 << 20;
+constexpr size_t CHUNK_BYTES = (size_t)512 << 10, NCHUNK = 16, STAGING_BYTES = CHUNK_BYTES * NCHUNK;
+constexpr size_t LARGE_COPY = (size_t)32 << 20;
 constexpr unsigned COPY_THREADS = 8;
 }  // namespace
 

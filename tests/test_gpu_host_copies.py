@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 def test_amplitudes_to_pageable_and_pinned_memory(ctx):
     import torch
     from ecgpu.synthetic import make_system
-    no, nv = 11, 150  # T2: 21.8 MB, six chunks and a remainder
+    no, nv = 13, 161  # T2: 35 MB, 66 chunks and a remainder
     B, h1, e0, _ = make_system(no, nv, 40, seed=3)
     ctx.set_system(B, h1, e0, no)
     _, T1, T2 = ctx.mp2()
