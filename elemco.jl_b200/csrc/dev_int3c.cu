@@ -99,8 +99,11 @@ __global__ void __launch_bounds__(128)
 
 namespace {
 
-// F_m(T) tables on the current device, written on its first use.
-int boys_table(const double** out) {
+// F_m(T) tables on the current device, written on its first use.  The table goes
+// up on the caller's stream, which is waited for before its address is handed
+// out: the contexts' streams do not wait for the default stream, and a copy from
+// pageable memory may return before the device has all of it.
+int boys_table(cudaStream_t s, const double** out) {
   static std::mutex mu;
   static const double* at[128] = {};
   int d = 0;
@@ -127,9 +130,11 @@ int boys_table(const double** out) {
       if (m > 0) F = (2.0L * T * F + et) / (2 * m - 1);
     }
   }
-  e = cudaMemcpyToSymbol(g_boys, tab.data(), tab.size() * sizeof(double));
   void* p = nullptr;
-  if (e == cudaSuccess) e = cudaGetSymbolAddress(&p, g_boys);
+  e = cudaGetSymbolAddress(&p, g_boys);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(p, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) at[d] = (const double*)p;
   *out = at[d];
   return (int)e;
@@ -248,9 +253,9 @@ int64_t Int3cPlan::table_doubles() const {
 }
 
 int Int3cPlan::run(stream_t st, double* tables, int64_t n, double* out) const {
-  const double* boys = nullptr;
-  if (int e = boys_table(&boys)) return e;
   cudaStream_t s = (cudaStream_t)st;
+  const double* boys = nullptr;
+  if (int e = boys_table(s, &boys)) return e;
   char* at = (char*)tables;
   int err = 0;
   auto put = [&](const void* p, size_t bytes) {
