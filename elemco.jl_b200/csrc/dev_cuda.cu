@@ -50,6 +50,7 @@ struct StreamState {
   void* staging = nullptr;  // pinned, STAGING_BYTES (d2h_large)
   bool staging_busy = false;
   unsigned long long tc_wait_ns = 0;  // 0: the default bound
+  int* wait_error = nullptr;  // time-out code of the stream's kernels, mapped host memory
 };
 std::mutex g_ss_mu;
 std::map<std::pair<cudaStream_t, int>, StreamState> g_ss;
@@ -74,6 +75,26 @@ bool capturing(cudaStream_t s) {
     return true;
   }
   return cs != cudaStreamCaptureStatusNone;
+}
+
+// Words of mapped host memory for the streams' time-out codes, 64 bytes apart;
+// a page of them is pinned at a time and a destroyed stream's word is reused.
+std::vector<int*> g_free_words;  // g_ss_mu
+int* take_word_locked() {
+  if (g_free_words.empty()) {
+    constexpr int PER_PAGE = 64, STEP = 16;
+    int* p = nullptr;
+    if (cudaHostAlloc((void**)&p, PER_PAGE * STEP * sizeof(int),
+                      cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    for (int i = PER_PAGE; i-- > 0;) g_free_words.push_back(p + i * STEP);
+  }
+  int* w = g_free_words.back();
+  g_free_words.pop_back();
+  *w = 0;
+  return w;
 }
 
 // Grow *p (holding *have bytes) to at least `want` bytes (plus `extra`
@@ -102,7 +123,11 @@ int stream_create(stream_t* s) {
   cudaStream_t st;
   int e = (int)cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
   *s = (stream_t)st;
-  if (!e && !wait_error()) e = (int)cudaErrorMemoryAllocation;  // before any capture
+  if (!e && !wait_error(*s)) {  // now, before any capture
+    e = (int)cudaErrorMemoryAllocation;
+    stream_destroy(*s);
+    *s = nullptr;
+  }
   return e;
 }
 
@@ -116,6 +141,7 @@ void stream_destroy(stream_t s) {
       if (it->second.splitk) cudaFree(it->second.splitk);
       if (it->second.split) cudaFree(it->second.split);
       if (it->second.staging) cudaFreeHost(it->second.staging);
+      if (it->second.wait_error) g_free_words.push_back(it->second.wait_error);
       g_ss.erase(it);
     }
   }
@@ -155,27 +181,17 @@ int sync(stream_t s) { return (int)cudaStreamSynchronize((cudaStream_t)s); }
 // The kernels write the code straight into host memory, so that reading it after
 // a synchronisation costs a load: copying one device variable per kernel back
 // took four synchronous copies, 30 to 40 us each time, four times an iteration.
-int* wait_error() {
-  static std::atomic<int*> word{nullptr};
-  int* p = word.load(std::memory_order_acquire);
-  if (p) return p;
-  static std::mutex mu;
-  std::lock_guard<std::mutex> lk(mu);
-  p = word.load(std::memory_order_relaxed);
-  if (!p) {
-    if (cudaHostAlloc((void**)&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) !=
-        cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
-    *p = 0;
-    word.store(p, std::memory_order_release);
-  }
-  return p;
+// A word per stream: a context reads and clears the time-outs of its own kernels
+// and of no other's, and after its stream is synchronised nothing writes it.
+int* wait_error(stream_t s) {
+  std::lock_guard<std::mutex> lk(g_ss_mu);
+  StreamState& ss = stream_state_locked((cudaStream_t)s);
+  if (!ss.wait_error) ss.wait_error = take_word_locked();
+  return ss.wait_error;
 }
 
-int tc_error(int* code) {
-  int* p = wait_error();
+int tc_error(stream_t s, int* code) {
+  int* p = wait_error(s);
   if (!p) return (int)cudaErrorMemoryAllocation;
   *code = *(volatile int*)p;
   if (*code) *(volatile int*)p = 0;

@@ -97,7 +97,7 @@ void sync_scalars(Ctx& c, int count) {
   check(dev::d2h(c.hscal, c.dscal, sizeof(double) * count, c.st), "d2h scalars");
   check(dev::sync(c.st), "stream sync");
   int tc = 0;
-  check(dev::tc_error(&tc), "tc_error");
+  check(dev::tc_error(c.st, &tc), "tc_error");
   if (tc)
     throw Error(ECG_ERR_TIMEOUT, "GEMM wait timed out (code " + std::to_string(tc) + ")");
 }

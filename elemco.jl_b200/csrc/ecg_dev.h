@@ -364,16 +364,16 @@ int gemm_splitk_noalloc(stream_t s, char ta, char tb, int64_t m, int64_t n, int6
 
 // Split-BF16 tensor-core GEMM (tcgen05, FP32 accumulate, ~FP32 accuracy),
 // same interface as gemm().  tc_error() returns and clears the time-out code
-// of the kernels with bounded mbarrier waits (0 = none; 1-4 tensor-core GEMM,
+// of stream s's kernels with bounded mbarrier waits (s synchronised; 0 = none; 1-4 tensor-core GEMM,
 // 17 TMA-staged FP64 GEMM, 33 FP32 (T) energy kernel, 49 FP64 K builds,
 // 65-68 tensor-core K builds).
 int gemm_mixed(stream_t s, char ta, char tb, int64_t m, int64_t n, int64_t k, double alpha,
                const double* A, int64_t lda, const double* B, int64_t ldb, double beta,
                double* C, int64_t ldc);
-int tc_error(int* code);
-// Where those kernels leave it: one word of pinned host memory that every
+int tc_error(stream_t s, int* code);
+// Where those kernels leave it: the stream's word of pinned host memory that the
 // device maps (nullptr: it could not be allocated).
-int* wait_error();
+int* wait_error(stream_t s);
 // Split-K scratch of stream s on the current device (at least n doubles;
 // grown on demand, after s has drained, never during stream capture: nullptr
 // then, or when the allocation fails) and its fixed-order reduction
