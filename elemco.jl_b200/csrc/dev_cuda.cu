@@ -50,7 +50,7 @@ struct StreamState {
   void* staging = nullptr;  // pinned, STAGING_BYTES (d2h_large)
   bool staging_busy = false;
   unsigned long long tc_wait_ns = 0;  // 0: the default bound
-  int* wait_error = nullptr;  // time-out code of the stream's kernels, mapped host memory
+  int* wait_error = nullptr;  // time-out codes [WAIT_KERNELS], mapped host memory
 };
 std::mutex g_ss_mu;
 std::map<std::pair<cudaStream_t, int>, StreamState> g_ss;
@@ -77,12 +77,13 @@ bool capturing(cudaStream_t s) {
   return cs != cudaStreamCaptureStatusNone;
 }
 
-// Words of mapped host memory for the streams' time-out codes, 64 bytes apart;
-// a page of them is pinned at a time and a destroyed stream's word is reused.
+// Mapped host memory for the streams' time-out codes, 64 bytes a stream; a page of
+// it is pinned at a time and a destroyed stream's part is reused.
 std::vector<int*> g_free_words;  // g_ss_mu
-int* take_word_locked() {
+int* take_words_locked() {
   if (g_free_words.empty()) {
     constexpr int PER_PAGE = 64, STEP = 16;
+    static_assert(WAIT_KERNELS <= STEP, "a stream's words");
     int* p = nullptr;
     if (cudaHostAlloc((void**)&p, PER_PAGE * STEP * sizeof(int),
                       cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
@@ -93,7 +94,7 @@ int* take_word_locked() {
   }
   int* w = g_free_words.back();
   g_free_words.pop_back();
-  *w = 0;
+  std::fill(w, w + WAIT_KERNELS, 0);
   return w;
 }
 
@@ -123,7 +124,7 @@ int stream_create(stream_t* s) {
   cudaStream_t st;
   int e = (int)cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
   *s = (stream_t)st;
-  if (!e && !wait_error(*s)) {  // now, before any capture
+  if (!e && !wait_error(*s, 0)) {  // now, before any capture
     e = (int)cudaErrorMemoryAllocation;
     stream_destroy(*s);
     *s = nullptr;
@@ -181,20 +182,22 @@ int sync(stream_t s) { return (int)cudaStreamSynchronize((cudaStream_t)s); }
 // The kernels write the code straight into host memory, so that reading it after
 // a synchronisation costs a load: copying one device variable per kernel back
 // took four synchronous copies, 30 to 40 us each time, four times an iteration.
-// A word per stream: a context reads and clears the time-outs of its own kernels
-// and of no other's, and after its stream is synchronised nothing writes it.
-int* wait_error(stream_t s) {
+// Words per stream: a context reads and clears the time-outs of its own kernels
+// and of no other's, and after its stream is synchronised nothing writes them.
+int* wait_error(stream_t s, int kernel) {
   std::lock_guard<std::mutex> lk(g_ss_mu);
   StreamState& ss = stream_state_locked((cudaStream_t)s);
-  if (!ss.wait_error) ss.wait_error = take_word_locked();
-  return ss.wait_error;
+  if (!ss.wait_error) ss.wait_error = take_words_locked();
+  return ss.wait_error ? ss.wait_error + kernel : nullptr;
 }
 
-int tc_error(stream_t s, int* code) {
-  int* p = wait_error(s);
+int tc_error(stream_t s, int* codes) {
+  volatile int* p = wait_error(s, 0);
   if (!p) return (int)cudaErrorMemoryAllocation;
-  *code = *(volatile int*)p;
-  if (*code) *(volatile int*)p = 0;
+  for (int i = 0; i < WAIT_KERNELS; ++i) {
+    codes[i] = p[i];
+    if (codes[i]) p[i] = 0;
+  }
   return 0;
 }
 

@@ -271,7 +271,7 @@ int launch_dtma(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap& mb, c
   if (gy > 65535 || nz > 65535) return (int)cudaErrorInvalidConfiguration;
   dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)nz);
   unsigned long long w = tc_wait((stream_t)st);
-  int* err = wait_error((stream_t)st);
+  int* err = wait_error((stream_t)st, WAIT_DGEMM);
   if (!err) return (int)cudaErrorMemoryAllocation;
   kern<<<grid, Cfg::THREADS, Cfg::SMEM, st>>>(ma, mb, out, k, kslice, split, w ? w : WAIT_NS,
                                               err);

@@ -352,7 +352,7 @@ int launch_energy(cudaStream_t st, dim3 grid, const CUtensorMap* maps, int nv,
     if (d >= 0 && d < 128) done[d].store(true, std::memory_order_release);
   }
   const unsigned long long w = tc_wait((stream_t)st);
-  int* err = wait_error((stream_t)st);
+  int* err = wait_error((stream_t)st, WAIT_ENERGY);
   if (!err) return (int)cudaErrorMemoryAllocation;
   kern<<<grid, L::THREADS, L::SMEM, st>>>(maps[0], maps[1], maps[2], maps[3], nv, eijk_tab, ev,
                                           tt_tab, tri, ntri, scratch, w ? w : WAIT_NS, err);

@@ -307,7 +307,7 @@ int kbuild(stream_t s, const KbGemm& g, int nitems, const KbItem* items) {
   cudaStream_t st = (cudaStream_t)s;
   const uint64_t w = tc_wait(s);
   const unsigned long long wns = w ? (unsigned long long)w : WAIT_NS;
-  int* err = wait_error(s);
+  int* err = wait_error(s, WAIT_KBUILD);
   if (!err) return (int)cudaErrorMemoryAllocation;
   const int slot = ktime_begin(s, KT_DGEMM);
   int e;

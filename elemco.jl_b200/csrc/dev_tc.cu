@@ -624,7 +624,7 @@ int launch_tc(cudaStream_t st, const TcMaps& maps, const TcSegs& segs, int kbt, 
   const int64_t items = (int64_t)mt * nt * S;
   const unsigned grid = (unsigned)(items < 148 ? items : 148);
   const unsigned long long wns = wait_bound(st);
-  int* err = wait_error((stream_t)st);
+  int* err = wait_error((stream_t)st, WAIT_TC);
   if (!err) return (int)cudaErrorMemoryAllocation;
   // useful BF16 products: 2 m n K per slice pair (zero padding not counted)
   const double work = 2.0 * (double)m * (double)n * (double)seg_depth(segs) * Cfg::NPAIR *

@@ -420,7 +420,7 @@ int tc_kbuild(stream_t s, const TcKbuild& g, int nitems, const KbItem* items, in
   }
   cudaStream_t st = (cudaStream_t)s;
   const uint64_t w = tc_wait(s);
-  int* err = wait_error(s);
+  int* err = wait_error(s, WAIT_TCKBUILD);
   if (!err) return (int)cudaErrorMemoryAllocation;
   const int slot = ktime_begin(s, KT_TCGEMM);
   tc_kbuild_kernel<<<(unsigned)std::min<int64_t>(total, 148), KT_THREADS, KT_SMEM, st>>>(

@@ -255,7 +255,7 @@ int ecg_cc_residual(ecg_ctx* c, int dc, const double* T1, const double* T2, doub
     cc_residual(*c, dc != 0);
     if (R1) check(dev::d2h(R1, c->R1(), c->n1() * 8, c->st), "d2h R1");
     if (R2) check(dev::d2h_large(R2, c->R2(), c->n2() * 8, c->st), "d2h R2");
-    check(dev::sync(c->st), "sync");
+    sync_checked(*c);
   });
 }
 
@@ -267,7 +267,7 @@ int ecg_cc_load(ecg_ctx* c, const double* T1, const double* T2, const ecg_cc_opt
     opts_or_default(opts, o);
     load_T_or_resident(*c, T1, T2);
     cc_init_iterations(*c, o);
-    check(dev::sync(c->st), "sync");
+    sync_checked(*c);
   });
 }
 
@@ -299,7 +299,7 @@ int ecg_cc_store(ecg_ctx* c, double* T1, double* T2) {
     need_system(*c);
     if (T1) check(dev::d2h(T1, c->T1(), c->n1() * 8, c->st), "d2h T1");
     if (T2) check(dev::d2h_large(T2, c->T2(), c->n2() * 8, c->st), "d2h T2");
-    check(dev::sync(c->st), "sync");
+    sync_checked(*c);
   });
 }
 
@@ -344,7 +344,7 @@ int ecg_cc_solve(ecg_ctx* c, int dc, const ecg_cc_opts* opts, double* T1, double
     if (it > o.maxit) it = o.maxit;
     check(dev::d2h(T1, c->T1(), c->n1() * 8, c->st), "d2h T1");
     check(dev::d2h_large(T2, c->T2(), c->n2() * 8, c->st), "d2h T2");
-    check(dev::sync(c->st), "sync");
+    sync_checked(*c);
     if (out) {
       out[0] = r.E;
       out[1] = r.ESS;
@@ -555,7 +555,7 @@ int ecg_cc_step_host(ecg_ctx* c, int dc, double* T1, double* T2, double* out) {
     IterResult r = cc_iteration(*c, dc != 0);
     if (T1) check(dev::d2h(T1, c->T1(), c->n1() * 8, c->st), "d2h T1");
     if (T2) check(dev::d2h_large(T2, c->T2(), c->n2() * 8, c->st), "d2h T2");
-    check(dev::sync(c->st), "sync");
+    sync_checked(*c);
     if (out) {
       out[0] = r.E;
       out[1] = r.ESS;
@@ -628,11 +628,7 @@ int ecg_diag_gemm(ecg_ctx* c, char ta, char tb, int64_t m, int64_t n, int64_t k,
     else
       check(dev::gemm(c->st, ta, tb, m, n, k, alpha, dA, lda, dB, ldb, beta, dC, ldc), "gemm");
     check(dev::d2h(C, dC, sC * 8, c->st), "d2h");
-    check(dev::sync(c->st), "sync");
-    int tc = 0;
-    check(dev::tc_error(c->st, &tc), "tc_error");
-    if (tc) throw Error(ECG_ERR_TIMEOUT, "GEMM wait timed out (code " +
-                                             std::to_string(tc) + ")");
+    sync_checked(*c);
   });
 }
 

@@ -93,13 +93,25 @@ void Ctx::free_all() {
 
 double scal(Ctx& c, int i) { return c.hscal[i]; }
 
+void sync_checked(Ctx& c) {
+  check(dev::sync(c.st), "stream sync");
+  int codes[dev::WAIT_KERNELS];
+  check(dev::tc_error(c.st, codes), "tc_error");
+  std::string list;
+  for (int t : codes)
+    if (t) list += (list.empty() ? "" : ", ") + std::to_string(t);
+  if (!list.empty()) throw Error(ECG_ERR_TIMEOUT, "bounded wait timed out (code " + list + ")");
+}
+
+void drop_time_outs(Ctx& c) noexcept {
+  if (!c.st) return;
+  int codes[dev::WAIT_KERNELS];
+  if (dev::sync(c.st) == 0) dev::tc_error(c.st, codes);
+}
+
 void sync_scalars(Ctx& c, int count) {
   check(dev::d2h(c.hscal, c.dscal, sizeof(double) * count, c.st), "d2h scalars");
-  check(dev::sync(c.st), "stream sync");
-  int tc = 0;
-  check(dev::tc_error(c.st, &tc), "tc_error");
-  if (tc)
-    throw Error(ECG_ERR_TIMEOUT, "GEMM wait timed out (code " + std::to_string(tc) + ")");
+  sync_checked(c);
 }
 
 // --------------------------------------------------------------- setup
@@ -246,7 +258,7 @@ void setup_system(Ctx& c, int no, int nv, int nq, const double* B, const double*
   {
     std::vector<double> tmp(n * n);
     check(dev::d2h(tmp.data(), c.fock, n * n * 8, c.st), "d2h");
-    check(dev::sync(c.st), "sync");
+    sync_checked(c);
     c.fock_host = tmp;
     std::vector<double> fvo(v * o);
     for (int64_t i = 0; i < o; ++i)
@@ -259,7 +271,7 @@ void setup_system(Ctx& c, int no, int nv, int nq, const double* B, const double*
   con.permute(1.0, c.klcd, "ijab", 0.0, c.Kvvoo, "abij");
   con(1.0, c.Bvo, "ckQ", c.Bvo, "dlQ", 0.0, c.V1, "ckdl");
   con.permute(1.0, c.V1, "ckdl", 0.0, c.V2, "cldk");
-  check(dev::sync(c.st), "setup sync");
+  sync_checked(c);
   c.have_system = true;
 }
 

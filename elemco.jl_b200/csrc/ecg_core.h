@@ -136,7 +136,13 @@ void diis_reset(Ctx& c, DiisState& d, int maxdiis, double resthr, int64_t len, b
 // DIIS perform on device vectors (src/solvers/diis.jl:246-305)
 void diis_perform(Ctx& c, DiisState& d, double* amps, const double* res);
 double scal(Ctx& c, int i);
-void sync_scalars(Ctx& c, int count);
+// Waits for the context's stream; a bounded device-side wait that ran out since the
+// last check is an ECG_ERR_TIMEOUT.  Every call whose results rest on kernels with
+// such waits (all FP64 and tensor-core GEMMs) ends with one.
+void sync_checked(Ctx& c);
+// Waits likewise and forgets time-outs: a call that failed leaves none to the next.
+void drop_time_outs(Ctx& c) noexcept;
+void sync_scalars(Ctx& c, int count);  // the first `count` scalars to hscal, sync_checked
 
 // Runs f, turning the library's exceptions into a status code and a message
 // (per context, or per thread for calls without one).
@@ -148,13 +154,16 @@ int guarded(Ctx* c, F&& f) {
     if (c) c->err.clear();
     return ECG_OK;
   } catch (const Error& e) {
+    if (c) drop_time_outs(*c);
     if (c) c->err = e.what();
     else noctx_error_store(e.what());
     return e.code;
   } catch (const std::bad_alloc&) {
+    if (c) drop_time_outs(*c);
     if (c) c->err = "host out of memory";
     return ECG_ERR_OOM;
   } catch (const std::exception& e) {
+    if (c) drop_time_outs(*c);
     if (c) c->err = e.what();
     return ECG_ERR_ARG;
   }

@@ -363,17 +363,18 @@ int gemm_splitk_noalloc(stream_t s, char ta, char tb, int64_t m, int64_t n, int6
                         double beta, double* C, int64_t ldc, int* nsplit);
 
 // Split-BF16 tensor-core GEMM (tcgen05, FP32 accumulate, ~FP32 accuracy),
-// same interface as gemm().  tc_error() returns and clears the time-out code
+// same interface as gemm().  tc_error() returns and clears the time-out codes
 // of stream s's kernels with bounded mbarrier waits (s synchronised; 0 = none; 1-4 tensor-core GEMM,
 // 17 TMA-staged FP64 GEMM, 33 FP32 (T) energy kernel, 49 FP64 K builds,
 // 65-68 tensor-core K builds).
 int gemm_mixed(stream_t s, char ta, char tb, int64_t m, int64_t n, int64_t k, double alpha,
                const double* A, int64_t lda, const double* B, int64_t ldb, double beta,
                double* C, int64_t ldc);
-int tc_error(stream_t s, int* code);
-// Where those kernels leave it: the stream's word of pinned host memory that the
-// device maps (nullptr: it could not be allocated).
-int* wait_error(stream_t s);
+int tc_error(stream_t s, int* codes);  // codes[WAIT_KERNELS]
+// Where those kernels leave them: a word of the stream's for each kind of kernel, in
+// pinned host memory that the device maps (nullptr: it could not be allocated).
+enum { WAIT_TC, WAIT_DGEMM, WAIT_ENERGY, WAIT_KBUILD, WAIT_TCKBUILD, WAIT_KERNELS };
+int* wait_error(stream_t s, int kernel);
 // Split-K scratch of stream s on the current device (at least n doubles;
 // grown on demand, after s has drained, never during stream capture: nullptr
 // then, or when the allocation fails) and its fixed-order reduction

@@ -377,7 +377,7 @@ int ecg_df_create(ecg_ctx* ctx, const ecg_shells* ao, const ecg_shells* fit, con
     // AAL[mn, L] = sum_P (mn|P) M[P, L]
     check(dev::gemm(c->st, 'N', 'N', n * n, nL, np, 1.0, Z, n * n, dM, np, 0.0, d->aal, n * n),
           "gemm AAL");
-    check(dev::sync(c->st), "sync");
+    sync_checked(*c);
   });
   if (st != ECG_OK) {
     ecg_df_destroy(d);
@@ -427,7 +427,7 @@ int ecg_df_fock(ecg_df* d, const double* h, const double* Cocc, int64_t nocc, do
             "gemm K");
     }
     check(dev::d2h(F, dF, n * n * 8, c->st), "d2h");
-    check(dev::sync(c->st), "sync");
+    sync_checked(*c);
   });
 }
 
@@ -452,7 +452,7 @@ int ecg_df_mo(ecg_df* d, const double* C, int64_t nmo, double* B) {
                     0, nmo * nmo),
           "gemm mmL");
     check(dev::d2h_large(B, dB, nmo * nmo * nL * 8, c->st), "d2h");
-    check(dev::sync(c->st), "sync");
+    sync_checked(*c);
   });
 }
 

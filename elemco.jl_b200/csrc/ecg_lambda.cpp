@@ -40,7 +40,7 @@ void lambda_prepare(Ctx& c, bool dc) {
   // vT[m,b,i,j] = sum_dc d_vovv[b,m,d,c] T2[d,c,j,i]
   con(1.0, dvovv, "bdcm", c.T2(), "dcji", 0.0, c.vT, "mbij");
   c.ws.release(mark);
-  check(dev::sync(c.st), "sync");
+  sync_checked(c);
   c.lambda_ready = true;
 }
 
@@ -53,13 +53,13 @@ void lambda_load_U(Ctx& c, const double* U1h, const double* U2h) {
 void lambda_store_U(Ctx& c, double* U1h, double* U2h) {
   check(dev::d2h(U1h, c.U, c.n1() * 8, c.st), "d2h U1");
   check(dev::d2h_large(U2h, c.U + c.n1(), c.n2() * 8, c.st), "d2h U2");
-  check(dev::sync(c.st), "sync");
+  sync_checked(c);
 }
 
 void lambda_store_R(Ctx& c, double* R1h, double* R2h) {
   if (R1h) check(dev::d2h(R1h, c.RU, c.n1() * 8, c.st), "d2h R1");
   if (R2h) check(dev::d2h_large(R2h, c.RU + c.n1(), c.n2() * 8, c.st), "d2h R2");
-  check(dev::sync(c.st), "sync");
+  sync_checked(c);
 }
 
 // D1 and dD1 (n x n, device) from U in c.U and T in c.T (cc_lagrange.jl:793-848).
@@ -113,7 +113,7 @@ void one_rdm(Ctx& c, double* D1h, double* dD1h) {
   const int64_t n = c.n;
   if (D1h) check(dev::d2h(D1h, c.D1, n * n * 8, c.st), "d2h D1");
   if (dD1h) check(dev::d2h(dD1h, c.dD1, n * n * 8, c.st), "d2h dD1");
-  check(dev::sync(c.st), "sync");
+  sync_checked(c);
 }
 
 // copy an r x q block at offset `off` of an n x n column-major matrix
