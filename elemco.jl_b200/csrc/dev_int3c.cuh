@@ -255,6 +255,7 @@ __device__ __forceinline__ void int3c_part(const Launch& g, const Part& p, int G
 #pragma unroll 1
     for (int x = lane; x < NAB; x += G) {
       const int a = pr.aoff + x % NA, b = pr.boff + x / NA;
+      if (pr.aoff == pr.boff && a < b) continue;  // of a shell with itself: (b, a) writes both
       const double v = f * acc[m * NAB + x];
       o[a + n * b] = v;
       o[b + n * a] = v;
