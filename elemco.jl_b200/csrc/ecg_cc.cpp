@@ -43,6 +43,9 @@ void Ctx::release_to(size_t nallocs) {
 
 void Ctx::ensure_ws(int64_t nd) {
   if (ws.capacity() >= nd) return;
+  // the old arena goes first (both may not fit together); until the new one is
+  // there the context has none, or its old size again where the new one is refused
+  const int64_t old = ws.capacity();
   if (st) dev::sync(st);
   for (size_t q = 0; q < allocs.size(); ++q)
     if (allocs[q].first == (void*)ws_base) {
@@ -51,7 +54,17 @@ void Ctx::ensure_ws(int64_t nd) {
       allocs.erase(allocs.begin() + q);
       break;
     }
-  ws_base = alloc(nd, "workspace");
+  ws_base = nullptr;
+  ws.init(nullptr, 0);
+  try {
+    ws_base = alloc(nd, "workspace");
+  } catch (...) {
+    if (old > 0) {
+      ws_base = alloc(old, "workspace");
+      ws.init(ws_base, old);
+    }
+    throw;
+  }
   ws.init(ws_base, nd);
 }
 
@@ -603,6 +616,7 @@ static void sym_pinv_solve(int m, const std::vector<double>& B, const std::vecto
 void diis_reset(Ctx& c, DiisState& d, int maxdiis, double resthr, int64_t len, bool cs) {
   if (maxdiis < 1 || maxdiis > 8) throw Error(ECG_ERR_ARG, "maxdiis must be in 1..8");
   if (d.len != len || (int)d.amp.size() != maxdiis) {
+    d.len = 0;  // no history, should an allocation be refused
     d.amp.assign(maxdiis, nullptr);
     d.res.assign(maxdiis, nullptr);
     for (int i = 0; i < maxdiis; ++i) {

@@ -17,12 +17,15 @@
 namespace ecg {
 
 static void ensure_lambda_buffers(Ctx& c) {
-  if (c.U) return;
-  c.U = c.alloc(c.n1() + c.n2(), "U");
-  c.RU = c.alloc(c.n1() + c.n2(), "RU");
-  c.vT = c.alloc((int64_t)c.no * c.no * c.no * c.nv, "vT");
-  c.D1 = c.alloc((int64_t)c.n * c.n, "D1");
-  c.dD1 = c.alloc((int64_t)c.n * c.n, "dD1");
+  // one by one: a call that the memory cap stopped in between goes on here
+  auto have = [&](double*& p, int64_t nd, const char* what) {
+    if (!p) p = c.alloc(nd, what);
+  };
+  have(c.U, c.n1() + c.n2(), "U");
+  have(c.RU, c.n1() + c.n2(), "RU");
+  have(c.vT, (int64_t)c.no * c.no * c.no * c.nv, "vT");
+  have(c.D1, (int64_t)c.n * c.n, "D1");
+  have(c.dD1, (int64_t)c.n * c.n, "dD1");
 }
 
 void lambda_prepare(Ctx& c, bool dc) {

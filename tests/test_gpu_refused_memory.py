@@ -1,0 +1,65 @@
+"""Calls that the memory cap stops half way: a status, no pointer to memory that is
+not there, and a context that goes on."""
+import numpy as np
+import pytest
+
+import ecgpu
+from ecgpu._lib import ECG_ERR_OOM, ECG_ERR_STATE
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(no, nv, nq):
+    from ecgpu.synthetic import make_system
+    B, h1, e0, _ = make_system(no, nv, nq, seed=6)
+    return B, h1, e0, no
+
+
+def _same(x, y):
+    return all(np.array_equal(a, b) for a, b in zip(x, y))
+
+
+def test_lambda_residual_under_a_growing_cap():
+    """Refused at each of its buffers and at the larger workspace in turn; after each
+    refusal the residual still runs, and the first call that fits is right."""
+    with ecgpu.Context(0) as c:
+        c.set_system(*_system(3, 20, 40))
+        _, T1, T2 = c.mp2()
+        U1, U2 = 2.0 * T1, 2.0 * T2 - T2.transpose(1, 0, 2, 3)
+        ref = c.cc_residual(T1, T2)
+        refused, cap = set(), 0
+        while True:
+            cap += 1 << 14
+            c.set_mem_cap(cap)
+            try:
+                R = c.lambda_residual(T1, T2, U1, U2)
+                break
+            except ecgpu.ECGError as e:
+                assert e.code == ECG_ERR_OOM
+                refused.add(str(e).rsplit(" ", 1)[1])
+            assert _same(c.cc_residual(T1, T2), ref)
+        assert {"U", "RU", "workspace"} <= refused, refused
+        c.set_mem_cap(0)
+        with ecgpu.Context(0) as d:
+            d.set_system(*_system(3, 20, 40))
+            assert _same(R, d.lambda_residual(T1, T2, U1, U2))
+
+
+def test_iterations_without_their_history():
+    """A cc_load whose longer DIIS history is refused leaves none: a step then is a
+    call-order error, and the next cc_load works."""
+    with ecgpu.Context(0) as c:
+        c.set_system(*_system(4, 24, 48))
+        _, T1, T2 = c.mp2()
+        c.cc_load(T1, T2, opts=c.opts(maxdiis=3))
+        ref = c.cc_step()
+        c.set_mem_cap(1 << 16)
+        with pytest.raises(ecgpu.ECGError) as e:
+            c.cc_load(T1, T2, opts=c.opts(maxdiis=6))
+        assert e.value.code == ECG_ERR_OOM
+        c.set_mem_cap(0)
+        with pytest.raises(ecgpu.ECGError) as e:
+            c.cc_step()
+        assert e.value.code == ECG_ERR_STATE
+        c.cc_load(T1, T2, opts=c.opts(maxdiis=6))
+        assert np.array_equal(c.cc_step(), ref)
