@@ -16,6 +16,7 @@
 #include <cstring>
 
 #include "ecg_core.h"
+#include "ladder_blocks.h"
 
 namespace ecg {
 
@@ -136,12 +137,10 @@ void sync_scalars(Ctx& c, int count) {
 // 2.01; o=14, v=100: 5.78 / 5.97 / 5.98, eight blocks 6.05), and the tiles with
 // b < a are skipped inside a block.
 static int64_t ladder_na(int64_t nv) {
-  const int64_t budget = (int64_t)1 << 28;  // doubles (2 GiB) for one V block
   // an even block start keeps the block's rows of B on 16 bytes for TMA
   int64_t na = ((nv + 7) / 8 + 1) / 2 * 2;
   na = std::max(na, (((int64_t)1 << 25) / (nv * nv * nv)) / 2 * 2);
-  na = std::min<int64_t>(na, std::max<int64_t>(1, budget / std::max<int64_t>(nv * nv * nv, 1)));
-  return std::max<int64_t>(1, std::min(na, nv));
+  return std::max<int64_t>(1, std::min({na, ladder_na_limit(nv), nv}));
 }
 
 // Pair tables for the symmetric ladder (host build, one upload).
@@ -384,9 +383,12 @@ void ladder(Ctx& c, const double* Bf, const double* BfT, const double* T2, doubl
   // (H2O)6/cc-pVTZ, the whole mixed ladder moves the mixed-product fixed
   // point by -4 uEh, the other short contractions by +10).
   const double big = 67108864.0;
-  const bool mv = c.mixed_active && (double)(v * c.lblocks[0].na) * (double)(v * v) * Q >= big;
-  const bool mp = c.mixed_active && (double)maxpp * nijp * ncdp >= big;
-  const bool mm = c.mixed_active && nijm > 0 && (double)maxpp * nijm * ncdm >= big;
+  // The size is that of an eighth of the virtual space whatever the blocks are, so
+  // that their size, a matter of speed and memory, does not decide the precision.
+  const int64_t na8 = ladder_eighth(v), pp8 = ladder_pairs(v, na8);
+  const bool mv = c.mixed_active && (double)(v * na8) * (double)(v * v) * Q >= big;
+  const bool mp = c.mixed_active && (double)pp8 * nijp * ncdp >= big;
+  const bool mm = c.mixed_active && nijm > 0 && (double)pp8 * nijm * ncdm >= big;
   constexpr int NSL = 3;
   dev::TcOperand oB, oTs, oTa, oVp, oVm;
   uint16_t *pB = nullptr, *pTs = nullptr, *pTa = nullptr, *pVp = nullptr, *pVm = nullptr;
