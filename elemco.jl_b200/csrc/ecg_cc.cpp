@@ -130,19 +130,6 @@ void sync_scalars(Ctx& c, int count) {
 
 // --------------------------------------------------------------- setup
 
-// a-block size of the symmetric ladder: Vblk holds v^2 na (v - a0) doubles.
-// An eighth of the virtual space, but as much of it as 256 MiB of V hold: at
-// small v a block's five launches cost more than they compute (CCSD iteration
-// of o=12, v=57 with 256 / 64 / 32 MiB: 1.76 / 1.80 / 1.84 ms, eight blocks
-// 2.01; o=14, v=100: 5.78 / 5.97 / 5.98, eight blocks 6.05), and the tiles with
-// b < a are skipped inside a block.
-static int64_t ladder_na(int64_t nv) {
-  // an even block start keeps the block's rows of B on 16 bytes for TMA
-  int64_t na = ((nv + 7) / 8 + 1) / 2 * 2;
-  na = std::max(na, (((int64_t)1 << 25) / (nv * nv * nv)) / 2 * 2);
-  return std::max<int64_t>(1, std::min({na, ladder_na_limit(nv), nv}));
-}
-
 // Pair tables for the symmetric ladder (host build, one upload).
 static void ladder_setup(Ctx& c) {
   const int v = c.nv, o = c.no;
