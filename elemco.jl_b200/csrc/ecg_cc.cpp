@@ -144,19 +144,24 @@ static void ladder_setup(Ctx& c) {
       ij.push_back(i);
       ij.push_back(j);
     }
-  const int na = (int)ladder_na(v);
-  c.lblocks.clear();
-  for (int a0 = 0; a0 < v; a0 += na) {
-    Ctx::LadderBlock b{a0, std::min(na, v - a0), 0, 0, (int64_t)pr.size() / 2};
-    for (int a = a0; a < a0 + b.na; ++a)
-      for (int bb = a; bb < v; ++bb) {
-        pr.push_back(a);
-        pr.push_back(bb);
-      }
-    b.npp = (int)((int64_t)pr.size() / 2 - b.poff);
-    b.npm = b.npp - b.na;
-    c.lblocks.push_back(b);
-  }
+  for (int a = 0; a < v; ++a)
+    for (int b = a; b < v; ++b) {
+      pr.push_back(a);
+      pr.push_back(b);
+    }
+  auto blocks = [&](int na, std::vector<Ctx::LadderBlock>& out) {
+    out.clear();
+    int64_t poff = 0;
+    for (int a0 = 0; a0 < v; a0 += na) {
+      Ctx::LadderBlock b{a0, std::min(na, v - a0), 0, 0, poff};
+      b.npp = (int)ladder_pairs(v - a0, b.na);
+      b.npm = b.npp - b.na;
+      poff += b.npp;
+      out.push_back(b);
+    }
+  };
+  blocks((int)ladder_na(o, v, c.nq), c.lblocks);
+  blocks((int)ladder_eighth(v), c.lblocks8);
   auto up = [&](std::vector<int>& x, const char* what) {
     int* d = (int*)c.alloc(((int64_t)x.size() + 1) / 2, what);
     check(dev::h2d(d, x.data(), x.size() * sizeof(int), c.st), "h2d tables");
@@ -222,9 +227,7 @@ void setup_system(Ctx& c, int no, int nv, int nq, const double* B, const double*
   c.hscal = (double*)dev::hmalloc_pinned(256 * sizeof(double));
   if (!c.hscal) throw Error(ECG_ERR_OOM, "pinned host scalars");
 
-  const int64_t n2 = c.n2(), na = ladder_na(v);
-  int64_t wsn = 16 * n2 + 6 * v * o * Q + 3 * v * v * Q + 2 * n * n * Q + 4 * o * o * o * o +
-                2 * na * v * v * v + 8 * n * n + (1 << 16);
+  const int64_t wsn = system_workspace(o, v, Q);
   c.ws_base = c.alloc(wsn, "workspace");
   c.ws.init(c.ws_base, wsn);
 
@@ -348,16 +351,6 @@ void ladder(Ctx& c, const double* Bf, const double* BfT, const double* T2, doubl
   double* Ta = c.ws.get(std::max<int64_t>(ldm * nijm, 1));
   check(dev::ladder_pack_t(s, (int)v, (int)o, T2, c.cdp, c.ijp, Ts, Ta, ldp, ldm),
         "ladder pack T");
-  int64_t maxpp = 0, maxv = 0;
-  for (auto& b : c.lblocks) {
-    maxpp = std::max<int64_t>(maxpp, b.npp);
-    maxv = std::max<int64_t>(maxv, v * b.na * v * (v - b.a0));
-  }
-  double* V = c.ws.get(maxv);
-  double* Vp = c.ws.get(ldp * maxpp);
-  double* Vm = c.ws.get(std::max<int64_t>(ldm * maxpp, 1));
-  double* Lp = c.ws.get(maxpp * nijp);
-  double* Lm = c.ws.get(std::max<int64_t>(maxpp * nijm, 1));
   const double* Bl = BfT;  // FP64 V builds read it in an even pitch
   int64_t ldb = v * v;
   // Mixed precision: the operands shared by every a-block (BfT for the V
@@ -376,6 +369,14 @@ void ladder(Ctx& c, const double* Bf, const double* BfT, const double* T2, doubl
   const bool mv = c.mixed_active && (double)(v * na8) * (double)(v * v) * Q >= big;
   const bool mp = c.mixed_active && (double)pp8 * nijp * ncdp >= big;
   const bool mm = c.mixed_active && nijm > 0 && (double)pp8 * nijm * ncdm >= big;
+  // the BF16 slices of a block are storage of their own, which stays small
+  const auto& blocks = mp || mm ? c.lblocks8 : c.lblocks;
+  const int64_t maxpp = blocks[0].npp;  // the first block has the most
+  double* V = c.ws.get(v * blocks[0].na * v * v);
+  double* Vp = c.ws.get(ldp * maxpp);
+  double* Vm = c.ws.get(std::max<int64_t>(ldm * maxpp, 1));
+  double* Lp = c.ws.get(maxpp * nijp);
+  double* Lm = c.ws.get(std::max<int64_t>(maxpp * nijm, 1));
   constexpr int NSL = 3;
   dev::TcOperand oB, oTs, oTa, oVp, oVm;
   uint16_t *pB = nullptr, *pTs = nullptr, *pTa = nullptr, *pVp = nullptr, *pVm = nullptr;
@@ -403,7 +404,7 @@ void ladder(Ctx& c, const double* Bf, const double* BfT, const double* T2, doubl
   }
   const bool fused = mp && mm;  // V+/- packed into BF16 slices directly
   const bool vf32 = fused && mv && Q <= dev::TC_ACC_K;
-  for (auto& b : c.lblocks) {
+  for (auto& b : blocks) {
     const int64_t nb = v - b.a0;
     // V[c,a',d,b''] = sum_Q BfT[c,a0+a',Q] BfT[d,a0+b'',Q], needed for b >= a only
     if (mv) {

@@ -83,7 +83,7 @@ struct Ctx {
     int a0, na, npp, npm;
     int64_t poff;  // offset (in pairs) into `pairs`
   };
-  std::vector<LadderBlock> lblocks;
+  std::vector<LadderBlock> lblocks, lblocks8;  // lblocks8: of an eighth of the virtual space
 
   DiisState diis;
   ecg_cc_opts opts;

@@ -33,7 +33,7 @@ void lambda_prepare(Ctx& c, bool dc) {
   ensure_lambda_buffers(c);
   const int64_t o = c.no, v = c.nv;
   // one o v^3 block for d_vovv plus a same-sized permute temporary
-  c.ensure_ws(2 * o * v * v * v + 16 * c.n2() + (1 << 20));
+  c.ensure_ws(2 * o * v * v * v + 14 * c.n2() + (1 << 20) - (1 << 15) - (o + v) * (o + v));
   dress(c, c.T1());
   Contractor con = c.con();
   const int64_t mark = c.ws.mark();

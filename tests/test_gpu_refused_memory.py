@@ -63,3 +63,26 @@ def test_iterations_without_their_history():
         assert e.value.code == ECG_ERR_STATE
         c.cc_load(T1, T2, opts=c.opts(maxdiis=6))
         assert np.array_equal(c.cc_step(), ref)
+
+
+# bytes that a system took with blocks of an eighth of the virtual space in the
+# ladder and term-by-term rings: set up, and with the Lambda equations' buffers
+SIZES = [((5, 19, 60), 4654816, 11344880), ((12, 57, 200), 172595432, 186068024),
+         ((16, 76, 280), 498504128, 569683648), ((1, 40, 60), 15056944, 15110400),
+         ((20, 20, 60), 38081360, 43315280)]
+
+
+@pytest.mark.parametrize("size,cap,cap_lambda", SIZES)
+def test_systems_fit_the_memory_they_took(size, cap, cap_lambda):
+    no, nv, nq = size
+    sys_ = _system(no, nv, nq)
+    with ecgpu.Context(0) as c, ecgpu.Context(0) as free:
+        c.set_mem_cap(cap)
+        for x in (c, free):
+            x.set_system(*sys_)
+        _, T1, T2 = c.mp2()
+        T1 = 0.02 * np.random.default_rng(1).standard_normal(T1.shape)
+        assert _same(c.cc_residual(T1, T2), free.cc_residual(T1, T2))
+        c.set_mem_cap(cap_lambda)
+        U1, U2 = 2.0 * T1, 2.0 * T2 - T2.transpose(1, 0, 2, 3)
+        assert _same(c.lambda_residual(T1, T2, U1, U2), free.lambda_residual(T1, T2, U1, U2))
