@@ -234,6 +234,10 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
   const bool lam = (U1h != nullptr);
   const bool mixed = c.mixed_active;
   dev::stream_t s = c.st;
+  if (o < 2) {  // no triplet
+    *et = *etb = 0.0;
+    return;
+  }
   // everything allocated here is freed on exit
   struct Scope {
     Ctx& c;
@@ -245,9 +249,7 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
   ops.mixed = mixed;
   ops.vq = (v + 1) / 2 * 2;
   ops.v2p = (v2 + 1) / 2 * 2;
-  double* On = c.alloc(o * o * o * v, "(T) ovoo");
   Contractor con = c.con();
-  con(1.0, c.Boo, "ljQ", c.Bvo, "ckQ", 0.0, On, "ljck");
   // vvvo[b,c,d,k] = (bd|ck): per k one GEMM over rows (b,d) into a slab
   // [b,d,c], whose orders [b,c,d] and [c,b,d] the K builds read
   const int64_t d3[3] = {v, v, v};
@@ -266,7 +268,22 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
     V2 = c.alloc(slab * o, "(T) vvvo [c,b,d,k]");
     Onp = c.alloc(ops.vq * o * o * o, "(T) -ovoo");
   }
+  // -ovoo: the ovoo segments share the vvvo segments' sign
   const size_t mark = c.allocs.size();
+  double* On = c.alloc(o * o * o * v, "(T) ovoo");
+  con(1.0, c.Boo, "ljQ", c.Bvo, "ckQ", 0.0, On, "ljck");
+  if (mixed) {
+    check(dev::axpby(s, o * o * o * v, -1.0, On, 0.0, On), "-ovoo");
+    check(dev::tc_split_stack(s, On, v, o, o * o, 1, 0, o * o, o, o, o * o * v, bo, &ops.Ons),
+          "split ovoo");
+  } else {  // as [c,l,j,k]
+    const int64_t dl[4] = {o, o, v, o};
+    const int pl[4] = {2, 0, 1, 3};
+    double* Oc = c.alloc(o * o * o * v, "(T) ovoo [c,l,j,k]");
+    check(dev::permute(s, 4, dl, pl, -1.0, On, 0.0, Oc), "-ovoo");
+    check(dev::repitch(s, v, o * o * o, Oc, v, Onp, ops.vq), "-ovoo pitch");
+  }
+  c.release_to(mark);
   double* D = c.alloc(v3, "(T) vvvo slab");
   double* Dt = mixed || pad ? c.alloc(v3, "(T) vvvo slab") : nullptr;
   const double* Bl = c.Bvv;
@@ -297,20 +314,11 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
       if (pad) check(dev::repitch(s, v2, v, Dt, v2, V, ops.v2p), "pad vvvo");
     }
   }
-  // -ovoo: the ovoo segments share the vvvo segments' sign
   if (mixed) {
-    check(dev::axpby(s, o * o * o * v, -1.0, On, 0.0, On), "-ovoo");
-    check(dev::tc_split_stack(s, On, v, o, o * o, 1, 0, o * o, o, o, o * o * v, bo, &ops.Ons),
-          "split ovoo");
     ops.V1s.base = bv;
     ops.V2s.base = bv + evs * o;
     ops.V1s.items = ops.V2s.items = o;
-  } else {  // as [c,l,j,k]
-    const int64_t dl[4] = {o, o, v, o};
-    const int pl[4] = {2, 0, 1, 3};
-    double* Oc = c.alloc(o * o * o * v, "(T) ovoo [c,l,j,k]");
-    check(dev::permute(s, 4, dl, pl, -1.0, On, 0.0, Oc), "-ovoo");
-    check(dev::repitch(s, v, o * o * o, Oc, v, Onp, ops.vq), "-ovoo pitch");
+  } else {
     ops.V1 = V1;
     ops.V2 = V2;
     ops.On = Onp;
@@ -352,25 +360,15 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
             tr.push_back({i, j, k, f, eps[i + i * n] + eps[j + j * n] + eps[k + k * n]});
           }
   const int64_t nt = (int64_t)tr.size();
-  if (nt == 0) {
-    *et = *etb = 0.0;
-    return;
-  }
-  // batches of NB triplets, one K slot each, within a 4 GiB budget
+  // batches of NB triplets, one K slot each, within a 4 GiB budget (fewer where
+  // memory ends before: see the allocation of K)
   const int64_t esz = mixed ? 4 : 8;
   const int64_t vp = mixed ? (v + 3) / 4 * 4 : v;  // K's a pitch (see k_map)
   const int64_t kstride = (vp * v2 + 31) / 32 * 32;
   const int64_t per = kstride * esz * (lam ? 2 : 1);
   int64_t nbmax = std::min<int64_t>({256, nt, ((int64_t)4 << 30) / per});
   if (c.triples_batch > 0) nbmax = std::min(nbmax, c.triples_batch);
-  const int NB = (int)std::max<int64_t>(1, nbmax);
-  void* K = c.alloc((NB * kstride * esz + 7) / 8, "(T) K slots");
-  void* KU = lam ? (void*)c.alloc((NB * kstride * esz + 7) / 8, "(T) K(Lambda) slots") : nullptr;
-  const std::vector<dev::KbItem> items = k_items(c, tr, NB, kstride);
-  static_assert(sizeof(dev::KbItem) % 8 == 0, "whole doubles");
-  dev::KbItem* items_d = reinterpret_cast<dev::KbItem*>(
-      c.alloc((int64_t)(items.size() * sizeof(dev::KbItem) / 8), "(T) item table"));
-  check(dev::h2d(items_d, items.data(), items.size() * sizeof(dev::KbItem), s), "h2d");
+  int NB = (int)std::max<int64_t>(1, nbmax);
 
   // energy terms per triplet: g = T1 (or U1/2), f[a,i] = fock[i, o+a], <ij|ab>, T2 (or U2c)
   std::vector<double> gh(v * o), fh(v * o);
@@ -448,6 +446,24 @@ void pert_triples(Ctx& c, const double* U1h, const double* U2h, double* et, doub
   check(dev::h2d(tri, trih.data(), 3 * ncube * sizeof(int), s), "h2d");
   double* part = c.alloc(dev::triples_energy_scratch_len((int)v, NB), "(T) partial sums");
   double* Et = c.alloc(2 * nt, "(T) energies");
+  static_assert(sizeof(dev::KbItem) % 8 == 0, "whole doubles");
+  dev::KbItem* items_d = reinterpret_cast<dev::KbItem*>(
+      c.alloc((int64_t)(kGemms * nt * sizeof(dev::KbItem) / 8), "(T) item table"));
+  void *K = nullptr, *KU = nullptr;
+  while (!K) {
+    const size_t slots = c.allocs.size();
+    try {
+      void* k = c.alloc((NB * kstride * esz + 7) / 8, "(T) K slots");
+      if (lam) KU = c.alloc((NB * kstride * esz + 7) / 8, "(T) K(Lambda) slots");
+      K = k;
+    } catch (const Error& e) {
+      c.release_to(slots);
+      if (e.code != ECG_ERR_OOM || NB == 1) throw;
+      NB /= 2;
+    }
+  }
+  const std::vector<dev::KbItem> items = k_items(c, tr, NB, kstride);
+  check(dev::h2d(items_d, items.data(), items.size() * sizeof(dev::KbItem), s), "h2d");
 
   // batch loop: the first batch runs directly (first-use set-up of the
   // kernels), the others are recorded as one CUDA graph and run once

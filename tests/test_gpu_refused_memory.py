@@ -86,3 +86,23 @@ def test_systems_fit_the_memory_they_took(size, cap, cap_lambda):
         c.set_mem_cap(cap_lambda)
         U1, U2 = 2.0 * T1, 2.0 * T2 - T2.transpose(1, 0, 2, 3)
         assert _same(c.lambda_residual(T1, T2, U1, U2), free.lambda_residual(T1, T2, U1, U2))
+
+
+# a system and what (T) took beside it
+SIZES_T = [((5, 19, 60), 4654816 + 2306000), ((10, 61, 200), 168437712 + 418787680),
+           ((16, 76, 280), 498504128 + 1014903376), ((20, 20, 60), 38081360 + 21566328),
+           ((17, 83, 304), 671143536 + 1330940256)]
+
+
+@pytest.mark.parametrize("size,cap", SIZES_T)
+def test_pert_t_fits_the_memory_it_took(size, cap):
+    """At odd virtual counts the copies in even pitches come on top, which batches of
+    fewer triplets make up for; the energies do not depend on the batches."""
+    no, nv, nq = size
+    sys_ = _system(no, nv, nq)
+    with ecgpu.Context(0) as c, ecgpu.Context(0) as free:
+        c.set_mem_cap(cap)
+        for x in (c, free):
+            x.set_system(*sys_)
+            x.mp2()
+        assert c.pert_t() == free.pert_t()
