@@ -47,6 +47,7 @@ struct StreamState {
   size_t splitk_len = 0;  // doubles
   void* split = nullptr;
   size_t split_bytes = 0;
+  size_t copy_room = SIZE_MAX;  // set_copy_room
   void* staging = nullptr;  // pinned, STAGING_BYTES (d2h_large)
   bool staging_busy = false;
   unsigned long long tc_wait_ns = 0;  // 0: the default bound
@@ -165,6 +166,34 @@ void* split_scratch(stream_t s, size_t bytes) {
   std::lock_guard<std::mutex> lk(g_ss_mu);
   StreamState& ss = stream_state_locked((cudaStream_t)s);
   return grow((cudaStream_t)s, &ss.split, &ss.split_bytes, bytes, bytes / 4);
+}
+
+// The same for copies that a call can do without: nullptr beyond the stream's room.
+static void* copy_scratch(stream_t s, size_t bytes) {
+  std::lock_guard<std::mutex> lk(g_ss_mu);
+  StreamState& ss = stream_state_locked((cudaStream_t)s);
+  if (bytes > ss.split_bytes && bytes + bytes / 4 > ss.copy_room) return nullptr;
+  return grow((cudaStream_t)s, &ss.split, &ss.split_bytes, bytes, bytes / 4);
+}
+
+size_t scratch_bytes(stream_t s) {
+  std::lock_guard<std::mutex> lk(g_ss_mu);
+  return stream_state_locked((cudaStream_t)s).split_bytes;
+}
+
+void release_scratch(stream_t s) {
+  std::lock_guard<std::mutex> lk(g_ss_mu);
+  StreamState& ss = stream_state_locked((cudaStream_t)s);
+  if (!ss.split || capturing((cudaStream_t)s)) return;
+  cudaStreamSynchronize((cudaStream_t)s);
+  cudaFree(ss.split);
+  ss.split = nullptr;
+  ss.split_bytes = 0;
+}
+
+void set_copy_room(stream_t s, size_t bytes) {
+  std::lock_guard<std::mutex> lk(g_ss_mu);
+  stream_state_locked((cudaStream_t)s).copy_room = bytes;
 }
 
 int set_tc_wait(stream_t s, uint64_t ns) {
@@ -1185,7 +1214,7 @@ static bool pack_for_tma(stream_t s, const Gemm& q, Gemm* out) {
   const double cp = 3.0 + 0.521 * (double)(((q.k + c.S - 1) / c.S + 15) / 16 * x) / eff +
                     (c.S > 1 ? 3.0 : 0.0);
   if (tma >= cp) return false;
-  double* buf = (double*)split_scratch(s, need);
+  double* buf = (double*)copy_scratch(s, need);
   if (!buf) return false;  // no scratch (stream capture, memory): cp.async takes it as it is
   for (Side* d : {&A, &B})
     if (!d->ok) {

@@ -131,8 +131,11 @@ const char* ecg_last_error(const ecg_ctx* c) {
 
 int ecg_set_mem_cap(ecg_ctx* c, uint64_t bytes) {
   if (!c) return ECG_ERR_ARG;
-  c->memcap = bytes;
-  return ECG_OK;
+  return guarded(c, [&] {
+    check(dev::set_device(c->device), "cudaSetDevice");
+    c->memcap = bytes;
+    c->count_memory(0);
+  });
 }
 
 int ecg_set_precision(ecg_ctx* c, int prec) {

@@ -20,14 +20,30 @@
 
 namespace ecg {
 
-double* Ctx::alloc(int64_t nd, const char* what) {
-  size_t bytes = (size_t)std::max<int64_t>(nd, 1) * sizeof(double);
+void Ctx::count_memory(int64_t bytes) {
+  memused += bytes;
+  if (st) dev::set_copy_room(st, !memcap ? SIZE_MAX : memcap > memused ? memcap - memused : 0);
+}
+
+void* Ctx::take_memory(size_t bytes, const char* what) {
+  // the stream's scratch, which the copies of odd pitches may fill, gives way
+  if (memcap && memused + dev::scratch_bytes(st) + bytes > memcap) dev::release_scratch(st);
   if (memcap && memused + bytes > memcap)
     throw Error(ECG_ERR_OOM, std::string("device memory cap exceeded allocating ") + what);
   void* p = dev::dmalloc(bytes);
+  if (!p && dev::scratch_bytes(st)) {
+    dev::release_scratch(st);
+    p = dev::dmalloc(bytes);
+  }
   if (!p) throw Error(ECG_ERR_OOM, std::string("cudaMalloc failed for ") + what);
+  count_memory((int64_t)bytes);
+  return p;
+}
+
+double* Ctx::alloc(int64_t nd, const char* what) {
+  const size_t bytes = (size_t)std::max<int64_t>(nd, 1) * sizeof(double);
+  void* p = take_memory(bytes, what);
   allocs.push_back({p, bytes});
-  memused += bytes;
   return (double*)p;
 }
 
@@ -38,7 +54,7 @@ void Ctx::release_to(size_t nallocs) {
     auto a = allocs.back();
     allocs.pop_back();
     dev::dfree(a.first);
-    memused -= a.second;
+    count_memory(-(int64_t)a.second);
   }
 }
 
@@ -51,7 +67,7 @@ void Ctx::ensure_ws(int64_t nd) {
   for (size_t q = 0; q < allocs.size(); ++q)
     if (allocs[q].first == (void*)ws_base) {
       dev::dfree(allocs[q].first);
-      memused -= allocs[q].second;
+      count_memory(-(int64_t)allocs[q].second);
       allocs.erase(allocs.begin() + q);
       break;
     }
@@ -75,7 +91,7 @@ void* Ctx::ensure_tc(size_t bytes) {
   for (size_t q = 0; q < allocs.size(); ++q)
     if (allocs[q].first == tc_base) {
       dev::dfree(allocs[q].first);
-      memused -= allocs[q].second;
+      count_memory(-(int64_t)allocs[q].second);
       allocs.erase(allocs.begin() + q);
       break;
     }
@@ -90,7 +106,8 @@ void Ctx::free_all() {
   if (st) dev::sync(st);
   for (auto& a : allocs) dev::dfree(a.first);
   allocs.clear();
-  memused = handle_bytes;  // handles keep their memory across systems
+  // handles keep their memory across systems
+  count_memory((int64_t)handle_bytes - (int64_t)memused);
   if (hscal) dev::hfree_pinned(hscal);
   hscal = nullptr;
   have_system = false;

@@ -101,6 +101,8 @@ struct Ctx {
   double* R2() { return R + n1(); }
 
   double* alloc(int64_t ndoubles, const char* what);
+  void* take_memory(size_t bytes, const char* what);  // counted, not on the stack of alloc()
+  void count_memory(int64_t bytes);                   // adds to memused
   void release_to(size_t nallocs);  // free allocations made after the first nallocs
   void ensure_ws(int64_t ndoubles);  // grow the workspace arena (outside any capture)
   void* ensure_tc(size_t bytes);     // grow the split-operand storage (contents are lost)

@@ -382,6 +382,12 @@ int* wait_error(stream_t s, int kernel);
 double* splitk_buffer(stream_t s, size_t n);
 // Scratch of stream s for gemm_mixed's BF16 operand slices (same rules).
 void* split_scratch(stream_t s, size_t bytes);
+// What stream s holds of it; release_scratch waits for s and gives it back.
+size_t scratch_bytes(stream_t s);
+void release_scratch(stream_t s);
+// The copies in even pitches that the FP64 GEMM makes for TMA live in it too, as
+// long as it stays within `bytes` (no bound to begin with).
+void set_copy_room(stream_t s, size_t bytes);
 // Bound (ns) of the tensor-core kernels' main-loop waits on stream s
 // (0 = the default second); the kernels' final waits keep the second.
 int set_tc_wait(stream_t s, uint64_t ns);

@@ -363,11 +363,7 @@ int ecg_df_create(ecg_ctx* ctx, const ecg_shells* ao, const ecg_shells* fit, con
     d->n = nao;
     d->nL = nL;
     d->bytes = (size_t)std::max<int64_t>((int64_t)nao * nao * nL, 1) * 8;
-    if (c->memcap && c->memused + d->bytes > c->memcap)
-      throw Error(ECG_ERR_OOM, "device memory cap exceeded allocating the DF factors");
-    d->aal = (double*)dev::dmalloc(d->bytes);
-    if (!d->aal) throw Error(ECG_ERR_OOM, "cudaMalloc failed for the DF factors");
-    c->memused += d->bytes;
+    d->aal = (double*)c->take_memory(d->bytes, "the DF factors");
     c->handle_bytes += d->bytes;
     Scope scope{*c, c->allocs.size()};
     int64_t n = 0, np = 0;
@@ -462,7 +458,7 @@ int ecg_df_destroy(ecg_df* d) {
     Ctx* c = d->ctx;
     if (c->st) dev::sync(c->st);
     dev::dfree(d->aal);
-    c->memused -= d->bytes;
+    c->count_memory(-(int64_t)d->bytes);
     c->handle_bytes -= d->bytes;
   }
   delete d;
