@@ -384,58 +384,60 @@ __global__ void __launch_bounds__(THREADS_TC, 1)
 
 // X(r,k) = src[r*sr + k*sk] (FP64, R x K) -> dst[s][r][k] BF16 (s < nsl), zero
 // padded to Rp x Kp.  32x32 tiles through shared memory so that reads are
-// coalesced whichever of sr / sk is the unit stride.
-__global__ void split_kernel(const double* __restrict__ src, int64_t R, int64_t K, int64_t sr,
+// coalesced whichever of sr / sk is the unit stride.  The items of a stack (TcStack;
+// one item: d = 1) go round the grid's y extent, which a stack of pairs can exceed.
+__global__ void split_kernel(const double* __restrict__ src0, int64_t R, int64_t K, int64_t sr,
                              int64_t sk, int64_t Rp, int64_t Kp, int nsl,
-                             __nv_bfloat16* __restrict__ dst, uint32_t dr, int64_t d, int64_t s0,
-                             int64_t s1) {
+                             __nv_bfloat16* __restrict__ dst0, uint32_t dr, int64_t items,
+                             int64_t d, int64_t s0, int64_t s1) {
   __shared__ double tile[32][33];
   // tile indices in 32 bits (an operand whose BF16 slices fit in device
   // memory has fewer than 2^25 tiles): one 64-bit division per tile would
   // cost more instructions than its 1024 elements
   const uint32_t tk = (uint32_t)((Kp + 31) / 32), ntile = tk * (uint32_t)((Rp + 31) / 32);
   const bool rfast = (sr == 1 || dr > 0);
-  // item blockIdx.y of a stack (TcStack; one item: d = 1)
-  src += ((int64_t)blockIdx.y % d) * s0 + ((int64_t)blockIdx.y / d) * s1;
-  dst += (int64_t)blockIdx.y * nsl * Rp * Kp;
   auto rowoff = [&](int64_t r) {
     if (dr == 0) return r * sr;
     const uint32_t q = (uint32_t)r / dr;
     return (int64_t)((uint32_t)r - q * dr) + (int64_t)q * sr;
   };
-  for (uint32_t t = blockIdx.x; t < ntile; t += gridDim.x) {
-    const int64_t r0 = (int64_t)(t / tk) * 32, k0 = (int64_t)(t % tk) * 32;
-    // the four loads of a thread are issued before any of them is used
-    double xs[4];
+  for (int64_t z = blockIdx.y; z < items; z += gridDim.y) {
+    const double* src = src0 + (z % d) * s0 + (z / d) * s1;
+    __nv_bfloat16* dst = dst0 + z * nsl * Rp * Kp;
+    for (uint32_t t = blockIdx.x; t < ntile; t += gridDim.x) {
+      const int64_t r0 = (int64_t)(t / tk) * 32, k0 = (int64_t)(t % tk) * 32;
+      // the four loads of a thread are issued before any of them is used
+      double xs[4];
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
-      const int j = threadIdx.y + 8 * jj;
-      int64_t r, k;
-      if (rfast) { r = r0 + threadIdx.x; k = k0 + j; } else { r = r0 + j; k = k0 + threadIdx.x; }
-      xs[jj] = (r < R && k < K) ? src[rowoff(r) + k * sk] : 0.0;
-    }
-#pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
-      const int j = threadIdx.y + 8 * jj;
-      if (rfast) tile[j][threadIdx.x] = xs[jj];   // tile[k][r]
-      else tile[threadIdx.x][j] = xs[jj];         // tile[k][r]
-    }
-    __syncthreads();
-    for (int j = threadIdx.y; j < 32; j += 8) {
-      const int64_t r = r0 + j, k = k0 + threadIdx.x;
-      if (r < Rp && k < Kp) {
-        const double x = tile[threadIdx.x][j];
-        const __nv_bfloat16 h0 = __double2bfloat16(x);
-        const double e1 = x - (double)__bfloat162float(h0);
-        const __nv_bfloat16 h1 = __double2bfloat16(e1);
-        const double e2 = e1 - (double)__bfloat162float(h1);
-        const int64_t o = r * Kp + k, sl = Rp * Kp;
-        dst[o] = h0;
-        dst[o + sl] = h1;
-        if (nsl == 3) dst[o + 2 * sl] = __double2bfloat16(e2);
+      for (int jj = 0; jj < 4; ++jj) {
+        const int j = threadIdx.y + 8 * jj;
+        int64_t r, k;
+        if (rfast) { r = r0 + threadIdx.x; k = k0 + j; } else { r = r0 + j; k = k0 + threadIdx.x; }
+        xs[jj] = (r < R && k < K) ? src[rowoff(r) + k * sk] : 0.0;
       }
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        const int j = threadIdx.y + 8 * jj;
+        if (rfast) tile[j][threadIdx.x] = xs[jj];   // tile[k][r]
+        else tile[threadIdx.x][j] = xs[jj];         // tile[k][r]
+      }
+      __syncthreads();
+      for (int j = threadIdx.y; j < 32; j += 8) {
+        const int64_t r = r0 + j, k = k0 + threadIdx.x;
+        if (r < Rp && k < Kp) {
+          const double x = tile[threadIdx.x][j];
+          const __nv_bfloat16 h0 = __double2bfloat16(x);
+          const double e1 = x - (double)__bfloat162float(h0);
+          const __nv_bfloat16 h1 = __double2bfloat16(e1);
+          const double e2 = e1 - (double)__bfloat162float(h1);
+          const int64_t o = r * Kp + k, sl = Rp * Kp;
+          dst[o] = h0;
+          dst[o + sl] = h1;
+          if (nsl == 3) dst[o + 2 * sl] = __double2bfloat16(e2);
+        }
+      }
+      __syncthreads();
     }
-    __syncthreads();
   }
 }
 
@@ -572,7 +574,7 @@ void launch_split(cudaStream_t st, const double* src, int64_t R, int64_t K, int6
                   int64_t sk, int64_t Rp, int64_t Kp, int nsl, __nv_bfloat16* dst) {
   const int64_t tiles = ((Rp + 31) / 32) * ((Kp + 31) / 32);
   const unsigned g = (unsigned)(tiles < 148 * 16 ? tiles : 148 * 16);
-  split_kernel<<<g, dim3(32, 8), 0, st>>>(src, R, K, sr, sk, Rp, Kp, nsl, dst, 0, 1, 0, 0);
+  split_kernel<<<g, dim3(32, 8), 0, st>>>(src, R, K, sr, sk, Rp, Kp, nsl, dst, 0, 1, 1, 0, 0);
   note_launches(1);
 }
 
@@ -685,16 +687,17 @@ int tc_split(stream_t s, const double* src, int64_t rows, int64_t k, int64_t sr,
 int tc_split_stack(stream_t s, const double* src, int64_t rows, int64_t k, int64_t sr, int64_t sk,
                    int64_t dr, int64_t items, int64_t d, int64_t s0, int64_t s1, void* dst,
                    TcStack* out) {
-  if (rows <= 0 || k <= 0 || items <= 0 || items > 65535 || d <= 0 || dr < 0 || !src || !dst ||
+  if (rows <= 0 || k <= 0 || items <= 0 || d <= 0 || dr < 0 || !src || !dst ||
       !out || rows >= ((int64_t)1 << 31))
     return (int)cudaErrorInvalidValue;
   if (((uintptr_t)dst & 15) != 0) return (int)cudaErrorMisalignedAddress;
   const int64_t Rp = pad_rows(rows), Kp = pad_k(k);
   const int64_t tiles = ((Rp + 31) / 32) * ((Kp + 31) / 32);
-  const dim3 g((unsigned)std::min<int64_t>(tiles, 148 * 16), (unsigned)items);
+  const dim3 g((unsigned)std::min<int64_t>(tiles, 148 * 16),
+               (unsigned)std::min<int64_t>(items, 512));
   split_kernel<<<g, dim3(32, 8), 0, (cudaStream_t)s>>>(src, rows, k, sr, sk, Rp, Kp, 2,
-                                                       (__nv_bfloat16*)dst, (uint32_t)dr, d, s0,
-                                                       s1);
+                                                       (__nv_bfloat16*)dst, (uint32_t)dr, items,
+                                                       d, s0, s1);
   note_launches(1);
   *out = TcStack{dst, rows, k, items};
   return (int)cudaGetLastError();
