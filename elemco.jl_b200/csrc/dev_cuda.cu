@@ -933,8 +933,19 @@ std::atomic<bool> g_tuning{false};
 // whether the table has entries of FP64 GEMMs ("dgemmt ..."): without them a
 // launch need not spell out its key
 std::atomic<bool> g_tune_fp64{false};
-void note_key(const std::string& key) {
-  if (key.compare(0, 7, "dgemmt ") == 0) g_tune_fp64.store(true);
+// Which TMA tiles the FP64 entries' numbers 1 to 3 stand for: an entry of the table
+// itself, written with them.  A file without it was tuned when these were 128x64,
+// 64x128 and 128x128 tiles, and its entries that name them are left out (the rule
+// then picks); numbers 0 and the cp.async tiles' mean what they did.
+const char* const TILES_KEY = "dgemmt-tiles";
+constexpr int TILES = 2;
+void note_key(const std::string& key) {  // g_tune_mu
+  if (key.compare(0, 7, "dgemmt ") != 0) return;
+  g_tune_fp64.store(true);
+  g_tune[TILES_KEY] = TILES;
+}
+bool foreign_tile(const std::string& key, int value) {
+  return key.compare(0, 7, "dgemmt ") == 0 && value % 8 > 4;
 }
 }  // namespace
 
@@ -985,8 +996,12 @@ int tune_parse(const std::string& text) {
     if (!e || *e != '\0') return -1;
     add[line.substr(0, sp)] = (int)v;
   }
+  const auto tiles = add.find(TILES_KEY);
+  const bool ours = tiles != add.end() && tiles->second == TILES;
+  if (tiles != add.end()) add.erase(tiles);
   std::lock_guard<std::mutex> lk(g_tune_mu);
   for (auto& kv : add) {
+    if (!ours && foreign_tile(kv.first, kv.second)) continue;
     g_tune[kv.first] = kv.second;
     note_key(kv.first);
   }

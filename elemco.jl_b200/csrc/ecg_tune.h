@@ -7,7 +7,8 @@
 // CUDA events; the output is saved before and restored after each run, so the
 // call's result is unaffected), records the fastest and runs it.  Without an
 // entry and with tuning off the launcher's fixed rule applies.  The table can
-// be saved to and loaded from a text file ("key value" lines).
+// be saved to and loaded from a text file ("key value" lines; the entry
+// "dgemmt-tiles" says which tiles the FP64 entries number).
 #pragma once
 #include <cstdint>
 #include <functional>

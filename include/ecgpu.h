@@ -93,7 +93,8 @@ int ecg_set_option(ecg_ctx* ctx, int32_t key, int64_t value);
  * own operands (the result is unchanged) and records the fastest.
  * ecg_tune_save writes the table to a text file ("key value" lines),
  * ecg_tune_load merges such a file into it; *entries (may be NULL) receives
- * the table size afterwards. */
+ * the table size afterwards.  Entries of an earlier version's file that name
+ * tiles this one does not have are left out. */
 int ecg_tune_save(ecg_ctx* ctx, const char* path, int64_t* entries);
 int ecg_tune_load(ecg_ctx* ctx, const char* path, int64_t* entries);
 

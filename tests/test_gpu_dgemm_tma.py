@@ -22,7 +22,8 @@ pytestmark = pytest.mark.gpu
 
 def _force(ctx, tmp_path, m, n, k, ta, tb, cfg, S):
     p = tmp_path / f"force_{m}_{n}_{k}_{ta}{tb}.txt"
-    p.write_text(f"dgemmt {m} {n} {k} 1 {int(ta == 'T')}{int(tb == 'T')} {8 * S + 4 + cfg}\n")
+    p.write_text("dgemmt-tiles 2\n"
+                 f"dgemmt {m} {n} {k} 1 {int(ta == 'T')}{int(tb == 'T')} {8 * S + 4 + cfg}\n")
     ctx.tune_load(p)
 
 
