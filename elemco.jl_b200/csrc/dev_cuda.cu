@@ -340,9 +340,9 @@ int d2h_large(void* dst, const void* src, size_t bytes, stream_t s) {
     }
   };
   std::vector<std::thread> threads;
+  const unsigned nthread = stop ? 0 : std::min({hw, COPY_THREADS, (unsigned)n});
   try {
-    for (unsigned t = 0; t < std::min({hw, COPY_THREADS, (unsigned)n}) && !stop; ++t)
-      threads.emplace_back(work);
+    for (unsigned t = 0; t < nthread; ++t) threads.emplace_back(work);
   } catch (...) {  // fewer threads, or none
   }
   if (threads.empty()) {
