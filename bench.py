@@ -697,9 +697,9 @@ def main():
     e_ach = ebytes / (ems / 1000.0) / 1e9 if ems > 0 else None
     rl_tc_t = {"bound": "tensor", "achieved": w_ach, "peak": peaks["bf16_sustained"],
                "unit": "TFLOP/s", "frac": w_ach / peaks["bf16_sustained"] if w_ach else None,
-               "traffic": traffic_of(f"mgemm_pert_t_{a.workload}"),
-               "kernel": "mgemm_bf16_kernel, batched four-segment (T) W GEMMs (2 BF16 slices, "
-                         "3 pairs), first batch of the sweep",
+               "traffic": traffic_of(f"tc_kbuild_pert_t_{a.workload}"),
+               "kernel": "tc_kbuild_kernel (tcgen05.mma kind::f16, TMA), (T) K builds of four "
+                         "segments (2 BF16 slices, 3 pairs), first batch of the sweep",
                "launches": wlaunch, "ms": wms,
                "peak_source": "bf16_tflops_sustained, " + peaks["source"]}
     rl_energy = {"bound": "hbm", "achieved": e_ach, "peak": peaks["hbm_gbs"], "unit": "GB/s",
