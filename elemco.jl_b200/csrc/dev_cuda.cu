@@ -209,8 +209,8 @@ uint64_t tc_wait(stream_t s) {
 int sync(stream_t s) { return (int)cudaStreamSynchronize((cudaStream_t)s); }
 
 // The kernels write the code straight into host memory, so that reading it after
-// a synchronisation costs a load: copying one device variable per kernel back
-// took four synchronous copies, 30 to 40 us each time, four times an iteration.
+// a synchronisation costs a load (a device variable per kernel: a synchronous copy
+// of 30 to 40 us each, four times an iteration).
 // Words per stream: a context reads and clears the time-outs of its own kernels
 // and of no other's, and after its stream is synchronised nothing writes them.
 int* wait_error(stream_t s, int kernel) {

@@ -16,13 +16,12 @@
 // eight); the classes (la >= lb, l) are instantiations, so that all loops over
 // components are unrolled and R lives in registers, and the threads of a warp
 // share the pair (H is read as a broadcast).  What bounds it: latency, of the
-// longest contraction at small molecules and of the spilled R of the f and g
-// classes at large ones.  The kernel before,
-// one thread a triple over run-time loops, expansion tables and a 100-term
-// series for each Boys function in local memory, Cartesian output and three
-// GEMMs to spherical functions, took 29.4 + 5.4 ms for (H2O)4 cc-pVTZ/RI and 2.9
-// ms for H2O cc-pVDZ/RI; the factors' whole call (allocations and fitting
-// product included) now takes 9.7 and 1.0 ms.
+// longest contraction at small molecules and of the f and g classes, whose R and
+// sums live in local memory and whose pairs are few, at large ones ((H2O)4 cc-pVTZ:
+// 61% of the kernels' 4.2 ms in three classes of 29 to 301 blocks).  Measured, the
+// factors' whole call (allocations and fitting product included): H2O cc-pVDZ/RI 1.0
+// ms, (H2O)4 cc-pVTZ/RI 9.7; with run-time loops, expansion tables in local memory
+// and Cartesian output the integrals alone took 2.9 and 34.8.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -15,17 +15,18 @@
 // (a k-block is 12 MMAs of some 100 cycles), then the K traffic (five passes of
 // 4 v^3 bytes a triplet).  Hence:
 //  * One launch takes all triplets of a batch and all four K segments.
-//  * tn covers v in whole tiles of any multiple of 16 columns (kt_width): v =
-//    209 took two 128-column tiles (22% padding) or 256 rows, now one of 224.
+//  * tn covers v in whole tiles of any multiple of 16 columns (kt_width): one of
+//    224 at v = 209, where 128-column tiles pad by 22%.
 //  * The segment of a k-block is found by selects (seg_at).
 //  * The epilogue is a rolled loop over 16-column chunks that fetches the next
 //    chunk of K ahead: unrolled over a tile, with all of K's values fetched
 //    before the accumulator was waited for, it was slower (v = 129 6.2 against
 //    5.4 ms), the issuing thread sharing the instruction cache with it.
 //  * One lane a warp polls the accumulator's barrier.
-// Measured, the three launches of the largest batch, against six or seven
-// batched GEMMs: v = 129 9.0 -> 5.4 ms, v = 209 13.7 -> 12.0, v = 318 14.1 ->
-// 12.9 (33 triplets, 1000 TFLOP/s).  Not kept: 32-deep k-blocks in five stages
+// Measured, the three launches of the largest batch (seven batched GEMMs of fixed
+// tiles took 9.0, 13.7 and 14.1 ms): v = 129 5.4 ms, v = 209 12.0, v = 318 12.9 (33
+// triplets, 1000 TFLOP/s; at v = 200 the tensor pipe is 39 to 45% active, L2 42 to
+// 49%, DRAM 23 to 40%).  Not kept: 32-deep k-blocks in five stages
 // and stages of one slice (more loads of less; 3 to 13% slower), L2 prefetch of
 // the next tile's rows (10 to 30% slower), 256-row tiles on CTA pairs
 // (cta_group::2; v = 318 15.3 ms, v = 129 6.7).
@@ -292,9 +293,8 @@ __global__ void __launch_bounds__(KT_THREADS, 1)
         }
       };
       if (out.beta) fetch(hw, nxt);
-      // every lane waits; the warp goes on only if all lanes saw the
-      // accumulator ready and no time-out was recorded, so the warp-wide
-      // tcgen05.ld below always runs converged
+      // one lane polls; the warp goes on only if it saw the accumulator ready and no
+      // time-out was recorded, so the warp-wide tcgen05.ld below always runs converged
       const bool ready =
           lane != 0 || mbar_wait(&tfull[acc], (uint32_t)((lt >> 1) & 1), wait_ns);
       if (!__all_sync(0xffffffffu, ready)) {

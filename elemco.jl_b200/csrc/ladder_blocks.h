@@ -41,9 +41,9 @@ inline int64_t system_workspace(int64_t no, int64_t nv, int64_t nq) {
 // a-block size of the symmetric ladder: Vblk holds v^2 na (v - a0) doubles.
 // An eighth of the virtual space, but as much of it as 256 MiB of V hold: at
 // small v a block's five launches cost more than they compute (CCSD iteration
-// of o=12, v=57 with 256 / 64 / 32 MiB: 1.76 / 1.80 / 1.84 ms, eight blocks
-// 2.01; o=14, v=100: 5.78 / 5.97 / 5.98, eight blocks 6.05), and the tiles with
-// b < a are skipped inside a block.  The workspace is what eight blocks and the
+// of o=12, v=57 in one block 1.17 ms, in two 1.21; with slower ring terms 1.76
+// and, in eight, 2.01; o=14, v=100 in four 5.78, in eight 6.05), and the tiles
+// with b < a are skipped inside a block.  The workspace is what eight blocks and the
 // other terms were given, and larger blocks take what of it is free beside the o^4
 // and n^2 matrices that the callers keep: they take no more memory.  Blocks are
 // then made alike (o=12, v=57: 30 + 27).

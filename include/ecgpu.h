@@ -69,11 +69,12 @@ int ecg_set_precision(ecg_ctx* ctx, int prec);
  *  ECG_OPT_TRIPLES_BATCH  at most this many occupied triplets per (T) batch
  *                         (one K slot each; the sweep's batches after the first
  *                         replay from one CUDA graph)
- *  ECG_OPT_TC_WAIT_NS     bound in ns on the tensor-core GEMM's main-loop
- *                         waits on this context's stream (default 1 s); a wait
- *                         that runs out makes the call return ECG_ERR_TIMEOUT
- *                         and the context stays usable (the kernel's final
- *                         waits on its own copies keep the 1 s bound)
+ *  ECG_OPT_TC_WAIT_NS     bound in ns on the main-loop waits of the GEMM, K-build
+ *                         and FP32 (T) energy kernels on this context's stream
+ *                         (default 1 s); a wait that runs out makes the call
+ *                         that queued it return ECG_ERR_TIMEOUT and the context
+ *                         stays usable (the kernels' final waits on their own
+ *                         copies keep the 1 s bound)
  *  ECG_OPT_AUTOTUNE       1: GEMM shapes without an entry in the tuning table
  *                         are tuned on first use (see ecg_tune_save); 0: the
  *                         table's entries, else the fixed rules, are used.
