@@ -134,7 +134,8 @@ void sync_checked(Ctx& c) {
   if (!list.empty()) throw Error(ECG_ERR_TIMEOUT, "bounded wait timed out (code " + list + ")");
 }
 
-void drop_time_outs(Ctx& c) noexcept {
+void after_failure(Ctx& c) noexcept {
+  c.ws.release(0);
   if (!c.st) return;
   int codes[dev::WAIT_KERNELS];
   if (dev::sync(c.st) == 0) dev::tc_error(c.st, codes);

@@ -142,8 +142,9 @@ double scal(Ctx& c, int i);
 // last check is an ECG_ERR_TIMEOUT.  Every call whose results rest on kernels with
 // such waits (all FP64 and tensor-core GEMMs) ends with one.
 void sync_checked(Ctx& c);
-// Waits likewise and forgets time-outs: a call that failed leaves none to the next.
-void drop_time_outs(Ctx& c) noexcept;
+// What a call that failed leaves to the next: its kernels are done, their time-outs
+// forgotten, and the workspace, which no call keeps anything in, is free again.
+void after_failure(Ctx& c) noexcept;
 void sync_scalars(Ctx& c, int count);  // the first `count` scalars to hscal, sync_checked
 
 // Runs f, turning the library's exceptions into a status code and a message
@@ -156,16 +157,16 @@ int guarded(Ctx* c, F&& f) {
     if (c) c->err.clear();
     return ECG_OK;
   } catch (const Error& e) {
-    if (c) drop_time_outs(*c);
+    if (c) after_failure(*c);
     if (c) c->err = e.what();
     else noctx_error_store(e.what());
     return e.code;
   } catch (const std::bad_alloc&) {
-    if (c) drop_time_outs(*c);
+    if (c) after_failure(*c);
     if (c) c->err = "host out of memory";
     return ECG_ERR_OOM;
   } catch (const std::exception& e) {
-    if (c) drop_time_outs(*c);
+    if (c) after_failure(*c);
     if (c) c->err = e.what();
     return ECG_ERR_ARG;
   }

@@ -134,3 +134,23 @@ def test_copies_for_odd_pitches_keep_to_the_cap():
         c.set_mem_cap(cap_lambda)
         c.lambda_residual(T1, T2, 2.0 * T1, 2.0 * T2 - T2.transpose(1, 0, 2, 3))
         assert before - torch.cuda.mem_get_info()[0] < cap_lambda - cap + (64 << 20)
+
+
+def test_workspace_is_free_after_a_refusal():
+    """Mixed iterations that the cap stops inside the ladder (the storage of its BF16
+    slices), again and again: the workspace they had taken is there for the next call."""
+    size = (6, 64, 160)
+    with ecgpu.Context(0) as c:
+        c.set_system(*_system(*size))
+        _, T1, T2 = c.mp2()
+        ref = c.cc_residual(T1, T2)
+        c.cc_load(T1, T2)
+        c.set_precision(ecgpu.ECG_PREC_MIXED)
+        c.set_mem_cap(1 << 16)
+        for _ in range(4):
+            with pytest.raises(ecgpu.ECGError) as e:
+                c.cc_step()
+            assert e.value.code == ECG_ERR_OOM and "split-operand" in str(e.value)
+        c.set_mem_cap(0)
+        c.set_precision(ecgpu.ECG_PREC_FP64)
+        assert _close(c.cc_residual(T1, T2), ref)
