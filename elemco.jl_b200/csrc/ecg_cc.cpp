@@ -233,7 +233,7 @@ void setup_system(Ctx& c, int no, int nv, int nq, const double* B, const double*
                                   {&c.dfvv, v * v}, {&c.J, Q}, {&c.dscal, 256}});
   const int64_t oovv = o * o * v * v;
   group("two-electron matrices",
-        {{&c.klcd, oovv}, {&c.Kvvoo, oovv}, {&c.V1, oovv}, {&c.V2, oovv}, {&c.TT, oovv}});
+        {{&c.klcd, oovv}, {&c.Kvvoo, oovv}, {&c.V1, oovv}, {&c.V2, oovv}});
   c.dBvv = c.alloc(v * v * Q, "dBvv");
   c.dBvvT = c.alloc(v * v * Q, "dBvvT");
   c.dBvo = c.alloc(v * o * Q, "dBvo");
@@ -390,11 +390,12 @@ void ladder(Ctx& c, const double* Bf, const double* BfT, const double* T2, doubl
   // the BF16 slices of a block are storage of their own, which stays small
   const auto& blocks = mp || mm ? c.lblocks8 : c.lblocks;
   const int64_t maxpp = blocks[0].npp;  // the first block has the most
-  double* V = c.ws.get(v * blocks[0].na * v * v);
+  // V+/- take V's place in the products, and L+/- its memory
+  double* V = c.ws.get(std::max(v * blocks[0].na * v * v, maxpp * (nijp + nijm)));
+  double* Lp = V;
+  double* Lm = V + maxpp * nijp;
   double* Vp = c.ws.get(ldp * maxpp);
   double* Vm = c.ws.get(std::max<int64_t>(ldm * maxpp, 1));
-  double* Lp = c.ws.get(maxpp * nijp);
-  double* Lm = c.ws.get(std::max<int64_t>(maxpp * nijm, 1));
   constexpr int NSL = 3;
   dev::TcOperand oB, oTs, oTa, oVp, oVm;
   uint16_t *pB = nullptr, *pTs = nullptr, *pTa = nullptr, *pVp = nullptr, *pVm = nullptr;
@@ -416,7 +417,8 @@ void ladder(Ctx& c, const double* Bf, const double* BfT, const double* T2, doubl
   }
   if (!mv && v % 2 == 1) {
     ldb = v * v + 1;
-    double* t = c.ws.get(ldb * Q);
+    // the only block's V is built before V+ is packed
+    double* t = ladder_pad_in_vp(v, Q, blocks[0].na) ? Vp : c.ws.get(ldb * Q);
     check(dev::repitch(s, v * v, Q, BfT, v * v, t, ldb), "pad BfT");
     Bl = t;
   }

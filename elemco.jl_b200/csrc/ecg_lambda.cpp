@@ -33,7 +33,7 @@ void lambda_prepare(Ctx& c, bool dc) {
   ensure_lambda_buffers(c);
   const int64_t o = c.no, v = c.nv;
   // one o v^3 block for d_vovv plus a same-sized permute temporary
-  c.ensure_ws(2 * o * v * v * v + 14 * c.n2() + (1 << 20) - (1 << 15) - (o + v) * (o + v));
+  c.ensure_ws(2 * o * v * v * v + 15 * c.n2() + (1 << 20) - (1 << 15) - (o + v) * (o + v));
   dress(c, c.T1());
   Contractor con = c.con();
   const int64_t mark = c.ws.mark();
@@ -276,14 +276,15 @@ LambdaResult lambda_solve(Ctx& c, bool dc, const ecg_cc_opts& o) {
   lambda_prepare(c, dc);
   double* U1 = c.U;
   double* U2 = c.U + n1;
+  const int64_t mark = c.ws.mark();
+  double* TT = c.ws.get(n2);
   // guess: U2 = 2 tau - tau[a,b,j,i], tau = T2 + T1 T1; U1 = 2 T1 (cctools.jl:919-930)
-  check(dev::outer(s, c.nv, c.no, c.nv, c.no, 1.0, c.T1(), c.T1(), 0.0, c.TT), "outer");
-  check(dev::axpby(s, n2, 1.0, c.T2(), 1.0, c.TT), "tau");
-  check(dev::axpby(s, n2, 2.0, c.TT, 0.0, U2), "U2");
-  c.con().permute(-1.0, c.TT, "abji", 1.0, U2, "abij");
+  check(dev::outer(s, c.nv, c.no, c.nv, c.no, 1.0, c.T1(), c.T1(), 0.0, TT), "outer");
+  check(dev::axpby(s, n2, 1.0, c.T2(), 1.0, TT), "tau");
+  check(dev::axpby(s, n2, 2.0, TT, 0.0, U2), "U2");
+  c.con().permute(-1.0, TT, "abji", 1.0, U2, "abij");
   check(dev::axpby(s, n1, 2.0, c.T1(), 0.0, U1), "U1");
-  // TT = T1 T1 for the correlation norm
-  check(dev::outer(s, c.nv, c.no, c.nv, c.no, 1.0, c.T1(), c.T1(), 0.0, c.TT), "outer");
+  c.ws.release(mark);
   diis_reset(c, c.ldiis, o.maxdiis, o.resthr, n1 + n2, false);
   const double thren = std::sqrt(o.thr) * o.conven;
   const double* eo = c.eps;
@@ -312,11 +313,12 @@ LambdaResult lambda_solve(Ctx& c, bool dc, const ecg_cc_opts& o) {
     const double NormR1 = 0.5 * c.hscal[2];
     diis_perform(c, c.ldiis, c.U, c.RU);
     // calc_correlation_norm (cc_lagrange.jl:1065-1078)
-    check(dev::dot(s, n2, U2, c.T2(), c.red, c.dscal + 10), "cnorm");
-    check(dev::dot(s, n2, U2, c.TT, c.red, c.dscal + 11), "cnorm");
-    check(dev::dot(s, n1, U1, c.T1(), c.red, c.dscal + 12), "cnorm");
-    sync_scalars(c, 13);
-    const double norm = c.hscal[10] + c.hscal[11] + c.hscal[12];
+    const dev::DotJob jobs[3] = {{dev::DOT_PLAIN, U2, c.T2(), n2, c.dscal + 10},
+                                 {dev::DOT_CS_T1, c.T1(), U2, 0, c.dscal + 11},
+                                 {dev::DOT_PLAIN, U1, c.T1(), n1, c.dscal + 13}};
+    check(dev::dots(s, c.nv, c.no, 3, jobs, c.red), "cnorm");
+    sync_scalars(c, 14);
+    const double norm = c.hscal[10] + c.hscal[11] + c.hscal[13];
     r.normR = NormR1 + NormR2;
     r.dnorm = norm - prev;
     r.norm = norm;

@@ -19,6 +19,12 @@ inline int64_t ladder_eighth(int64_t nv) {
 // Pairs a <= b of the first block, which has the most of them.
 inline int64_t ladder_pairs(int64_t nv, int64_t na) { return na * nv - na * (na - 1) / 2; }
 
+// Whether the copy of B in an even pitch (odd nv, FP64) fits V+'s place, which a
+// single block leaves free until V is built.
+inline bool ladder_pad_in_vp(int64_t nv, int64_t nq, int64_t na) {
+  return na == nv && (nv * nv + 1) * nq <= (nv * (nv + 1) / 2 + 1) / 2 * 2 * ladder_pairs(nv, na);
+}
+
 // Doubles of workspace that ladder() takes with blocks of na.
 inline int64_t ladder_need(int64_t no, int64_t nv, int64_t nq, int64_t na) {
   auto get = [](int64_t n) { return (std::max<int64_t>(n, 1) + 31) / 32 * 32; };
@@ -26,15 +32,15 @@ inline int64_t ladder_need(int64_t no, int64_t nv, int64_t nq, int64_t na) {
   const int64_t ijp = no * (no + 1) / 2, ijm = no * (no - 1) / 2;
   const int64_t ldp = (cdp + 1) / 2 * 2, ldm = std::max<int64_t>((cdm + 1) / 2 * 2, 2);
   const int64_t pp = ladder_pairs(nv, na);
-  return get(ldp * ijp) + get(ldm * ijm) + get(na * nv * nv * nv) + get(ldp * pp) +
-         get(ldm * pp) + get(pp * ijp) + get(pp * ijm) +
-         (nv % 2 ? get((nv * nv + 1) * nq) : 0);
+  return get(ldp * ijp) + get(ldm * ijm) +
+         get(std::max(na * nv * nv * nv, pp * (ijp + ijm))) + get(ldp * pp) + get(ldm * pp) +
+         (nv % 2 && !ladder_pad_in_vp(nv, nq, na) ? get((nv * nv + 1) * nq) : 0);
 }
 
 // Doubles of workspace of a system.
 inline int64_t system_workspace(int64_t no, int64_t nv, int64_t nq) {
   const int64_t n = no + nv, n2 = no * no * nv * nv;
-  return 14 * n2 + 6 * nv * no * nq + 3 * nv * nv * nq + 2 * n * n * nq + 4 * no * no * no * no +
+  return 15 * n2 + 6 * nv * no * nq + 3 * nv * nv * nq + 2 * n * n * nq + 4 * no * no * no * no +
          3 * ladder_eighth(nv) * nv * nv * nv + 6 * n * n + (1 << 15);
 }
 
@@ -46,7 +52,7 @@ inline int64_t system_workspace(int64_t no, int64_t nv, int64_t nq) {
 // with b < a are skipped inside a block.  The workspace is what eight blocks and the
 // other terms were given, and larger blocks take what of it is free beside the o^4
 // and n^2 matrices that the callers keep: they take no more memory.  Blocks are
-// then made alike (o=12, v=57: 30 + 27).
+// then made alike (o=16, v=76: 38 + 38).
 inline int64_t ladder_na(int64_t no, int64_t nv, int64_t nq) {
   const int64_t lim = std::min(ladder_na_limit(nv), nv), n = no + nv;
   const int64_t least = std::min(((nv + 7) / 8 + 1) / 2 * 2, lim);
